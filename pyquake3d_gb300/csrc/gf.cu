@@ -3,9 +3,15 @@
 //   setup_sources / setup_receivers   once per mesh: per-source record (frame,
 //                                     angles, side vectors) and per-receiver
 //                                     record (centroid, frame)
-//   assemble_dense                    one (receiver, source) pair per thread,
-//                                     both unit slips, 6 tractions -> FP64 K
-//                                     (+ FP32 copy) with 16-byte stores
+//   setup_tiles                       once per mesh: the vertices and edges that
+//                                     the triangles of a tile share
+//   assemble_seg                      full space: per (tile of sources,
+//                                     receiver) every vertex distance and edge
+//                                     matrix once, then one (receiver, source)
+//                                     pair per thread, both unit slips, 6
+//                                     tractions -> FP64 K (+ FP32 copy) with
+//                                     16-byte stores
+//   assemble_dense_hs                 half space: one pair per thread
 //   points_one_source / point_many_sources
 //                                     the two host-pointer entry points of the
 //                                     reference TDstressFS_C.so
@@ -23,6 +29,7 @@
 #include "common.cuh"
 #include "gf_device.cuh"
 #include "hs_device.cuh"
+#include "seg_device.cuh"
 
 namespace pq3d {
 namespace gf {
@@ -41,28 +48,124 @@ struct ValSrc {   // fields held in a small array
 struct SrcVal { double f[kSrcStride]; };
 struct FscVal { double f[kFscStride]; };
 
-__global__ void setup_sources_kernel(const double *__restrict__ nodes, const int64_t *__restrict__ tris, int64_t N,
-                                     double *__restrict__ src)
+__device__ __forceinline__ void load_triangle(const double *__restrict__ nodes, const int64_t *__restrict__ tris,
+                                              int64_t j, double a[3], double b[3], double c[3])
 {
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= N) return;
-    const double *P1 = nodes + 3 * (tris[3 * j] - 1);
-    const double *P2 = nodes + 3 * (tris[3 * j + 1] - 1);
-    const double *P3 = nodes + 3 * (tris[3 * j + 2] - 1);
-    double a[3] = {P1[0], P1[1], P1[2]}, b[3] = {P2[0], P2[1], P2[2]}, c[3] = {P3[0], P3[1], P3[2]};
-    setup_source(a, b, c, src + j, (int)N);
+    const double *A = nodes + 3 * (tris[3 * j] - 1), *B = nodes + 3 * (tris[3 * j + 1] - 1),
+                 *C = nodes + 3 * (tris[3 * j + 2] - 1);
+    for (int q = 0; q < 3; ++q) { a[q] = A[q]; b[q] = B[q]; c[q] = C[q]; }
 }
 
-__global__ void setup_receivers_kernel(const double *__restrict__ nodes, const int64_t *__restrict__ tris, int64_t N,
-                                       double *__restrict__ recv)
+// Source and receiver records of element j, in one launch: blocks [0, nb) the
+// sources, [nb, 2 nb) the receivers (both are short chains of FP64 latency).
+__global__ void setup_elements_kernel(const double *__restrict__ nodes, const int64_t *__restrict__ tris, int64_t N,
+                                      unsigned nb, double *__restrict__ src, double *__restrict__ recv,
+                                      double *__restrict__ seg)
 {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    const double *A = nodes + 3 * (tris[3 * i] - 1);
-    const double *B = nodes + 3 * (tris[3 * i + 1] - 1);
-    const double *C = nodes + 3 * (tris[3 * i + 2] - 1);
-    double a[3] = {A[0], A[1], A[2]}, b[3] = {B[0], B[1], B[2]}, c[3] = {C[0], C[1], C[2]};
-    setup_receiver(a, b, c, recv + kRecvStride * i);
+    const bool source = blockIdx.x < nb;
+    const int64_t j = (blockIdx.x - (source ? 0u : nb)) * (int64_t)blockDim.x + threadIdx.x;
+    if (j >= N) return;
+    double a[3], b[3], c[3];
+    load_triangle(nodes, tris, j, a, b, c);
+    if (source) setup_source(a, b, c, src + j, (int)N);
+    else setup_receiver(a, b, c, recv + kRecvStride * j);
+    if (!source && seg) setup_seg(a, b, c, seg + j, N);
+}
+
+// ---------------------------------------------------------------------------
+// tiles of sources: the triangles [tile * ts, tile * ts + ts) and the distinct
+// vertices and edges they use
+
+constexpr int kTileMax = 256;   // triangles of a tile at most
+constexpr int kTileItems = 3 * kTileMax;
+
+struct __align__(8) TileEdge {   // local edge: from vertex a to vertex b (the smaller node id first)
+    double L, iL;
+    float near2;
+    uint16_t a, b;
+};
+struct __align__(8) TileTri {    // local edges of P1 P2, P2 P3, P3 P1; bit 15: walked from b to a
+    uint16_t e[3], pad;
+};
+struct Tile {
+    int32_t nv, ne, pad[2];
+    double vert[kTileItems][3];
+    TileEdge edge[kTileItems];
+    TileTri tri[kTileMax];
+};
+constexpr int kSegDoubles = (int)(sizeof(Tile) / sizeof(double));
+static_assert(sizeof(Tile) % 16 == 0, "tiles start 16-byte aligned");
+
+inline int64_t tile_count(int64_t N) { return (N + kTileMax - 1) / kTileMax; }
+// equal tiles: the last one of N = 1,600 would hold 64 of 256 triangles, and
+// its blocks would idle while the others finish
+inline int tile_size(int64_t N) { return (int)((N + tile_count(N) - 1) / tile_count(N)); }
+
+// One block per tile: the node ids and the node pairs go into hash tables in
+// shared memory; the thread that places a key takes the next local index.
+// (The numbering depends on the order of arrival; no value computed from the
+// tables does.)
+constexpr int kHash = 2048;
+__global__ void __launch_bounds__(kTileMax)
+setup_tiles_kernel(const double *__restrict__ nodes, const int64_t *__restrict__ tris, int64_t N, int ts,
+                   Tile *__restrict__ tiles)
+{
+    __shared__ unsigned long long vkey[kHash], ekey[kHash];
+    __shared__ uint16_t vidx[kHash], eidx[kHash];
+    __shared__ int nv, ne;
+    const int t = threadIdx.x;
+    for (int i = t; i < kHash; i += kTileMax) vkey[i] = ekey[i] = ~0ull;
+    if (t == 0) nv = ne = 0;
+    __syncthreads();
+    Tile &T = tiles[blockIdx.x];
+    const int64_t j = (int64_t)blockIdx.x * ts + t;
+    const bool on = t < ts && j < N;
+    int vs[3], es[3];
+    bool vown[3], eown[3];
+    int64_t id[3];
+    // at most 768 keys in 2,048 places: the probe ends
+    auto place = [](unsigned long long *key, uint16_t *idx, int *count, unsigned long long k, int &slot) {
+        slot = (int)((k * 0x9E3779B97F4A7C15ull) >> 53);
+        for (int probe = 0; probe < kHash; ++probe, slot = (slot + 1) & (kHash - 1)) {
+            const unsigned long long old = atomicCAS(&key[slot], ~0ull, k);
+            if (old == ~0ull) {
+                idx[slot] = (uint16_t)atomicAdd(count, 1);
+                return true;
+            }
+            if (old == k) return false;
+        }
+        return false;
+    };
+    if (on) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) id[q] = tris[3 * j + q];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const unsigned long long p = (unsigned long long)id[q], r = (unsigned long long)id[(q + 1) % 3];
+            vown[q] = place(vkey, vidx, &nv, p, vs[q]);
+            eown[q] = place(ekey, eidx, &ne, p < r ? (p << 32 | r) : (r << 32 | p), es[q]);
+        }
+    }
+    __syncthreads();
+    if (on) {
+        TileTri tri;
+        tri.pad = 0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const int n = (q + 1) % 3;
+            const bool rev = id[q] > id[n];
+            if (vown[q])
+                for (int c = 0; c < 3; ++c) T.vert[vidx[vs[q]]][c] = nodes[3 * (id[q] - 1) + c];
+            const int e = eidx[es[q]];
+            if (eown[q]) {
+                const SegEdge r = seg_edge_record(nodes + 3 * (id[q] - 1), nodes + 3 * (id[n] - 1));
+                T.edge[e] = TileEdge{r.L, r.iL, r.near2, vidx[vs[rev ? n : q]], vidx[vs[rev ? q : n]]};
+            }
+            tri.e[q] = (uint16_t)(e | (rev ? 0x8000 : 0));
+        }
+        T.tri[t] = tri;
+    }
+    if (t == 0) { T.nv = nv; T.ne = ne; }
 }
 
 // Half-space records of source j: the mirrored triangle's source record
@@ -81,47 +184,126 @@ __global__ void setup_hs_kernel(const double *__restrict__ nodes, const int64_t 
     setup_fsc(a, b, c, fsc + j, (int)N);
 }
 
-constexpr int kTJ = 128;   // sources per block (one per thread)
-constexpr int kTI = 32;    // receivers per block (looped by every thread)
+// ---------------------------------------------------------------------------
+// Full-space dense assembly from the tiles.  Per batch of receivers: (1) every
+// vertex of the tile from every receiver, (2) every edge's matrix, both items
+// spread evenly over the block, (3) a thread per triangle adds its three edge
+// matrices and applies them to its two slip directions.
+//
+// Bound: the FP64 pipe (2 lanes per clock and SM).  About 21 FP64 operations
+// per vertex, 95 per edge and 54 per pair; on a structured mesh a tile of 256
+// triangles has 0.7 vertices and 1.7 edges per triangle, so a pair takes ~230
+// (520 as three angular dislocations per pair).  256 triangles per tile: 128
+// have 1.9 edges per triangle; more would leave one block per SM.
+constexpr int kSegThreads = 256;
+constexpr int kSegRecv = 64;              // receivers of a block at most
+constexpr int kSegSmem = 104 * 1024;      // two blocks per SM; holds the 768 vertices and edges of a tile
+                                          // that shares none for one receiver (90 KB)
+constexpr int kVertD = 6, kMatD = 9;
+static_assert((kVertD + kMatD) * kTileItems * sizeof(double) <= kSegSmem, "one receiver of any tile fits");
 
-// K64 / K32 point at row 3*row0; leading dimension 2N.
-template <bool kWrite32>
-__global__ void __launch_bounds__(kTJ)
-assemble_dense_kernel(const double *__restrict__ src, const double *__restrict__ recv, int64_t N, int64_t row0,
-                      int64_t row1, double nu, double k, double two_mu, double lam, double *__restrict__ K64,
-                      float *__restrict__ K32)
+// The pair by its angular dislocations (receivers on an edge of the source).
+__device__ __noinline__ void pair_angular(const double *src, int64_t N, const double *R, double nu, double k,
+                                          double two_mu, double lam, double ts[3], double td[3])
 {
-    __shared__ double s_src[F_COUNT * kTJ];
-    __shared__ double s_rcv[kTI * kRecvStride];
+    const SoaSrc F{src, (int)N};
+    pair_tractions(F, R, nu, k, two_mu, lam, ts, td);
+}
+
+// K64 / K32 point at row 3*row0; leading dimension 2N; nr receivers per block.
+template <bool kWrite32>
+__global__ void __launch_bounds__(kSegThreads, 2)
+assemble_seg_kernel(const Tile *__restrict__ tiles, int ts, const double *__restrict__ src,
+                    const double *__restrict__ recv, int64_t N, int64_t row0, int64_t row1, int nr, SegMat mat,
+                    double nu, double k, double two_mu, double lam, double *__restrict__ K64, float *__restrict__ K32)
+{
+    extern __shared__ double s_buf[];
+    __shared__ double s_rcv[kSegRecv * kRecvStride];
     const int t = threadIdx.x;
-    const int64_t j0 = (int64_t)blockIdx.x * kTJ;
-    const int64_t i0 = row0 + (int64_t)blockIdx.y * kTI;
-    const int64_t j = j0 + t;
-    for (int f = 0; f < F_COUNT; ++f) s_src[f * kTJ + t] = (j < N) ? src[f * N + j] : 0.0;
-    const int nrec = (int)((row1 - i0) < kTI ? (row1 - i0) : kTI);
-    // receiver records with e1 and e2 multiplied by the traction scale
-    const double axis_scale = traction_axis_scale(k, two_mu);
-    for (int q = t; q < nrec * kRecvStride; q += kTJ) {
-        const int fq = q % kRecvStride;
-        const double v = recv[i0 * kRecvStride + q];
-        s_rcv[q] = (fq >= 3 && fq < 9) ? v * axis_scale : v;
-    }
-    __syncthreads();
-    if (j >= N) return;
-    const SoaSrc F{s_src + t, kTJ};
-    const int64_t ld = 2 * N;
-    for (int ii = 0; ii < nrec; ++ii) {
-        double ts[3], td[3];
-        pair_tractions<SoaSrc, true>(F, s_rcv + ii * kRecvStride, nu, k, two_mu, lam, ts, td);
-        const int64_t r = 3 * (i0 + ii - row0);
+    const Tile &T = tiles[blockIdx.x];
+    const int nv = T.nv, ne = T.ne;
+    const int64_t i0 = row0 + (int64_t)blockIdx.y * nr;
+    const int nrec = (int)((row1 - i0) < nr ? (row1 - i0) : nr);
+    for (int q = t; q < nrec * kRecvStride; q += kSegThreads) s_rcv[q] = recv[i0 * kRecvStride + q];
+    const int batch = min(nrec, kSegSmem / (int)sizeof(double) / (nv * kVertD + ne * kMatD));
+    double *sv = s_buf, *sm = s_buf + (size_t)batch * nv * kVertD;
+    // this thread's triangle: edges, and its slip directions times mu/(4 pi)
+    const int64_t j = (int64_t)blockIdx.x * ts + t;
+    const bool on = t < ts && j < N;
+    int e[3];
+    unsigned sg[3];
+    double bs[3], bd[3];
+    if (on) {
+        const TileTri tri = T.tri[t];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            *reinterpret_cast<double2 *>(K64 + (r + c) * ld + 2 * j) = make_double2(ts[c], td[c]);
-            if (kWrite32)
-                *reinterpret_cast<float2 *>(K32 + (r + c) * ld + 2 * j) = make_float2(d2f_rn_bits(ts[c]), d2f_rn_bits(td[c]));
+        for (int q = 0; q < 3; ++q) {
+            e[q] = (tri.e[q] & 0x7fff) * kMatD;
+            sg[q] = (unsigned)(tri.e[q] & 0x8000) << 16;
+            bs[q] = mat.scale * src[(F_SX + q) * N + j];
+            bd[q] = mat.scale * src[(F_DX + q) * N + j];
+        }
+    }
+    const int64_t ld = 2 * N;
+    for (int b0 = 0; b0 < nrec; b0 += batch) {
+        const int nb = min(batch, nrec - b0);
+        __syncthreads();   // the receivers are in; the last batch's readers are done
+        for (int q = t; q < nb * nv; q += kSegThreads) {
+            const int r = q / nv, v = q - r * nv;
+            const SegVert p = seg_vertex(s_rcv + (b0 + r) * kRecvStride, T.vert[v][0], T.vert[v][1], T.vert[v][2]);
+            double *o = sv + q * kVertD;
+            reinterpret_cast<double2 *>(o)[0] = make_double2(p.x, p.y);
+            reinterpret_cast<double2 *>(o)[1] = make_double2(p.z, p.r);
+            reinterpret_cast<double2 *>(o)[2] = make_double2(p.ir, p.ir3);
+        }
+        __syncthreads();
+        for (int q = t; q < nb * ne; q += kSegThreads) {
+            const int r = q / ne;
+            const TileEdge ed = T.edge[q - r * ne];
+            auto vert = [&](int v) {
+                const double2 *o = reinterpret_cast<const double2 *>(sv + (r * nv + v) * kVertD);
+                return SegVert{o[0].x, o[0].y, o[1].x, o[1].y, o[2].x, o[2].y};
+            };
+            double M[9];
+            seg_matrix(seg_terms(vert(ed.a), vert(ed.b), ed.L, ed.iL, ed.near2, mat.kap), mat.kap, mat.ci, M);
+#pragma unroll
+            for (int c = 0; c < 9; ++c) sm[q * kMatD + c] = M[c];
+        }
+        __syncthreads();
+        if (!on) continue;
+        for (int r = 0; r < nb; ++r) {
+            const double *R = s_rcv + (b0 + r) * kRecvStride, *Mr = sm + r * ne * kMatD;
+            double vs[3], vd[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                vs[a] = R[3 + 3 * a] * bs[0] + R[4 + 3 * a] * bs[1] + R[5 + 3 * a] * bs[2];
+                vd[a] = R[3 + 3 * a] * bd[0] + R[4 + 3 * a] * bd[1] + R[5 + 3 * a] * bd[2];
+            }
+            double ts3[3], td3[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                double m[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+                    m[a] = (flip_sign(Mr[e[0] + 3 * c + a], sg[0]) + flip_sign(Mr[e[1] + 3 * c + a], sg[1])) +
+                           flip_sign(Mr[e[2] + 3 * c + a], sg[2]);
+                ts3[c] = m[0] * vs[0] + m[1] * vs[1] + m[2] * vs[2];
+                td3[c] = m[0] * vd[0] + m[1] * vd[1] + m[2] * vd[2];
+            }
+            if (seg_bad(ts3[0])) pair_angular(src + j, N, R, nu, k, two_mu, lam, ts3, td3);
+            const int64_t row = 3 * (i0 + b0 + r - row0);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                *reinterpret_cast<double2 *>(K64 + (row + c) * ld + 2 * j) = make_double2(ts3[c], td3[c]);
+                if (kWrite32)
+                    *reinterpret_cast<float2 *>(K32 + (row + c) * ld + 2 * j) =
+                        make_float2(d2f_rn_bits(ts3[c]), d2f_rn_bits(td3[c]));
+            }
         }
     }
 }
+
+constexpr int kTJ = 128;   // half space: sources per block (one per thread)
+constexpr int kTI = 32;    // receivers per block (looped by every thread)
 
 // Half-space variant: main record in shared memory, image record and side
 // table read from their structure-of-arrays tables (coalesced over sources).
@@ -354,50 +536,111 @@ static int point_many_sources(double x, double y, double z, const double *P1, co
 }
 
 // Workspace: source table [kSrcStride][N], receiver table [N][kRecvStride],
-// then (half-space) image table [kImgStride][N] and side table [kFscStride][N].
+// then for the half space the image table [kImgStride][N] and the side table
+// [kFscStride][N], for the full space (from an even offset) the tiles.
+static size_t tiles_offset(int64_t N) { return ((size_t)N * (kSrcStride + kRecvStride) + 1) & ~(size_t)1; }
 static size_t ws_bytes(int64_t N, bool half)
 {
-    return (size_t)N * (kSrcStride + kRecvStride + (half ? kImgStride + kFscStride : 0)) * sizeof(double);
+    const size_t h = (size_t)N * (kSrcStride + kRecvStride + kImgStride + kFscStride);
+    return (half ? h : tiles_offset(N) + (size_t)tile_count(N) * kSegDoubles) * sizeof(double);
+}
+
+static void setup_elements(const double *nodes, const int64_t *tris, int64_t N, double *src, double *recv,
+                           double *seg, cudaStream_t st)
+{
+    const unsigned nb = (unsigned)((N + 127) / 128);
+    setup_elements_kernel<<<2 * nb, 128, 0, st>>>(nodes, tris, N, nb, src, recv, seg);
+}
+
+// Receivers per block: the grid's tail costs up to one block's time, so the
+// count (16 .. kSegRecv) with the fewest receivers on a slot's path wins; one
+// extra receiver stands for a block's start.
+static int seg_receivers(int64_t tiles, int64_t rows, int64_t slots)
+{
+    int best = kSegRecv;
+    int64_t cost = INT64_MAX;
+    for (int nr = kSegRecv; nr >= 16; --nr) {
+        const int64_t waves = (tiles * ((rows + nr - 1) / nr) + slots - 1) / slots;
+        const int64_t c = waves * (nr + 1);
+        if (c < cost) { cost = c; best = nr; }
+    }
+    return best;
+}
+
+struct SegCfg {
+    int device = -1;
+    int sms = 0;
+};
+static thread_local SegCfg g_seg;
+
+static int seg_config(int *sms)
+{
+    int dev;
+    PQ3D_CUDA_TRY(cudaGetDevice(&dev));
+    if (g_seg.device != dev) {
+        PQ3D_CUDA_TRY(cudaDeviceGetAttribute(&g_seg.sms, cudaDevAttrMultiProcessorCount, dev));
+        PQ3D_CUDA_TRY(cudaFuncSetAttribute(assemble_seg_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           kSegSmem));
+        PQ3D_CUDA_TRY(cudaFuncSetAttribute(assemble_seg_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           kSegSmem));
+        g_seg.device = dev;
+    }
+    *sms = g_seg.sms;
+    return PQ3D_OK;
 }
 
 static int assemble_rows(const double *nodes, const int64_t *tris, int64_t N, int64_t row0, int64_t row1, double mu,
-                         double lam, double *K64, float *K32, double *src, double *recv, bool do_setup,
-                         cudaStream_t st, bool half = false)
+                         double lam, double *K64, float *K32, double *ws, bool do_setup, cudaStream_t st,
+                         bool half = false)
 {
+    double *src = ws, *recv = src + (size_t)kSrcStride * N;
     double *img = recv + (size_t)kRecvStride * N, *fsc = img + (size_t)kImgStride * N;
+    Tile *tiles = (Tile *)(ws + tiles_offset(N));
+    const int ts = tile_size(N);
+    const int64_t nt = (N + ts - 1) / ts;
     if (do_setup) {
         const int th = 128;
-        const unsigned nb = (unsigned)((N + th - 1) / th);
-        setup_sources_kernel<<<nb, th, 0, st>>>(nodes, tris, N, src);
-        setup_receivers_kernel<<<nb, th, 0, st>>>(nodes, tris, N, recv);
-        if (half) setup_hs_kernel<<<nb, th, 0, st>>>(nodes, tris, N, img, fsc);
+        setup_elements(nodes, tris, N, src, recv, nullptr, st);
+        if (half) setup_hs_kernel<<<(unsigned)((N + th - 1) / th), th, 0, st>>>(nodes, tris, N, img, fsc);
+        else setup_tiles_kernel<<<(unsigned)nt, kTileMax, 0, st>>>(nodes, tris, N, ts, tiles);
         PQ3D_CUDA_TRY(cudaGetLastError());
     }
+    if (row0 == row1) return PQ3D_OK;
     const double nu = poisson(mu, lam);
-    dim3 grid((unsigned)((N + kTJ - 1) / kTJ), (unsigned)((row1 - row0 + kTI - 1) / kTI));
     if (half) {
+        dim3 grid((unsigned)((N + kTJ - 1) / kTJ), (unsigned)((row1 - row0 + kTI - 1) / kTI));
         if (K32)
             assemble_dense_hs_kernel<true><<<grid, kTJ, 0, st>>>(src, recv, img, fsc, N, row0, row1, nu, kfac(nu),
                                                                 2.0 * mu, lam, K64, K32);
         else
             assemble_dense_hs_kernel<false><<<grid, kTJ, 0, st>>>(src, recv, img, fsc, N, row0, row1, nu, kfac(nu),
                                                                  2.0 * mu, lam, K64, K32);
-    } else if (K32)
-        assemble_dense_kernel<true><<<grid, kTJ, 0, st>>>(src, recv, N, row0, row1, nu, kfac(nu), 2.0 * mu, lam,
-                                                         K64, K32);
+        PQ3D_CUDA_TRY(cudaGetLastError());
+        return PQ3D_OK;
+    }
+    int sms = 0;
+    const int rc = seg_config(&sms);
+    if (rc) return rc;
+    const int nr = seg_receivers(nt, row1 - row0, 2 * (int64_t)sms);
+    const SegMat mat = seg_material(nu, 2.0 * mu, lam);
+    dim3 grid((unsigned)nt, (unsigned)((row1 - row0 + nr - 1) / nr));
+    if (K32)
+        assemble_seg_kernel<true><<<grid, kSegThreads, kSegSmem, st>>>(tiles, ts, src, recv, N, row0, row1, nr, mat, nu,
+                                                                       kfac(nu), 2.0 * mu, lam, K64, K32);
     else
-        assemble_dense_kernel<false><<<grid, kTJ, 0, st>>>(src, recv, N, row0, row1, nu, kfac(nu), 2.0 * mu, lam,
-                                                          K64, K32);
+        assemble_seg_kernel<false><<<grid, kSegThreads, kSegSmem, st>>>(tiles, ts, src, recv, N, row0, row1, nr, mat,
+                                                                        nu, kfac(nu), 2.0 * mu, lam, K64, nullptr);
     PQ3D_CUDA_TRY(cudaGetLastError());
     return PQ3D_OK;
 }
 
 // ---------------------------------------------------------------------------
 // Fixed scratch for pq3d_assemble_dense_noalloc: the source and receiver
-// tables of one call (kSrcStride + kRecvStride doubles per element) for up to
-// kNoAllocMaxN elements, 14.2 MB held by every GPU that loads this library.
+// tables and the tiles of one call for up to kNoAllocMaxN elements, 19.1 MB
+// held by every GPU that loads this library.
 constexpr int64_t kNoAllocMaxN = 32768;
-static __device__ __align__(256) double g_noalloc_scratch[(size_t)(kSrcStride + kRecvStride) * kNoAllocMaxN];
+static __device__ __align__(256) double g_noalloc_scratch[(size_t)(kSrcStride + kRecvStride) * kNoAllocMaxN +
+                                                          (size_t)(kNoAllocMaxN / kTileMax) * kSegDoubles];
 
 // Device address of the fixed scratch on the current device, looked up with
 // that device current on every call (cheap): a cached address would go stale
@@ -467,7 +710,10 @@ extern "C" void TDstressFS_C1(const double *X, const double *Y, const double *Z,
 }
 
 // the size that serves both full- and half-space assemblies
-extern "C" size_t pq3d_gf_workspace_bytes(int64_t N) { return N > 0 ? ws_bytes(N, true) : 0; }
+extern "C" size_t pq3d_gf_workspace_bytes(int64_t N)
+{
+    return N > 0 ? std::max(ws_bytes(N, true), ws_bytes(N, false)) : 0;
+}
 
 extern "C" int pq3d_assemble_dense(const double *nodes, const int64_t *tris, int64_t N, int64_t row0, int64_t row1,
                                    double mu, double lambda_, int halfspace, double *K64, float *K32, void *workspace,
@@ -481,10 +727,8 @@ extern "C" int pq3d_assemble_dense(const double *nodes, const int64_t *tris, int
     PQ3D_REQUIRE(workspace_bytes >= ws_bytes(N, halfspace != 0), "pq3d_assemble_dense: workspace too small (%zu < %zu)",
                  workspace_bytes, ws_bytes(N, halfspace != 0));
     if (row0 == row1) return PQ3D_OK;
-    double *src = (double *)workspace;
-    double *recv = src + (size_t)kSrcStride * N;
-    return assemble_rows(nodes, tris, N, row0, row1, mu, lambda_, K64, K32, src, recv, true, (cudaStream_t)stream,
-                         halfspace != 0);
+    return assemble_rows(nodes, tris, N, row0, row1, mu, lambda_, K64, K32, (double *)workspace, true,
+                         (cudaStream_t)stream, halfspace != 0);
 }
 
 // Device address of page-locked host memory mapped into the device address
@@ -524,8 +768,7 @@ static int assemble_host_direct(const double *nodes_host, int64_t n_nodes, const
     PQ3D_D_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     PQ3D_D_TRY(cudaMemcpyAsync(d_nodes, nodes_host, 3 * n_nodes * sizeof(double), cudaMemcpyHostToDevice, st));
     PQ3D_D_TRY(cudaMemcpyAsync(d_tris, tris_host, 3 * N * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-    rc = assemble_rows(d_nodes, d_tris, N, 0, N, mu, lambda_, dK64, dK32, d_ws, d_ws + (size_t)kSrcStride * N, true,
-                       st, half);
+    rc = assemble_rows(d_nodes, d_tris, N, 0, N, mu, lambda_, dK64, dK32, d_ws, true, st, half);
     if (rc) goto done;
     PQ3D_D_TRY(cudaStreamSynchronize(st));
 done:
@@ -580,24 +823,16 @@ extern "C" int pq3d_assemble_dense_host(const double *nodes_host, int64_t n_node
     PQ3D_H_TRY(cudaMemcpyAsync(d_nodes, nodes_host, 3 * n_nodes * sizeof(double), cudaMemcpyHostToDevice, st[0]));
     PQ3D_H_TRY(cudaMemcpyAsync(d_tris, tris_host, 3 * N * sizeof(int64_t), cudaMemcpyHostToDevice, st[0]));
     {
-        double *src = d_ws, *recv = d_ws + (size_t)kSrcStride * N;
-        const int th = 128;
-        const unsigned nb = (unsigned)((N + th - 1) / th);
-        setup_sources_kernel<<<nb, th, 0, st[0]>>>(d_nodes, d_tris, N, src);
-        setup_receivers_kernel<<<nb, th, 0, st[0]>>>(d_nodes, d_tris, N, recv);
-        if (half) {
-            double *img = recv + (size_t)kRecvStride * N;
-            setup_hs_kernel<<<nb, th, 0, st[0]>>>(d_nodes, d_tris, N, img, img + (size_t)kImgStride * N);
-        }
-        PQ3D_H_TRY(cudaGetLastError());
+        // the tables, with no rows assembled yet
+        rc = assemble_rows(d_nodes, d_tris, N, 0, 0, mu, lambda_, nullptr, nullptr, d_ws, true, st[0], half);
+        if (rc) goto done;
         PQ3D_H_TRY(cudaEventRecord(setup_done, st[0]));
         PQ3D_H_TRY(cudaStreamWaitEvent(st[1], setup_done, 0));
         int blk = 0;
         for (int64_t r0 = 0; r0 < N; r0 += rb, ++blk) {
             const int b = blk & 1;
             const int64_t r1 = std::min<int64_t>(N, r0 + rb);
-            rc = assemble_rows(d_nodes, d_tris, N, r0, r1, mu, lambda_, d_K64[b], d_K32[b], src, recv, false, st[b],
-                               half);
+            rc = assemble_rows(d_nodes, d_tris, N, r0, r1, mu, lambda_, d_K64[b], d_K32[b], d_ws, false, st[b], half);
             if (rc) goto done;
             PQ3D_H_TRY(cudaMemcpyAsync(K64_host + 3 * r0 * ld, d_K64[b], 3 * (r1 - r0) * ld * sizeof(double),
                                        cudaMemcpyDeviceToHost, st[b]));
@@ -643,8 +878,7 @@ extern "C" int pq3d_assemble_dense_noalloc(const double *nodes, const int64_t *t
     if (row0 == row1) return PQ3D_OK;
     // every table entry the assembly reads is rewritten by this call's set-up
     // kernels, so nothing has to be cleared between calls
-    return assemble_rows(nodes, tris, N, row0, row1, mu, lambda_, K64, K32, scratch, scratch + (size_t)kSrcStride * N,
-                         true, (cudaStream_t)stream);
+    return assemble_rows(nodes, tris, N, row0, row1, mu, lambda_, K64, K32, scratch, true, (cudaStream_t)stream);
 }
 
 extern "C" int pq3d_gf_setup(const double *nodes, const int64_t *tris, int64_t N, int halfspace, void *workspace,
@@ -652,17 +886,17 @@ extern "C" int pq3d_gf_setup(const double *nodes, const int64_t *tris, int64_t N
 {
     clear_error();
     PQ3D_REQUIRE(nodes && tris && workspace && N > 0, "pq3d_gf_setup: bad arguments");
-    PQ3D_REQUIRE(workspace_bytes >= ws_bytes(N, halfspace != 0) && aligned16(workspace),
-                 "pq3d_gf_setup: workspace too small");
+    PQ3D_REQUIRE(workspace_bytes >= (halfspace ? ws_bytes(N, true)
+                                               : (size_t)N * (kSrcStride + kRecvStride + kSegStride) * sizeof(double)) &&
+                     aligned16(workspace), "pq3d_gf_setup: workspace too small");
     double *src = (double *)workspace;
     double *recv = src + (size_t)kSrcStride * N;
-    const int th = 128;
-    const unsigned nb = (unsigned)((N + th - 1) / th);
-    setup_sources_kernel<<<nb, th, 0, (cudaStream_t)stream>>>(nodes, tris, N, src);
-    setup_receivers_kernel<<<nb, th, 0, (cudaStream_t)stream>>>(nodes, tris, N, recv);
+    // full space: the edge records where the half space has its image table
+    setup_elements(nodes, tris, N, src, recv, halfspace ? nullptr : recv + (size_t)kRecvStride * N, (cudaStream_t)stream);
     if (halfspace) {
         double *img = recv + (size_t)kRecvStride * N;
-        setup_hs_kernel<<<nb, th, 0, (cudaStream_t)stream>>>(nodes, tris, N, img, img + (size_t)kImgStride * N);
+        setup_hs_kernel<<<(unsigned)((N + 127) / 128), 128, 0, (cudaStream_t)stream>>>(nodes, tris, N, img,
+                                                                                     img + (size_t)kImgStride * N);
     }
     PQ3D_CUDA_TRY(cudaGetLastError());
     return PQ3D_OK;
