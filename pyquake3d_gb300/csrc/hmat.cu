@@ -32,6 +32,7 @@
 #include "common.cuh"
 #include "gf_device.cuh"
 #include "hs_device.cuh"
+#include "seg_device.cuh"
 
 namespace pq3d {
 namespace hm {
@@ -46,75 +47,234 @@ struct GSrc {   // source fields from the global structure-of-arrays table
 
 constexpr int kThreads = 256;
 
-// The six tractions of pair (receiver record R, source element j): full
-// space, or half space (image record and free-surface side table).
+// A pair by its angular dislocations (receivers on an edge of the source).
+__device__ __noinline__ void pair_angular(const double *src, int64_t N, const double *R, double nu, double kf,
+                                          double two_mu, double lam, double ts[3], double td[3])
+{
+    pair_tractions(GSrc{src, N}, R, nu, kf, two_mu, lam, ts, td);
+}
+
+// Tractions of pair (receiver record R, source element j): full space (the
+// edge sums of seg_device.cuh; aux = edge records), or half space (aux = image
+// records, fsc = free-surface side table).  row: one traction component of
+// both slips; col: the three components of one slip (the other's work is
+// left out: ~310 and ~350 FP64 operations against 400 for all six and 520 as
+// angular dislocations).
 template <bool kHalf>
 struct PairGen {
-    const double *src, *img, *fsc;
+    const double *src, *aux, *fsc;
     int64_t N;
     double nu, kf, two_mu, lam;
+    SegMat mat;
     __device__ __forceinline__ void operator()(int64_t j, const double *R, double ts[3], double td[3]) const
     {
         if (kHalf)
-            pair_tractions_hs(GSrc{src + j, N}, GSrc{img + j, N}, GSrc{fsc + j, N}, R, nu, kf, two_mu, lam, ts, td);
-        else
-            pair_tractions(GSrc{src + j, N}, R, nu, kf, two_mu, lam, ts, td);
+            pair_tractions_hs(GSrc{src + j, N}, GSrc{aux + j, N}, GSrc{fsc + j, N}, R, nu, kf, two_mu, lam, ts, td);
+        else if (!seg_pair(GSrc{src + j, N}, GSrc{aux + j, N}, R, mat, ts, td))
+            pair_angular(src + j, N, R, nu, kf, two_mu, lam, ts, td);
+    }
+    __device__ __forceinline__ void row(int64_t j, const double *R, int c, double &ts, double &td) const
+    {
+        if (!kHalf && seg_pair_row(GSrc{src + j, N}, GSrc{aux + j, N}, R, c, mat, ts, td)) return;
+        double s[3], d[3];
+        if (kHalf) (*this)(j, R, s, d);
+        else pair_angular(src + j, N, R, nu, kf, two_mu, lam, s, d);
+        ts = s[c];
+        td = d[c];
+    }
+    __device__ __forceinline__ void col(int64_t j, const double *R, bool dip, double t[3]) const
+    {
+        if (!kHalf && seg_pair_col(GSrc{src + j, N}, GSrc{aux + j, N}, R, dip, mat, t)) return;
+        double s[3], d[3];
+        if (kHalf) (*this)(j, R, s, d);
+        else pair_angular(src + j, N, R, nu, kf, two_mu, lam, s, d);
+        for (int c = 0; c < 3; ++c) t[c] = dip ? d[c] : s[c];
     }
 };
 
-__device__ __forceinline__ void block_argmax(double v, int idx, double *sv, int *si, double &best, int &bidx)
-{
-    // max |v| with the smallest index on ties; result broadcast to all threads
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double ov = __shfl_xor_sync(0xffffffffu, v, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+// ---------------------------------------------------------------------------
+// ACA.  A block is worked on by a group of kAcaSmall threads (a quarter of a
+// CTA), by a CTA, or by a cluster of kAcaCluster CTAs; each kind only meets at
+// its own barriers, and the kinds share one launch (every cluster of CTAs takes
+// one huge block, eight large ones or thirty-two small ones).
+//
+// Bound: the FP64 pipe -- per iteration n + m pair evaluations of 310 - 350
+// operations, 2 k (M + Nc) multiply-adds for the residual row and column and
+// as many for the k cross products.  One 256-thread CTA per block in block
+// order kept the pipe 76 % busy while an SM had a block, but 49 % over the
+// launch (N = 20,000: 83 ms): most threads idled at the pivot searches of the
+// many blocks of 64 x 64 pairs, and the few largest blocks, a sixth of all
+// pairs, ran on one SM each long after the others.  Hence the three kinds, the
+// largest blocks first, 16 warps per SM and four barriers an iteration (the
+// residual, its norm and its pivot in the loop that evaluates the pairs).
+constexpr int kAcaThreads = 256;
+constexpr int kAcaSmall = 64;     // (the barrier counts of AcaGroup::sync)
+constexpr int kAcaGroups = kAcaThreads / kAcaSmall;
+constexpr int kAcaCluster = 8;
+constexpr int kAcaWarps = kAcaCluster * kAcaThreads / 32;
+// the largest side (elements) of a block for a small group: its rows and
+// columns take at most 4 rounds of the group
+constexpr int kAcaSmallSide = 256;
+// a block with more elements than the average share of kAcaSlots CTAs (two
+// per SM) would end last on one CTA: it gets a cluster, from 512 elements on
+// (below, its iterations are a round or two of a CTA)
+constexpr int kAcaSlots = 304;
+constexpr int kAcaHugeMin = 512;
+
+struct __align__(16) AcaSlot {
+    long long v;    // bits of the largest |value| (signed order: -1.0, no candidate, lies below all)
+    double s;
+    int i, pad[3];
+};
+
+struct AcaGroup {
+    int t, size, id;      // thread and threads of the group; barrier: 0 the cluster's, 1 .. 4 of the CTA
+    AcaSlot *slot;        // [2][warps of the group], in turn: one barrier per reduction
+    int turn;
+    __device__ __forceinline__ void sync() const
+    {
+        // literal barrier ids: a register id makes the CTA hold all 16 barriers
+        __syncwarp();
+        if (id == 0)
+            asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        else if (id == 1) asm volatile("barrier.sync 1, %0;" ::"r"(size) : "memory");
+        else if (id == 2) asm volatile("barrier.sync 2, 64;" ::: "memory");
+        else if (id == 3) asm volatile("barrier.sync 3, 64;" ::: "memory");
+        else asm volatile("barrier.sync 4, 64;" ::: "memory");
+    }
+    static __device__ __forceinline__ void pick(long long &v, int &idx, long long ov, int oi)
+    {
         if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
     }
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __syncthreads();
-    if (lane == 0) { sv[w] = v; si[w] = idx; }
-    __syncthreads();
-    best = sv[0];
-    bidx = si[0];
-    for (int q = 1; q < (int)(blockDim.x >> 5); ++q)
-        if (sv[q] > best || (sv[q] == best && si[q] < bidx)) { best = sv[q]; bidx = si[q]; }
-}
-
-__device__ __forceinline__ double block_sum(double v, double *sv)
-{
+    // the largest v >= 0 (or -1.0) with the smallest index on ties, and the
+    // sum of s; every thread of the group gets both, in the same order of
+    // operations.  The comparisons are integer ones (FP64 compares run on the
+    // FP64 pipe).
+    __device__ __forceinline__ void reduce(double value, int idx, double s, double &best, int &bidx, double &sum)
+    {
+        long long v = __double_as_longlong(value);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        for (int o = 16; o > 0; o >>= 1) {
+            const long long ov = __shfl_xor_sync(0xffffffffu, v, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+            pick(v, idx, ov, oi);
+        }
+        const int w = t >> 5, lane = t & 31, nw = size >> 5;
+        AcaSlot *buf = slot + (turn & 1) * nw;
+        turn ^= 1;
+        if (id != 0) {
+            if (lane == 0) buf[w] = AcaSlot{v, s, idx, {0, 0, 0}};
+        } else if (lane < kAcaCluster) {   // into this warp's slot of every CTA of the cluster
+            uint32_t at = (uint32_t)__cvta_generic_to_shared(&buf[w]);
+            asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(at) : "r"(lane));
+            asm volatile("st.shared::cluster.v2.b64 [%0], {%1, %2};" ::"r"(at), "l"(v), "l"(__double_as_longlong(s))
+                         : "memory");
+            asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(at + 16), "r"(idx) : "memory");
+        }
+        sync();
+        v = __double_as_longlong(-1.0);
+        idx = 0x7fffffff;
+        s = 0.0;
+        for (int q = lane; q < nw; q += 32) {
+            pick(v, idx, buf[q].v, buf[q].i);
+            s += buf[q].s;
+        }
+        for (int o = min(nw, 32) >> 1; o > 0; o >>= 1) {
+            const long long ov = __shfl_xor_sync(0xffffffffu, v, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+            pick(v, idx, ov, oi);
+        }
+        best = __longlong_as_double(__shfl_sync(0xffffffffu, v, 0));
+        bidx = __shfl_sync(0xffffffffu, idx, 0);
+        sum = __shfl_sync(0xffffffffu, s, 0);
+    }
+};
+
+// Work order: huge, large and small blocks, each kind by size class, the
+// largest first (a counting sort over half octaves of m + n in one CTA; the
+// order within a class does not matter).  split = {huge blocks, large blocks}.
+constexpr int kAcaClasses = 64;
+__global__ void __launch_bounds__(1024)
+aca_order_kernel(const int64_t *__restrict__ blk, int nblocks, int32_t *__restrict__ order, int32_t *__restrict__ split)
+{
+    __shared__ int count[3 * kAcaClasses];
+    __shared__ unsigned long long total;
+    const int t = threadIdx.x;
+    if (t < 3 * kAcaClasses) count[t] = 0;
+    if (t == 0) total = 0;
     __syncthreads();
-    if (lane == 0) sv[w] = v;
+    auto side_m = [&](int b) { return blk[4 * b + 1] - blk[4 * b]; };
+    auto side_n = [&](int b) { return blk[4 * b + 3] - blk[4 * b + 2]; };
+    unsigned long long mine = 0;
+    for (int b = t; b < nblocks; b += blockDim.x) mine += (unsigned long long)(side_m(b) + side_n(b));
+    atomicAdd(&total, mine);
     __syncthreads();
-    double s = 0.0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s += sv[q];
-    return s;
+    const int64_t huge = max((int64_t)kAcaHugeMin, (int64_t)(total / kAcaSlots));
+    auto cls = [&](int b) {
+        const int64_t m = side_m(b), n = side_n(b);
+        const int kind = m + n > huge ? 0 : (max(m, n) > kAcaSmallSide ? 1 : 2);
+        return kind * kAcaClasses + kAcaClasses - 1 - min(kAcaClasses - 1, (int)(2.0f * log2f((float)(m + n))));
+    };
+    for (int b = t; b < nblocks; b += blockDim.x) atomicAdd(&count[cls(b)], 1);
+    __syncthreads();
+    if (t == 0) {
+        int s = 0;
+        for (int c = 0; c < 3 * kAcaClasses; ++c) {
+            if (c == kAcaClasses) split[0] = s;
+            if (c == 2 * kAcaClasses) split[1] = s - split[0];
+            const int n = count[c];
+            count[c] = s;
+            s += n;
+        }
+    }
+    __syncthreads();
+    for (int b = t; b < nblocks; b += blockDim.x) order[atomicAdd(&count[cls(b)], 1)] = b;
 }
 
-// One CTA per admissible block.  U: kcap x M (row l = u_l), V: kcap x Nc.
-// kAcaThreads per CTA (246 registers in full space: one CTA per SM).  Other
-// shapes measured no better (N = 100,000, ACA launches: 1.28 s with 256
-// threads; 128 and 64 threads with 2 and 4 CTAs per SM 1.55 s and 2.69 s --
-// the residual updates, norms and pivot searches of an iteration scale with
-// the CTA's threads; 256 threads capped at 128 registers for 2 CTAs per SM
-// 1.34 s; 512 threads at 128 registers 1.26 s): the FP64 pipe, busy with the
-// GF evaluations of the pivot rows and columns, sets the pace.
-constexpr int kAcaThreads = 256;
-constexpr int kAcaMinBlocks = 1;
+// U: kcap x M (row l = u_l), V: kcap x Nc.  Full space: 128 registers for two
+// CTAs per SM.
 template <bool kHalf>
-__global__ void __launch_bounds__(kAcaThreads, kHalf ? 1 : kAcaMinBlocks)
+__global__ void __cluster_dims__(kAcaCluster, 1, 1) __launch_bounds__(kAcaThreads, kHalf ? 1 : 2)
 aca_kernel(PairGen<kHalf> gen, const double *__restrict__ recv, const int64_t *__restrict__ perm,
-           const int64_t *__restrict__ blk, const int32_t *__restrict__ kcap, double tol,
-           double *__restrict__ UV, const int64_t *__restrict__ uv_off,
-           uint8_t *__restrict__ used_ws, const int64_t *__restrict__ used_off, int32_t *__restrict__ rank_out,
-           int32_t *__restrict__ status_out)
+           const int64_t *__restrict__ blk, const int32_t *__restrict__ order, const int32_t *__restrict__ split,
+           int nblocks, const int32_t *__restrict__ kcap, double tol, double *__restrict__ UV,
+           const int64_t *__restrict__ uv_off, uint8_t *__restrict__ used_ws, const int64_t *__restrict__ used_off,
+           int32_t *__restrict__ rank_out, int32_t *__restrict__ status_out)
 {
-    __shared__ double sv[kAcaThreads / 32];
-    __shared__ int si[kAcaThreads / 32];
-    const int b = blockIdx.x;
+    __shared__ AcaSlot slots[2 * kAcaWarps];
+    const int nh = split[0], nl = split[1];
+    const int lc = (nl + kAcaCluster - 1) / kAcaCluster;   // clusters of large blocks
+    const int ci = blockIdx.x / kAcaCluster, cr = blockIdx.x % kAcaCluster;
+    AcaGroup g;
+    g.turn = 0;
+    g.slot = slots;
+    int pos, end;
+    if (ci < nh) {
+        g.t = cr * kAcaThreads + threadIdx.x;
+        g.size = kAcaCluster * kAcaThreads;
+        g.id = 0;
+        pos = ci;
+        end = nh;
+    } else if (ci < nh + lc) {
+        g.t = threadIdx.x;
+        g.size = kAcaThreads;
+        g.id = 1;
+        pos = nh + (ci - nh) * kAcaCluster + cr;
+        end = nh + nl;
+    } else {
+        const int q = threadIdx.x / kAcaSmall;
+        g.t = threadIdx.x % kAcaSmall;
+        g.size = kAcaSmall;
+        g.id = 1 + q;
+        g.slot = slots + 2 * q * (kAcaSmall / 32);
+        pos = nh + nl + ((ci - nh - lc) * kAcaCluster + cr) * kAcaGroups + q;
+        end = nblocks;
+    }
+    if (pos >= end) return;   // whole groups (and whole clusters) leave
+    if (g.id == 0) g.sync();  // every CTA of the cluster runs before its shared memory is written to
+    const int b = order[pos];
     const int64_t r0 = blk[4 * b], r1 = blk[4 * b + 1], c0 = blk[4 * b + 2], c1 = blk[4 * b + 3];
     const int m = (int)(r1 - r0), n = (int)(c1 - c0);
     const int M = 3 * m, Nc = 2 * n;
@@ -122,39 +282,39 @@ aca_kernel(PairGen<kHalf> gen, const double *__restrict__ recv, const int64_t *_
     double *U = UV + uv_off[b];
     double *V = U + (int64_t)K * M;
     uint8_t *used = used_ws + used_off[b];
-    const int t = threadIdx.x;
+    const int t = g.t;
     double frob2 = 0.0;
     int k = 0, istar = 0, status = 1;
     int guard = 0;
     while (k < K && guard < M + K) {
         ++guard;
+        if (t == 0) used[istar] = 1;
         // residual row istar (receiver p, component c) over all columns
         const int pr = istar / 3, cr = istar % 3;
         const double *R = recv + kRecvStride * perm[r0 + pr];
         double *v = V + (int64_t)k * Nc;
-        for (int q = t; q < n; q += kAcaThreads) {
-            double ts[3], td[3];
-            gen(perm[c0 + q], R, ts, td);
-            v[2 * q] = ts[cr];
-            v[2 * q + 1] = td[cr];
-        }
-        __syncthreads();
-        double best = 0.0;
-        int jstar = 0;
-        {
-            double mv = -1.0;
-            int mi = 0x7fffffff;
-            for (int col = t; col < Nc; col += kAcaThreads) {
-                double x = v[col];
-                for (int l = 0; l < k; ++l) x -= U[(int64_t)l * M + istar] * V[(int64_t)l * Nc + col];
-                v[col] = x;
-                const double ax = fabs(x);
-                if (ax > mv) { mv = ax; mi = col; }
+        double mv = -1.0, sum = 0.0;
+        int mi = 0x7fffffff;
+        for (int q = t; q < n; q += g.size) {
+            double xs, xd;
+            gen.row(perm[c0 + q], R, cr, xs, xd);
+            const double *Uc = U + istar, *Vc = V + 2 * q;
+#pragma unroll 4
+            for (int l = 0; l < k; ++l) {
+                const double f = Uc[(int64_t)l * M];
+                xs -= f * Vc[(int64_t)l * Nc];
+                xd -= f * Vc[(int64_t)l * Nc + 1];
             }
-            block_argmax(mv, mi, sv, si, best, jstar);
+            v[2 * q] = xs;
+            v[2 * q + 1] = xd;
+            sum += xs * xs + xd * xd;
+            const double as = fabs(xs), ad = fabs(xd);
+            if (as > mv) { mv = as; mi = 2 * q; }
+            if (ad > mv) { mv = ad; mi = 2 * q + 1; }
         }
-        if (t == 0) used[istar] = 1;
-        __syncthreads();
+        double best, nv2;
+        int jstar;
+        g.reduce(mv, mi, sum, best, jstar, nv2);
         if (!(best > 0.0) || !isfinite(best)) {
             // row represented exactly (or not finite): next unused row, no new term
             if (!isfinite(best)) { status = 2; break; }
@@ -163,43 +323,50 @@ aca_kernel(PairGen<kHalf> gen, const double *__restrict__ recv, const int64_t *_
                 if (!used[r]) { nxt = r; break; }
             if (nxt < 0) { status = 0; break; }
             istar = nxt;
+            g.sync();   // every thread has looked before the row is marked
             continue;
         }
-        const double pivot = v[jstar];
+        const double pivot = v[jstar], ipiv = 1.0 / pivot;
+        const bool recip = isfinite(ipiv);
         // residual column jstar (source q, slip s) over all rows, scaled by the pivot
         const int qc = jstar / 2, sc = jstar % 2;
         const int64_t jb = perm[c0 + qc];
         double *u = U + (int64_t)k * M;
-        for (int p = t; p < m; p += kAcaThreads) {
-            double ts[3], td[3];
-            gen(jb, recv + kRecvStride * perm[r0 + p], ts, td);
-            const double *tt = sc ? td : ts;
-            u[3 * p] = tt[0];
-            u[3 * p + 1] = tt[1];
-            u[3 * p + 2] = tt[2];
+        mv = -1.0;
+        mi = 0x7fffffff;
+        double nu2 = 0.0;
+        for (int p = t; p < m; p += g.size) {
+            double x[3];
+            gen.col(jb, recv + kRecvStride * perm[r0 + p], sc != 0, x);
+            const double *Uc = U + 3 * p, *Vc = V + jstar;
+#pragma unroll 4
+            for (int l = 0; l < k; ++l) {
+                const double f = Vc[(int64_t)l * Nc];
+                x[0] -= f * Uc[(int64_t)l * M];
+                x[1] -= f * Uc[(int64_t)l * M + 1];
+                x[2] -= f * Uc[(int64_t)l * M + 2];
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double y = recip ? x[c] * ipiv : x[c] / pivot, ay = fabs(y);
+                u[3 * p + c] = y;
+                nu2 += y * y;
+                if (ay > mv && !used[3 * p + c]) { mv = ay; mi = 3 * p + c; }   // largest |u| among unused rows
+            }
         }
-        __syncthreads();
-        for (int row = t; row < M; row += kAcaThreads) {
-            double x = u[row];
-            for (int l = 0; l < k; ++l) x -= V[(int64_t)l * Nc + jstar] * U[(int64_t)l * M + row];
-            u[row] = x / pivot;
-        }
-        __syncthreads();
-        // norms: |S_k|^2 = |S_{k-1}|^2 + 2 sum_l (u.u_l)(v.v_l) + |u|^2 |v|^2
-        double nu2 = 0.0, nv2 = 0.0;
-        for (int row = t; row < M; row += kAcaThreads) nu2 += u[row] * u[row];
-        for (int col = t; col < Nc; col += kAcaThreads) nv2 += v[col] * v[col];
-        nu2 = block_sum(nu2, sv);
-        nv2 = block_sum(nv2, sv);
-        // the k cross products (u.u_l)(v.v_l): one warp per term l (warp
-        // shuffles, no block barrier), then one block sum of the warps' parts
+        g.sync();
+        // |S_k|^2 = |S_{k-1}|^2 + 2 sum_l (u.u_l)(v.v_l) + |u|^2 |v|^2: the k
+        // cross products one warp per term l, the sum with the others' reduction
         double cross_w = 0.0;
         {
-            const int w = t >> 5, lane = t & 31;
-            for (int l = w; l < k; l += kAcaThreads / 32) {
+            const int lane = t & 31;
+            for (int l = t >> 5; l < k; l += g.size >> 5) {
                 double du = 0.0, dv = 0.0;
-                for (int row = lane; row < M; row += 32) du += u[row] * U[(int64_t)l * M + row];
-                for (int col = lane; col < Nc; col += 32) dv += v[col] * V[(int64_t)l * Nc + col];
+                const double *Ul = U + (int64_t)l * M, *Vl = V + (int64_t)l * Nc;
+#pragma unroll 4
+                for (int row = lane; row < M; row += 32) du += u[row] * Ul[row];
+#pragma unroll 4
+                for (int col = lane; col < Nc; col += 32) dv += v[col] * Vl[col];
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
                     du += __shfl_xor_sync(0xffffffffu, du, o);
@@ -208,22 +375,15 @@ aca_kernel(PairGen<kHalf> gen, const double *__restrict__ recv, const int64_t *_
                 cross_w += du * dv;
             }
         }
-        const double cross = block_sum((t & 31) == 0 ? cross_w : 0.0, sv);
+        double bv, cross, skip;
+        int bi, sbi;
+        g.reduce(mv, mi, nu2, bv, bi, nu2);
+        g.reduce(-1.0, 0, (t & 31) == 0 ? cross_w : 0.0, skip, sbi, cross);
         frob2 += 2.0 * cross + nu2 * nv2;
         ++k;
         if (sqrt(nu2 * nv2) <= tol * sqrt(fmax(frob2, 0.0))) { status = 0; break; }
-        // next pivot row: largest |u| among unused rows
-        double mv = -1.0;
-        int mi = 0x7fffffff;
-        for (int row = t; row < M; row += kAcaThreads) {
-            const double ax = fabs(u[row]);
-            if (!used[row] && ax > mv) { mv = ax; mi = row; }
-        }
-        double bv;
-        int bi;
-        block_argmax(mv, mi, sv, si, bv, bi);
         if (bv < 0.0) { status = 0; break; }   // every row used: exact
-        istar = bi;
+        istar = bi;   // the next pivot row
     }
     if (t == 0) {
         rank_out[b] = k;
@@ -680,14 +840,15 @@ using namespace pq3d::hm;
 static inline double poisson_(double mu, double lam) { return 1.0 / (1.0 + lam / mu) / 2.0; }
 
 // Table layout written by pq3d_gf_setup: source [kSrcStride][N], receiver
-// [N][kRecvStride], image [kImgStride][N], side table [kFscStride][N].
+// [N][kRecvStride], then full space: edge records [kSegStride][N]; half space:
+// image [kImgStride][N], side table [kFscStride][N].
 template <bool kHalf>
 static PairGen<kHalf> make_gen(const double *tables, int64_t N, double mu, double lambda_)
 {
     const double nu = poisson_(mu, lambda_);
-    const double *img = tables + (size_t)(kSrcStride + kRecvStride) * N;
-    return PairGen<kHalf>{tables, img, img + (size_t)kImgStride * N, N, nu, 1.0 / (8.0 * kPi * (1.0 - nu)),
-                          2.0 * mu, lambda_};
+    const double *aux = tables + (size_t)(kSrcStride + kRecvStride) * N;
+    return PairGen<kHalf>{tables, aux, aux + (size_t)kImgStride * N, N, nu, 1.0 / (8.0 * kPi * (1.0 - nu)),
+                          2.0 * mu, lambda_, seg_material(nu, 2.0 * mu, lambda_)};
 }
 
 extern "C" int pq3d_hmat_aca(const double *tables, int64_t N, const int64_t *perm, int nblocks, const int64_t *blk,
@@ -701,13 +862,25 @@ extern "C" int pq3d_hmat_aca(const double *tables, int64_t N, const int64_t *per
     if (nblocks <= 0) return PQ3D_OK;
     const double *recv = tables + (size_t)kSrcStride * N;
     cudaStream_t st = (cudaStream_t)stream;
+    // the work order lives for this launch only (stream-ordered scratch); a
+    // grid of nblocks clusters serves any split, those past the last block leave
+    PQ3D_REQUIRE(nblocks <= INT32_MAX / kAcaCluster, "pq3d_hmat_aca: too many blocks");
+    int32_t *split = nullptr;
+    PQ3D_CUDA_TRY(cudaMallocAsync(&split, ((size_t)nblocks + 2) * sizeof(int32_t), st));
+    int32_t *order = split + 2;
+    const unsigned grid = (unsigned)nblocks * kAcaCluster;
+    aca_order_kernel<<<1, 1024, 0, st>>>(blk, nblocks, order, split);
     if (halfspace)
-        aca_kernel<true><<<nblocks, kAcaThreads, 0, st>>>(make_gen<true>(tables, N, mu, lambda_), recv, perm, blk, kcap,
-                                                       tol, UV, uv_off, used, used_off, rank, status);
+        aca_kernel<true><<<grid, kAcaThreads, 0, st>>>(make_gen<true>(tables, N, mu, lambda_), recv, perm, blk, order,
+                                                       split, nblocks, kcap, tol, UV, uv_off, used, used_off, rank,
+                                                       status);
     else
-        aca_kernel<false><<<nblocks, kAcaThreads, 0, st>>>(make_gen<false>(tables, N, mu, lambda_), recv, perm, blk,
-                                                        kcap, tol, UV, uv_off, used, used_off, rank, status);
-    PQ3D_CUDA_TRY(cudaGetLastError());
+        aca_kernel<false><<<grid, kAcaThreads, 0, st>>>(make_gen<false>(tables, N, mu, lambda_), recv, perm, blk, order,
+                                                        split, nblocks, kcap, tol, UV, uv_off, used, used_off, rank,
+                                                        status);
+    const cudaError_t launched = cudaGetLastError();
+    PQ3D_CUDA_TRY(cudaFreeAsync(split, st));
+    PQ3D_CUDA_TRY(launched);
     return PQ3D_OK;
 }
 
