@@ -59,8 +59,7 @@ __device__ __forceinline__ void load_triangle(const double *__restrict__ nodes, 
 // Source and receiver records of element j, in one launch: blocks [0, nb) the
 // sources, [nb, 2 nb) the receivers (both are short chains of FP64 latency).
 __global__ void setup_elements_kernel(const double *__restrict__ nodes, const int64_t *__restrict__ tris, int64_t N,
-                                      unsigned nb, double *__restrict__ src, double *__restrict__ recv,
-                                      double *__restrict__ seg)
+                                      unsigned nb, double *__restrict__ src, double *__restrict__ recv)
 {
     const bool source = blockIdx.x < nb;
     const int64_t j = (blockIdx.x - (source ? 0u : nb)) * (int64_t)blockDim.x + threadIdx.x;
@@ -69,7 +68,6 @@ __global__ void setup_elements_kernel(const double *__restrict__ nodes, const in
     load_triangle(nodes, tris, j, a, b, c);
     if (source) setup_source(a, b, c, src + j, (int)N);
     else setup_receiver(a, b, c, recv + kRecvStride * j);
-    if (!source && seg) setup_seg(a, b, c, seg + j, N);
 }
 
 // ---------------------------------------------------------------------------
@@ -546,10 +544,10 @@ static size_t ws_bytes(int64_t N, bool half)
 }
 
 static void setup_elements(const double *nodes, const int64_t *tris, int64_t N, double *src, double *recv,
-                           double *seg, cudaStream_t st)
+                           cudaStream_t st)
 {
     const unsigned nb = (unsigned)((N + 127) / 128);
-    setup_elements_kernel<<<2 * nb, 128, 0, st>>>(nodes, tris, N, nb, src, recv, seg);
+    setup_elements_kernel<<<2 * nb, 128, 0, st>>>(nodes, tris, N, nb, src, recv);
 }
 
 // Receivers per block: the grid's tail costs up to one block's time, so the
@@ -600,7 +598,7 @@ static int assemble_rows(const double *nodes, const int64_t *tris, int64_t N, in
     const int64_t nt = (N + ts - 1) / ts;
     if (do_setup) {
         const int th = 128;
-        setup_elements(nodes, tris, N, src, recv, nullptr, st);
+        setup_elements(nodes, tris, N, src, recv, st);
         if (half) setup_hs_kernel<<<(unsigned)((N + th - 1) / th), th, 0, st>>>(nodes, tris, N, img, fsc);
         else setup_tiles_kernel<<<(unsigned)nt, kTileMax, 0, st>>>(nodes, tris, N, ts, tiles);
         PQ3D_CUDA_TRY(cudaGetLastError());
@@ -887,12 +885,11 @@ extern "C" int pq3d_gf_setup(const double *nodes, const int64_t *tris, int64_t N
     clear_error();
     PQ3D_REQUIRE(nodes && tris && workspace && N > 0, "pq3d_gf_setup: bad arguments");
     PQ3D_REQUIRE(workspace_bytes >= (halfspace ? ws_bytes(N, true)
-                                               : (size_t)N * (kSrcStride + kRecvStride + kSegStride) * sizeof(double)) &&
+                                               : (size_t)N * (kSrcStride + kRecvStride) * sizeof(double)) &&
                      aligned16(workspace), "pq3d_gf_setup: workspace too small");
     double *src = (double *)workspace;
     double *recv = src + (size_t)kSrcStride * N;
-    // full space: the edge records where the half space has its image table
-    setup_elements(nodes, tris, N, src, recv, halfspace ? nullptr : recv + (size_t)kRecvStride * N, (cudaStream_t)stream);
+    setup_elements(nodes, tris, N, src, recv, (cudaStream_t)stream);
     if (halfspace) {
         double *img = recv + (size_t)kRecvStride * N;
         setup_hs_kernel<<<(unsigned)((N + 127) / 128), 128, 0, (cudaStream_t)stream>>>(nodes, tris, N, img,

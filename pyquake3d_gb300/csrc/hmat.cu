@@ -32,7 +32,6 @@
 #include "common.cuh"
 #include "gf_device.cuh"
 #include "hs_device.cuh"
-#include "seg_device.cuh"
 
 namespace pq3d {
 namespace hm {
@@ -47,58 +46,29 @@ struct GSrc {   // source fields from the global structure-of-arrays table
 
 constexpr int kThreads = 256;
 
-// A pair by its angular dislocations (receivers on an edge of the source).
-__device__ __noinline__ void pair_angular(const double *src, int64_t N, const double *R, double nu, double kf,
-                                          double two_mu, double lam, double ts[3], double td[3])
-{
-    pair_tractions(GSrc{src, N}, R, nu, kf, two_mu, lam, ts, td);
-}
-
-// Tractions of pair (receiver record R, source element j): full space (the
-// edge sums of seg_device.cuh; aux = edge records), or half space (aux = image
-// records, fsc = free-surface side table).  row: one traction component of
-// both slips; col: the three components of one slip (the other's work is
-// left out: ~310 and ~350 FP64 operations against 400 for all six and 520 as
-// angular dislocations).
+// The six tractions of pair (receiver record R, source element j): full
+// space, or half space (image record and free-surface side table).
 template <bool kHalf>
 struct PairGen {
-    const double *src, *aux, *fsc;
+    const double *src, *img, *fsc;
     int64_t N;
     double nu, kf, two_mu, lam;
-    SegMat mat;
     __device__ __forceinline__ void operator()(int64_t j, const double *R, double ts[3], double td[3]) const
     {
         if (kHalf)
-            pair_tractions_hs(GSrc{src + j, N}, GSrc{aux + j, N}, GSrc{fsc + j, N}, R, nu, kf, two_mu, lam, ts, td);
-        else if (!seg_pair(GSrc{src + j, N}, GSrc{aux + j, N}, R, mat, ts, td))
-            pair_angular(src + j, N, R, nu, kf, two_mu, lam, ts, td);
-    }
-    __device__ __forceinline__ void row(int64_t j, const double *R, int c, double &ts, double &td) const
-    {
-        if (!kHalf && seg_pair_row(GSrc{src + j, N}, GSrc{aux + j, N}, R, c, mat, ts, td)) return;
-        double s[3], d[3];
-        if (kHalf) (*this)(j, R, s, d);
-        else pair_angular(src + j, N, R, nu, kf, two_mu, lam, s, d);
-        ts = s[c];
-        td = d[c];
-    }
-    __device__ __forceinline__ void col(int64_t j, const double *R, bool dip, double t[3]) const
-    {
-        if (!kHalf && seg_pair_col(GSrc{src + j, N}, GSrc{aux + j, N}, R, dip, mat, t)) return;
-        double s[3], d[3];
-        if (kHalf) (*this)(j, R, s, d);
-        else pair_angular(src + j, N, R, nu, kf, two_mu, lam, s, d);
-        for (int c = 0; c < 3; ++c) t[c] = dip ? d[c] : s[c];
+            pair_tractions_hs(GSrc{src + j, N}, GSrc{img + j, N}, GSrc{fsc + j, N}, R, nu, kf, two_mu, lam, ts, td);
+        else
+            pair_tractions(GSrc{src + j, N}, R, nu, kf, two_mu, lam, ts, td);
     }
 };
 
 // ---------------------------------------------------------------------------
 // ACA.  A block is worked on by a group of kAcaSmall threads (a quarter of a
 // CTA), by a CTA, or by a cluster of kAcaCluster CTAs; each kind only meets at
-// its own barriers, and the kinds share one launch (every cluster of CTAs takes
-// one huge block, eight large ones or thirty-two small ones).
+// its own barriers.  The clusters are one launch, the rest another beside it
+// (clusters alone leave the SMs of a GPC that make no eighth idle).
 //
-// Bound: the FP64 pipe -- per iteration n + m pair evaluations of 310 - 350
+// Bound: the FP64 pipe -- per iteration n + m pair evaluations of 520
 // operations, 2 k (M + Nc) multiply-adds for the residual row and column and
 // as many for the k cross products.  One 256-thread CTA per block in block
 // order kept the pipe 76 % busy while an SM had a block, but 49 % over the
@@ -112,14 +82,15 @@ constexpr int kAcaSmall = 64;     // (the barrier counts of AcaGroup::sync)
 constexpr int kAcaGroups = kAcaThreads / kAcaSmall;
 constexpr int kAcaCluster = 8;
 constexpr int kAcaWarps = kAcaCluster * kAcaThreads / 32;
-// the largest side (elements) of a block for a small group: its rows and
-// columns take at most 4 rounds of the group
+// A block with more elements (m + n) than the average share of kAcaSlots CTAs
+// (one per SM) would end last on one CTA: it gets a cluster, from 256 elements
+// on.  A small group is for blocks of at most kAcaSmallSide elements a side
+// (four rounds of the group) and of at most the share of a group's slot: with
+// few blocks (N = 3,600: 216) the SMs would idle while groups of 64 threads
+// walk 256-element sides.
 constexpr int kAcaSmallSide = 256;
-// a block with more elements than the average share of kAcaSlots CTAs (two
-// per SM) would end last on one CTA: it gets a cluster, from 512 elements on
-// (below, its iterations are a round or two of a CTA)
-constexpr int kAcaSlots = 304;
-constexpr int kAcaHugeMin = 512;
+constexpr int kAcaSlots = 152;
+constexpr int kAcaHugeMin = 256;
 
 struct __align__(16) AcaSlot {
     long long v;    // bits of the largest |value| (signed order: -1.0, no candidate, lies below all)
@@ -212,9 +183,10 @@ aca_order_kernel(const int64_t *__restrict__ blk, int nblocks, int32_t *__restri
     atomicAdd(&total, mine);
     __syncthreads();
     const int64_t huge = max((int64_t)kAcaHugeMin, (int64_t)(total / kAcaSlots));
+    const int64_t small = (int64_t)(total / (kAcaSlots * kAcaGroups));
     auto cls = [&](int b) {
         const int64_t m = side_m(b), n = side_n(b);
-        const int kind = m + n > huge ? 0 : (max(m, n) > kAcaSmallSide ? 1 : 2);
+        const int kind = m + n > huge ? 0 : (max(m, n) > kAcaSmallSide || m + n > small ? 1 : 2);
         return kind * kAcaClasses + kAcaClasses - 1 - min(kAcaClasses - 1, (int)(2.0f * log2f((float)(m + n))));
     };
     for (int b = t; b < nblocks; b += blockDim.x) atomicAdd(&count[cls(b)], 1);
@@ -233,11 +205,14 @@ aca_order_kernel(const int64_t *__restrict__ blk, int nblocks, int32_t *__restri
     for (int b = t; b < nblocks; b += blockDim.x) order[atomicAdd(&count[cls(b)], 1)] = b;
 }
 
-// U: kcap x M (row l = u_l), V: kcap x Nc.  Full space: 128 registers for two
-// CTAs per SM.
+// U: kcap x M (row l = u_l), V: kcap x Nc.  One CTA per SM: at 128 registers for
+// two, the compiler contracts the pair's products differently, and the last
+// terms of a block, 1e-4 of its size, carry such a change of 1e-16 into 1e-11 of
+// the product (two CTAs: 102 instead of 110 ms at N = 30,000).
+// clusters: this launch is one of clusters, for the huge blocks.
 template <bool kHalf>
-__global__ void __cluster_dims__(kAcaCluster, 1, 1) __launch_bounds__(kAcaThreads, kHalf ? 1 : 2)
-aca_kernel(PairGen<kHalf> gen, const double *__restrict__ recv, const int64_t *__restrict__ perm,
+__global__ void __launch_bounds__(kAcaThreads, 1)
+aca_kernel(bool clusters, PairGen<kHalf> gen, const double *__restrict__ recv, const int64_t *__restrict__ perm,
            const int64_t *__restrict__ blk, const int32_t *__restrict__ order, const int32_t *__restrict__ split,
            int nblocks, const int32_t *__restrict__ kcap, double tol, double *__restrict__ UV,
            const int64_t *__restrict__ uv_off, uint8_t *__restrict__ used_ws, const int64_t *__restrict__ used_off,
@@ -245,23 +220,21 @@ aca_kernel(PairGen<kHalf> gen, const double *__restrict__ recv, const int64_t *_
 {
     __shared__ AcaSlot slots[2 * kAcaWarps];
     const int nh = split[0], nl = split[1];
-    const int lc = (nl + kAcaCluster - 1) / kAcaCluster;   // clusters of large blocks
-    const int ci = blockIdx.x / kAcaCluster, cr = blockIdx.x % kAcaCluster;
     AcaGroup g;
     g.turn = 0;
     g.slot = slots;
-    int pos, end;
-    if (ci < nh) {
-        g.t = cr * kAcaThreads + threadIdx.x;
+    int pos = blockIdx.x, end;
+    if (clusters) {
+        g.t = (pos % kAcaCluster) * kAcaThreads + threadIdx.x;
         g.size = kAcaCluster * kAcaThreads;
         g.id = 0;
-        pos = ci;
+        pos /= kAcaCluster;
         end = nh;
-    } else if (ci < nh + lc) {
+    } else if (pos < nl) {
         g.t = threadIdx.x;
         g.size = kAcaThreads;
         g.id = 1;
-        pos = nh + (ci - nh) * kAcaCluster + cr;
+        pos += nh;
         end = nh + nl;
     } else {
         const int q = threadIdx.x / kAcaSmall;
@@ -269,7 +242,7 @@ aca_kernel(PairGen<kHalf> gen, const double *__restrict__ recv, const int64_t *_
         g.size = kAcaSmall;
         g.id = 1 + q;
         g.slot = slots + 2 * q * (kAcaSmall / 32);
-        pos = nh + nl + ((ci - nh - lc) * kAcaCluster + cr) * kAcaGroups + q;
+        pos = nh + nl + (pos - nl) * kAcaGroups + q;
         end = nblocks;
     }
     if (pos >= end) return;   // whole groups (and whole clusters) leave
@@ -296,10 +269,15 @@ aca_kernel(PairGen<kHalf> gen, const double *__restrict__ recv, const int64_t *_
         double mv = -1.0, sum = 0.0;
         int mi = 0x7fffffff;
         for (int q = t; q < n; q += g.size) {
-            double xs, xd;
-            gen.row(perm[c0 + q], R, cr, xs, xd);
+            double ts[3], td[3];
+            gen(perm[c0 + q], R, ts, td);
+            v[2 * q] = ts[cr];
+            v[2 * q + 1] = td[cr];
+        }
+        for (int q = t; q < n; q += g.size) {   // this thread's own columns: no barrier
+            double xs = v[2 * q], xd = v[2 * q + 1];
             const double *Uc = U + istar, *Vc = V + 2 * q;
-#pragma unroll 4
+#pragma unroll 8
             for (int l = 0; l < k; ++l) {
                 const double f = Uc[(int64_t)l * M];
                 xs -= f * Vc[(int64_t)l * Nc];
@@ -326,8 +304,7 @@ aca_kernel(PairGen<kHalf> gen, const double *__restrict__ recv, const int64_t *_
             g.sync();   // every thread has looked before the row is marked
             continue;
         }
-        const double pivot = v[jstar], ipiv = 1.0 / pivot;
-        const bool recip = isfinite(ipiv);
+        const double pivot = v[jstar];
         // residual column jstar (source q, slip s) over all rows, scaled by the pivot
         const int qc = jstar / 2, sc = jstar % 2;
         const int64_t jb = perm[c0 + qc];
@@ -336,10 +313,17 @@ aca_kernel(PairGen<kHalf> gen, const double *__restrict__ recv, const int64_t *_
         mi = 0x7fffffff;
         double nu2 = 0.0;
         for (int p = t; p < m; p += g.size) {
-            double x[3];
-            gen.col(jb, recv + kRecvStride * perm[r0 + p], sc != 0, x);
+            double ts[3], td[3];
+            gen(jb, recv + kRecvStride * perm[r0 + p], ts, td);
+            const double *tt = sc ? td : ts;
+            u[3 * p] = tt[0];
+            u[3 * p + 1] = tt[1];
+            u[3 * p + 2] = tt[2];
+        }
+        for (int p = t; p < m; p += g.size) {   // this thread's own rows
+            double x[3] = {u[3 * p], u[3 * p + 1], u[3 * p + 2]};
             const double *Uc = U + 3 * p, *Vc = V + jstar;
-#pragma unroll 4
+#pragma unroll 8
             for (int l = 0; l < k; ++l) {
                 const double f = Vc[(int64_t)l * Nc];
                 x[0] -= f * Uc[(int64_t)l * M];
@@ -348,7 +332,7 @@ aca_kernel(PairGen<kHalf> gen, const double *__restrict__ recv, const int64_t *_
             }
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const double y = recip ? x[c] * ipiv : x[c] / pivot, ay = fabs(y);
+                const double y = x[c] / pivot, ay = fabs(y);
                 u[3 * p + c] = y;
                 nu2 += y * y;
                 if (ay > mv && !used[3 * p + c]) { mv = ay; mi = 3 * p + c; }   // largest |u| among unused rows
@@ -840,15 +824,43 @@ using namespace pq3d::hm;
 static inline double poisson_(double mu, double lam) { return 1.0 / (1.0 + lam / mu) / 2.0; }
 
 // Table layout written by pq3d_gf_setup: source [kSrcStride][N], receiver
-// [N][kRecvStride], then full space: edge records [kSegStride][N]; half space:
-// image [kImgStride][N], side table [kFscStride][N].
+// [N][kRecvStride], image [kImgStride][N], side table [kFscStride][N].
 template <bool kHalf>
 static PairGen<kHalf> make_gen(const double *tables, int64_t N, double mu, double lambda_)
 {
     const double nu = poisson_(mu, lambda_);
-    const double *aux = tables + (size_t)(kSrcStride + kRecvStride) * N;
-    return PairGen<kHalf>{tables, aux, aux + (size_t)kImgStride * N, N, nu, 1.0 / (8.0 * kPi * (1.0 - nu)),
-                          2.0 * mu, lambda_, seg_material(nu, 2.0 * mu, lambda_)};
+    const double *img = tables + (size_t)(kSrcStride + kRecvStride) * N;
+    return PairGen<kHalf>{tables, img, img + (size_t)kImgStride * N, N, nu, 1.0 / (8.0 * kPi * (1.0 - nu)),
+                          2.0 * mu, lambda_};
+}
+
+// The second stream of an ACA call and the events that fork it off the
+// caller's stream and join it again; one set per host thread and device.
+struct AcaFork {
+    int device = -1;
+    cudaStream_t stream = nullptr;
+    cudaEvent_t begin = nullptr, end = nullptr;
+};
+
+static int aca_fork(AcaFork **out)
+{
+    static thread_local AcaFork f;
+    int dev;
+    PQ3D_CUDA_TRY(cudaGetDevice(&dev));
+    if (f.device != dev) {
+        if (f.device >= 0) {   // another device before: its set goes
+            cudaStreamDestroy(f.stream);
+            cudaEventDestroy(f.begin);
+            cudaEventDestroy(f.end);
+            f = AcaFork();
+        }
+        PQ3D_CUDA_TRY(cudaStreamCreateWithFlags(&f.stream, cudaStreamNonBlocking));
+        PQ3D_CUDA_TRY(cudaEventCreateWithFlags(&f.begin, cudaEventDisableTiming));
+        PQ3D_CUDA_TRY(cudaEventCreateWithFlags(&f.end, cudaEventDisableTiming));
+        f.device = dev;
+    }
+    *out = &f;
+    return PQ3D_OK;
 }
 
 extern "C" int pq3d_hmat_aca(const double *tables, int64_t N, const int64_t *perm, int nblocks, const int64_t *blk,
@@ -862,23 +874,42 @@ extern "C" int pq3d_hmat_aca(const double *tables, int64_t N, const int64_t *per
     if (nblocks <= 0) return PQ3D_OK;
     const double *recv = tables + (size_t)kSrcStride * N;
     cudaStream_t st = (cudaStream_t)stream;
-    // the work order lives for this launch only (stream-ordered scratch); a
-    // grid of nblocks clusters serves any split, those past the last block leave
+    // the work order lives for this call only (stream-ordered scratch); grids
+    // of nblocks clusters and CTAs serve any split, those past the last leave
     PQ3D_REQUIRE(nblocks <= INT32_MAX / kAcaCluster, "pq3d_hmat_aca: too many blocks");
+    AcaFork *fork;
+    int rc = aca_fork(&fork);
+    if (rc) return rc;
     int32_t *split = nullptr;
     PQ3D_CUDA_TRY(cudaMallocAsync(&split, ((size_t)nblocks + 2) * sizeof(int32_t), st));
-    int32_t *order = split + 2;
-    const unsigned grid = (unsigned)nblocks * kAcaCluster;
-    aca_order_kernel<<<1, 1024, 0, st>>>(blk, nblocks, order, split);
-    if (halfspace)
-        aca_kernel<true><<<grid, kAcaThreads, 0, st>>>(make_gen<true>(tables, N, mu, lambda_), recv, perm, blk, order,
-                                                       split, nblocks, kcap, tol, UV, uv_off, used, used_off, rank,
-                                                       status);
-    else
-        aca_kernel<false><<<grid, kAcaThreads, 0, st>>>(make_gen<false>(tables, N, mu, lambda_), recv, perm, blk, order,
-                                                        split, nblocks, kcap, tol, UV, uv_off, used, used_off, rank,
-                                                        status);
-    const cudaError_t launched = cudaGetLastError();
+    aca_order_kernel<<<1, 1024, 0, st>>>(blk, nblocks, split + 2, split);
+    auto launch = [&](auto kernel, auto gen) -> cudaError_t {
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = kAcaCluster;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)nblocks * kAcaCluster);
+        cfg.blockDim = dim3(kAcaThreads);
+        cfg.stream = st;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        cudaError_t e = cudaEventRecord(fork->begin, st);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(fork->stream, fork->begin, 0);
+        if (e == cudaSuccess)
+            e = cudaLaunchKernelEx(&cfg, kernel, true, gen, recv, perm, blk, (const int32_t *)(split + 2),
+                                   (const int32_t *)split, nblocks, kcap, tol, UV, uv_off, used, used_off, rank, status);
+        if (e != cudaSuccess) return e;
+        kernel<<<nblocks, kAcaThreads, 0, fork->stream>>>(false, gen, recv, perm, blk, split + 2, split, nblocks, kcap,
+                                                          tol, UV, uv_off, used, used_off, rank, status);
+        e = cudaGetLastError();
+        // joined whatever happened: a capturing stream must not be left forked
+        const cudaError_t e1 = cudaEventRecord(fork->end, fork->stream);
+        const cudaError_t e2 = cudaStreamWaitEvent(st, fork->end, 0);
+        return e != cudaSuccess ? e : (e1 != cudaSuccess ? e1 : e2);
+    };
+    const cudaError_t launched = halfspace ? launch(aca_kernel<true>, make_gen<true>(tables, N, mu, lambda_))
+                                           : launch(aca_kernel<false>, make_gen<false>(tables, N, mu, lambda_));
     PQ3D_CUDA_TRY(cudaFreeAsync(split, st));
     PQ3D_CUDA_TRY(launched);
     return PQ3D_OK;

@@ -216,144 +216,5 @@ __device__ __forceinline__ bool seg_bad(double t)
 #endif
 }
 
-// One row of that matrix: the normal traction, or that along e1.
-__device__ __forceinline__ void seg_row(const SegTerms &s, double kap, double ci, bool normal, double m[3])
-{
-    const double hz = kap * s.gz;
-    const double m02 = s.tz * s.gy + s.ty * hz;
-    if (normal) {
-        const double qz = s.dz * s.al + (s.tz * s.be + ci * s.i30);
-        m[0] = qz * s.ux - 2.0 * m02;
-        m[1] = qz * s.uy + 2.0 * (s.tz * s.gx + s.tx * hz);
-        m[2] = qz * s.uz;
-    } else {
-        const double qx = s.dx * s.al + s.tx * s.be, hx = kap * s.gx;
-        m[0] = qx * s.ux - (s.tx * s.gy + s.ty * hx);
-        m[1] = qx * s.uy + (s.tx * (s.gx + hx) - s.tz * (s.gz + hz));
-        m[2] = qx * s.uz + m02;
-    }
-    if (s.on) m[0] = seg_nan();
-}
-
-// T += M b.
-__device__ __forceinline__ void seg_apply(const SegTerms &s, double kap, double ci, const double b[3], double T[3])
-{
-    const double ax = s.gy * b[2] - s.gz * b[1], ay = s.gz * b[0] - s.gx * b[2], az = s.gx * b[1] - s.gy * b[0];
-    const double hx = kap * s.gx, hy = kap * s.gy, hz = kap * s.gz;
-    const double cx = b[1] * s.tz - b[2] * s.ty, cy = b[2] * s.tx - b[0] * s.tz, cz = b[0] * s.ty - b[1] * s.tx;
-    double f = b[0] * s.ux + b[1] * s.uy + b[2] * s.uz;
-    if (s.on) f = seg_nan();
-    const double fa = f * s.al, fb = f * s.be;
-    T[0] += (ax * s.tz + s.tx * az) - (cx * hz + hx * cz) + (s.dx * fa + s.tx * fb);
-    T[1] += (ay * s.tz + s.ty * az) - (cy * hz + hy * cz) + (s.dy * fa + s.ty * fb);
-    T[2] += 2.0 * (az * s.tz - cz * hz) + (s.dz * fa + (s.tz * fb + ci * (s.i30 * f)));
-}
-
-// Per-source record of the pair form below ([kSegStride][N]): vertices 1 and
-// 3, and length and reciprocal of the edges P1 P2, P2 P3, P3 P1; vertex 2 and
-// the slip axes are in the source record.
-constexpr int kSegStride = 12;
-
-__host__ __device__ inline void setup_seg(const double P1[3], const double P2[3], const double P3[3], double *f,
-                                          int64_t fstride)
-{
-    const SegEdge e[3] = {seg_edge_record(P1, P2), seg_edge_record(P2, P3), seg_edge_record(P3, P1)};
-    for (int q = 0; q < 3; ++q) {
-        f[q * fstride] = P1[q];
-        f[(3 + q) * fstride] = P3[q];
-        f[(6 + 2 * q) * fstride] = e[q].L;
-        f[(7 + 2 * q) * fstride] = e[q].iL;
-    }
-}
-
-// f(k, terms of edge k) for the three edges of the source F (source record)
-// with seg record G, seen from the receiver R.
-template <class Src, class Fn>
-__device__ __forceinline__ void seg_edges(const Src &F, const Src &G, const double *R, double kap, Fn f)
-{
-    const SegVert v1 = seg_vertex(R, G(0), G(1), G(2)), v2 = seg_vertex(R, F(F_P2X), F(F_P2Y), F(F_P2Z)),
-                  v3 = seg_vertex(R, G(3), G(4), G(5));
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const double L = G(6 + 2 * k);
-        f(seg_terms(k == 0 ? v1 : (k == 1 ? v2 : v3), k == 0 ? v2 : (k == 1 ? v3 : v1), L, G(7 + 2 * k),
-                    1e-12f * seg_small(L * L), kap));
-    }
-}
-
-// The six tractions of a pair (pair_tractions' arguments and results); false
-// where the pair has to go there.
-template <class Src>
-__device__ __forceinline__ bool seg_pair(const Src &F, const Src &G, const double *R, const SegMat &m, double ts[3],
-                                         double td[3])
-{
-    double S[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    seg_edges(F, G, R, m.kap, [&](const SegTerms &s) {
-        double M[9];
-        seg_matrix(s, m.kap, m.ci, M);
-#pragma unroll
-        for (int c = 0; c < 9; ++c) S[c] += M[c];
-    });
-    double bs[3], bd[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        bs[a] = m.scale * (R[3 + 3 * a] * F(F_SX) + R[4 + 3 * a] * F(F_SY) + R[5 + 3 * a] * F(F_SZ));
-        bd[a] = m.scale * (R[3 + 3 * a] * F(F_DX) + R[4 + 3 * a] * F(F_DY) + R[5 + 3 * a] * F(F_DZ));
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        ts[c] = S[3 * c] * bs[0] + S[3 * c + 1] * bs[1] + S[3 * c + 2] * bs[2];
-        td[c] = S[3 * c] * bd[0] + S[3 * c + 1] * bd[1] + S[3 * c + 2] * bd[2];
-    }
-    return !seg_bad(ts[0]);
-}
-
-// Component c of the tractions of unit strike (ts) and unit dip slip (td).
-// The frame is turned so that the wanted direction is e1 (c < 2: (e_c, n x
-// e_c, n)) or the normal.
-template <class Src>
-__device__ __forceinline__ bool seg_pair_row(const Src &F, const Src &G, const double *R, int c, const SegMat &m,
-                                             double &ts, double &td)
-{
-    const bool normal = c == 2;
-    double Q[kRecvStride];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        Q[q] = R[q];
-        Q[3 + q] = c == 1 ? R[6 + q] : R[3 + q];
-        Q[6 + q] = c == 1 ? -R[3 + q] : R[6 + q];
-        Q[9 + q] = R[9 + q];
-    }
-    double S[3] = {0.0, 0.0, 0.0};
-    seg_edges(F, G, Q, m.kap, [&](const SegTerms &s) {
-        double r[3];
-        seg_row(s, m.kap, m.ci, normal, r);
-        S[0] += r[0];
-        S[1] += r[1];
-        S[2] += r[2];
-    });
-    double g[3];   // back to the mesh's axes
-#pragma unroll
-    for (int a = 0; a < 3; ++a) g[a] = m.scale * (S[0] * Q[3 + a] + S[1] * Q[6 + a] + S[2] * Q[9 + a]);
-    ts = g[0] * F(F_SX) + g[1] * F(F_SY) + g[2] * F(F_SZ);
-    td = g[0] * F(F_DX) + g[1] * F(F_DY) + g[2] * F(F_DZ);
-    return !seg_bad(ts);
-}
-
-// The three tractions of unit strike (dip = false) or unit dip slip.
-template <class Src>
-__device__ __forceinline__ bool seg_pair_col(const Src &F, const Src &G, const double *R, bool dip, const SegMat &m,
-                                             double T[3])
-{
-    const int o = dip ? F_DX : F_SX;
-    double b[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-        b[a] = m.scale * (R[3 + 3 * a] * F(o) + R[4 + 3 * a] * F(o + 1) + R[5 + 3 * a] * F(o + 2));
-    T[0] = T[1] = T[2] = 0.0;
-    seg_edges(F, G, R, m.kap, [&](const SegTerms &s) { seg_apply(s, m.kap, m.ci, b, T); });
-    return !(seg_bad(T[0]) || seg_bad(T[1]) || seg_bad(T[2]));
-}
-
 }  // namespace gf
 }  // namespace pq3d
