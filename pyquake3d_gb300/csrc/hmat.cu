@@ -22,9 +22,8 @@
 //     output row in a fixed order (no atomics, the same result for a run alone
 //     or in a batch).  The ACA tolerance (1e-4) dominates this rounding by
 //     orders of magnitude.
-//   * several right-hand sides run in one launch (one grid row per run); each
-//     run streams the blocks itself (a single-pass multi-run product would
-//     need a GEMM-style tiling of the near field; not done).
+//   * several right-hand sides share every loaded entry in groups of up to 8
+//     runs (leaf_rows_runs_kernel, lowrank_T_runs_kernel).
 // Index space: elements are renumbered so that every cluster is a contiguous
 // range (perm[p] = element at position p); a block is a pair of ranges.
 #include <math.h>
@@ -515,8 +514,8 @@ __global__ void permute_split_kernel(const double *__restrict__ X, const int64_t
 constexpr int kTWarps = 4;
 constexpr int kTGroupsPerWarp = 2;
 
-__device__ __forceinline__ FF t_row_part(const float *__restrict__ v, const float2 *__restrict__ x, int c_begin,
-                                         int c_end, int lane)
+__device__ __forceinline__ FF t_row_part(const float *__restrict__ v, const float2 *__restrict__ x, int xs,
+                                         int c_begin, int c_end, int lane)
 {
     FF sum{0.f, 0.f};
     for (int c0k = c_begin; c0k < c_end; c0k += 1024) {
@@ -531,7 +530,7 @@ __device__ __forceinline__ FF t_row_part(const float *__restrict__ v, const floa
 #pragma unroll
             for (int u = 0; u < 16; ++u) {
                 k[u] = __ldg(v + col + 32 * u);
-                xv[u] = x[col + 32 * u];
+                xv[u] = x[(col + 32 * u) * xs];
             }
 #pragma unroll
             for (int u = 0; u < 16; u += 2) {
@@ -545,14 +544,14 @@ __device__ __forceinline__ FF t_row_part(const float *__restrict__ v, const floa
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 k[u] = __ldg(v + col + 32 * u);
-                xv[u] = x[col + 32 * u];
+                xv[u] = x[(col + 32 * u) * xs];
             }
             acc2_add(a0, k[0], xv[0]);
             acc2_add(a1, k[1], xv[1]);
             acc2_add(a0, k[2], xv[2]);
             acc2_add(a1, k[3], xv[3]);
         }
-        for (; col < cend; col += 32) acc2_add(a0, __ldg(v + col), x[col]);
+        for (; col < cend; col += 32) acc2_add(a0, __ldg(v + col), x[col * xs]);
         // the hi and lo parts of the FP32 partial sums of this chunk
         sum = ff_add(sum, FF{a0.s, 0.f});
         sum = ff_add(sum, FF{a1.s, 0.f});
@@ -645,13 +644,212 @@ lowrank_T_kernel(const float *__restrict__ data, const longlong2 *__restrict__ t
     const int Nc = (int)(info.y >> 32);
     const int piece = (Nc / kTWarps + 31) / 32 * 32;
     const int c_begin = min(Nc, wid * piece), c_end = min(Nc, (wid + 1) * piece);
-    const FF s = t_row_part(data + info.x, xr + (int32_t)(info.y & 0xffffffffll), c_begin, c_end, lane);
+    const FF s = t_row_part(data + info.x, xr + (int32_t)(info.y & 0xffffffffll), 1, c_begin, c_end, lane);
     if (lane == 0) part[wid] = s;
     __syncthreads();
     if (threadIdx.x == 0) {
         FF t = part[0];
         for (int k = 1; k < kTWarps; ++k) t = ff_add(t, part[k]);
         T[w * (int64_t)B + r] = make_float2(t.hi, t.lo);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Several right-hand sides: every loaded entry of H is used for up to 8 runs
+// (4 in the rank rows), with each run's arithmetic -- the same terms, partial
+// sums and order -- that of the one-run kernels above, so that a run's bits do
+// not depend on its batch.
+//
+// The runs that take part are numbered in order (list[0] of them, list[1 + i]
+// = run i) and go into groups of 8, the last one 2, 4 or 8 wide.  The x and T
+// values of two runs lie side by side, [pair][column] of 16 bytes: a warp's 32
+// columns of a pair are four full lines (with all 8 runs of a column together,
+// its loads touched every line of 2 KB four times over).
+//
+// Bound: FP32 issue (2 FMAs per entry and run, one packed f32x2 FMA) beside
+// HBM.  N = 30,000, B = 16: 2.17 ms with a CTA per (leaf, run) -- 16 walks over
+// the blocks from L2, 19 instructions per 192 products -- against 0.27 ms of
+// FMAs and 0.2 ms of HBM.
+
+__host__ __device__ inline int group_width(int left) { return left > 4 ? 8 : (left > 2 ? 4 : 2); }
+// slots of n runs (B > 1)
+__host__ __device__ inline int64_t run_slots(int n)
+{
+    return n <= 1 ? n : 8 * (int64_t)(n / 8) + (n % 8 ? group_width(n % 8) : 0);
+}
+
+__global__ void run_list_kernel(int B, const int32_t *act, int act_stride, int32_t *__restrict__ list)
+{
+    const int lane = threadIdx.x;
+    int n = 0;
+    for (int r0 = 0; r0 < B; r0 += 32) {
+        const bool on = r0 + lane < B && run_on(act, act_stride, r0 + lane);
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (on) list[1 + n + __popc(m & ((1u << lane) - 1u))] = r0 + lane;
+        n += __popc(m);
+    }
+    if (lane == 0) list[0] = n;
+}
+
+// the (hi, lo) products of one entry and one run: two FMAs in one instruction
+__device__ __forceinline__ uint64_t pack2(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void fma2(uint64_t &acc, uint64_t k, uint64_t x)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(k), "l"(x));
+}
+
+typedef ulonglong2 Pair2;   // (hi, lo) of two runs, as f32x2 operands
+
+__global__ void permute_split_runs_kernel(const double *__restrict__ X, const int64_t *__restrict__ perm, int64_t N,
+                                          const int32_t *__restrict__ list, Pair2 *__restrict__ Xs)
+{
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int left = list[0] - 8 * (int)blockIdx.y;
+    if (i >= 2 * N || left <= 0) return;
+    const int64_t col = 2 * perm[i >> 1] + (i & 1);
+    const int32_t *run = list + 1 + 8 * blockIdx.y;
+    for (int h = 0; h < group_width(left) / 2; ++h) {
+        float2 v[2];
+        for (int j = 0; j < 2; ++j)
+            v[j] = 2 * h + j < left ? split2(X[(int64_t)run[2 * h + j] * 2 * N + col]) : make_float2(0.f, 0.f);
+        Xs[(4 * (int64_t)blockIdx.y + h) * 2 * N + i] = make_ulonglong2(pack2(v[0].x, v[0].y), pack2(v[1].x, v[1].y));
+    }
+}
+
+// t_row_group for NR runs (pair h of the x values at x + h * xs, of the sums at T + h * ts).  The 4 NR sums
+// are reduced together: at each step of the butterfly a lane keeps half of
+// them (16 additions for 16 sums instead of 80; every sum is added in
+// warp_sum_ff's tree, and the two-sum is symmetric in its operands).
+template <int NR>
+__device__ __forceinline__ void t_row_group_runs(const float *__restrict__ v, int nc, int g, const Pair2 *__restrict__ x,
+                                                 int64_t xs, int lane, Pair2 *__restrict__ T, int64_t ts)
+{
+    FF sum[4 * NR];
+#pragma unroll
+    for (int q = 0; q < 4 * NR; ++q) sum[q] = FF{0.f, 0.f};
+    for (int c0k = 0; c0k < nc; c0k += 1024) {
+        uint64_t a[4 * NR];
+#pragma unroll
+        for (int q = 0; q < 4 * NR; ++q) a[q] = 0ull;
+        const int cend = min(nc, c0k + 1024);
+        constexpr int U = 4;   // columns per lane in flight
+        for (int col = c0k + lane; col - lane < cend; col += 32 * U) {
+            Pair2 xv[U][NR / 2];
+            float k[U][4];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int c = col + 32 * u;
+                const bool ok = c < cend;
+#pragma unroll
+                for (int h = 0; h < NR / 2; ++h)
+                    xv[u][h] = ok ? x[h * xs + c] : make_ulonglong2(0ull, 0ull);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) k[u][j] = (ok && j < g) ? __ldg(v + (int64_t)j * nc + c) : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint64_t kk = pack2(k[u][j], k[u][j]);
+#pragma unroll
+                    for (int h = 0; h < NR / 2; ++h) {
+                        fma2(a[j * NR + 2 * h], kk, xv[u][h].x);
+                        fma2(a[j * NR + 2 * h + 1], kk, xv[u][h].y);
+                    }
+                }
+        }
+#pragma unroll
+        for (int q = 0; q < 4 * NR; ++q) {
+            const float2 p = unpack2(a[q]);
+            sum[q] = ff_add(sum[q], FF{p.x, 0.f});
+            sum[q] = ff_add(sum[q], FF{p.y, 0.f});
+        }
+    }
+    int idx = 0, o = 16;
+#pragma unroll
+    for (int n = 2 * NR; n >= 1; n >>= 1, o >>= 1) {   // n sums stay
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int q = 0; q < n; ++q) {
+            const FF keep = up ? sum[q + n] : sum[q], give = up ? sum[q] : sum[q + n];
+            FF other;
+            other.hi = __shfl_xor_sync(0xffffffffu, give.hi, o);
+            other.lo = __shfl_xor_sync(0xffffffffu, give.lo, o);
+            sum[q] = ff_add(keep, other);
+        }
+        idx = 2 * idx + (up ? 1 : 0);
+    }
+    for (int p = o; p > 0; p >>= 1) {
+        FF other;
+        other.hi = __shfl_xor_sync(0xffffffffu, sum[0].hi, p);
+        other.lo = __shfl_xor_sync(0xffffffffu, sum[0].lo, p);
+        sum[0] = ff_add(sum[0], other);
+    }
+    if ((lane & (2 * o - 1)) == 0 && idx / NR < g)
+        reinterpret_cast<float2 *>(T + (idx % NR / 2) * ts + idx / NR)[idx & 1] = make_float2(sum[0].hi, sum[0].lo);
+}
+
+__global__ void __launch_bounds__(kTWarps * 32, 4)
+lowrank_T_runs_kernel(const float *__restrict__ data, const longlong2 *__restrict__ t_info,
+                      const int32_t *__restrict__ t_sched, const longlong2 *__restrict__ t_grp, int64_t ngrp,
+                      int64_t nshort, int64_t nlong, int64_t short_ctas, const Pair2 *__restrict__ Xs, int64_t N,
+                      int64_t t_rows, int nquads, Pair2 *__restrict__ T, const int32_t *__restrict__ list)
+{
+    __shared__ FF part[kTWarps];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int quad = (int)(blockIdx.x % (unsigned)nquads), grp = quad >> 1, half = quad & 1;
+    const int64_t cta = blockIdx.x / (unsigned)nquads;
+    const int left = list[0] - 8 * grp;
+    if (left <= 4 * half) return;   // uniform per CTA
+    const int nr = min(4, group_width(left));
+    const Pair2 *xg = Xs + (4 * grp + 2 * half) * 2 * N;
+    Pair2 *Tg = T + (4 * grp + 2 * half) * t_rows;
+    if (cta < short_ctas) {
+        const int64_t g0 = (cta * kTWarps + wid) * kTGroupsPerWarp;
+        if (g0 >= ngrp) return;
+        const int64_t g1 = min(ngrp, g0 + kTGroupsPerWarp);
+        longlong2 nrec = t_grp[g0];
+        for (int64_t gi = g0; gi < g1; ++gi) {
+            const longlong2 rec = nrec;
+            if (gi + 1 < g1) nrec = t_grp[gi + 1];
+            const int64_t off = rec.x & ((1ll << 40) - 1);
+            const int nc = (int)((rec.x >> 40) & 0xffff), g = (int)(rec.x >> 56);
+            const int64_t w0 = (int64_t)((uint64_t)rec.y >> 32);
+            const Pair2 *x = xg + (rec.y & 0xffffffffll);
+            if (nr == 4) t_row_group_runs<4>(data + off, nc, g, x, 2 * N, lane, Tg + w0, t_rows);
+            else t_row_group_runs<2>(data + off, nc, g, x, 2 * N, lane, Tg + w0, t_rows);
+        }
+        return;
+    }
+    const int64_t q = cta - short_ctas;
+    if (q >= nlong) return;   // uniform per CTA
+    const int row = t_sched[nshort + q];
+    const longlong2 info = t_info[row];
+    const int Nc = (int)(info.y >> 32);
+    const int piece = (Nc / kTWarps + 31) / 32 * 32;
+    const int c_begin = min(Nc, wid * piece), c_end = min(Nc, (wid + 1) * piece);
+    for (int j = 0; j < min(nr, left - 4 * half); ++j) {
+        const float2 *x = reinterpret_cast<const float2 *>(xg + (j >> 1) * 2 * N + (info.y & 0xffffffffll)) + (j & 1);
+        const FF s = t_row_part(data + info.x, x, 2, c_begin, c_end, lane);
+        __syncthreads();
+        if (lane == 0) part[wid] = s;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            FF t = part[0];
+            for (int k = 1; k < kTWarps; ++k) t = ff_add(t, part[k]);
+            reinterpret_cast<float2 *>(Tg + (j >> 1) * t_rows + row)[j & 1] = make_float2(t.hi, t.lo);
+        }
     }
 }
 
@@ -743,6 +941,37 @@ __device__ __forceinline__ void leaf_range(const BlkDesc *desc, const int *wpre,
     }
 }
 
+// Descriptors and column prefix sums of the blocks qs .. qs + nq of a leaf
+// whose rows start at p0 (all threads of the CTA).
+__device__ __forceinline__ void load_leaf_blocks(BlkDesc *desc, int *wpre, int nq, int64_t qs, int64_t p0,
+                                                 const int64_t *__restrict__ off, const int64_t *__restrict__ blk,
+                                                 const int32_t *__restrict__ rank,
+                                                 const int32_t *__restrict__ leaf_blocks,
+                                                 const int64_t *__restrict__ t_off)
+{
+    __syncthreads();
+    for (int i = threadIdx.x; i < nq; i += kThreads) {
+        const int bb = leaf_blocks[qs + i];
+        const int64_t r0 = blk[4 * bb], c0 = blk[4 * bb + 2];
+        const int k = rank[bb];
+        BlkDesc d;
+        d.off = off[bb];
+        d.row0 = 3 * (int)(p0 - r0);
+        d.M = 3 * (int)(blk[4 * bb + 1] - r0);
+        d.dense = k < 0;
+        d.w = k < 0 ? 2 * (int)(blk[4 * bb + 3] - c0) : k;
+        d.x0 = k < 0 ? 2 * c0 : t_off[bb];
+        desc[i] = d;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int s = 0;
+        for (int i = 0; i < nq; ++i) { wpre[i] = s; s += desc[i].w; }
+        wpre[nq] = s;
+    }
+    __syncthreads();
+}
+
 __global__ void __launch_bounds__(kThreads, 3)
 leaf_rows_kernel(const float *__restrict__ data, const int64_t *__restrict__ off, const int64_t *__restrict__ blk,
                  const int32_t *__restrict__ rank, const int64_t *__restrict__ leaf, const int64_t *__restrict__ leaf_ptr,
@@ -769,27 +998,7 @@ leaf_rows_kernel(const float *__restrict__ data, const int64_t *__restrict__ off
         for (int i = 0; i < kMaxR; ++i) acc[i] = FF{0.f, 0.f};
         for (int64_t qs = q0; qs < q1; qs += kMaxLeafBlocks) {
             const int nq = (int)min((int64_t)kMaxLeafBlocks, q1 - qs);
-            __syncthreads();
-            for (int i = threadIdx.x; i < nq; i += kThreads) {
-                const int bb = leaf_blocks[qs + i];
-                const int64_t r0 = blk[4 * bb], c0 = blk[4 * bb + 2];
-                const int k = rank[bb];
-                BlkDesc d;
-                d.off = off[bb];
-                d.row0 = 3 * (int)(p0 - r0);
-                d.M = 3 * (int)(blk[4 * bb + 1] - r0);
-                d.dense = k < 0;
-                d.w = k < 0 ? 2 * (int)(blk[4 * bb + 3] - c0) : k;
-                d.x0 = k < 0 ? 2 * c0 : t_off[bb];
-                desc[i] = d;
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                int s = 0;
-                for (int i = 0; i < nq; ++i) { wpre[i] = s; s += desc[i].w; }
-                wpre[nq] = s;
-            }
-            __syncthreads();
+            load_leaf_blocks(desc, wpre, nq, qs, p0, off, blk, rank, leaf_blocks, t_off);
             const int64_t W = wpre[nq];
             const int64_t lo = W * wid / kWarps, hi = W * (wid + 1) / kWarps;
             switch (R) {
@@ -813,6 +1022,196 @@ leaf_rows_kernel(const float *__restrict__ data, const int64_t *__restrict__ off
             Yr[3 * perm[p0 + row / 3] + row % 3] = s;
         }
     }
+}
+
+// The leaf rows for NR runs: as leaf_rows_kernel, a CTA per (leaf, group of
+// runs), the work columns in the same 8 ranges.  Lanes own up to kRunRows / NR
+// rows (24 f32x2 accumulators a lane).  The x values of 32 columns come into
+// shared memory by asynchronous copies (a lane takes its column's pairs), the
+// next 32 while these are used; the entries of the next 4 columns are loaded
+// while 4 are used; the float-float sums, touched once per block segment, live
+// in shared memory.
+constexpr int kRunRows = 24;
+constexpr int kRunMaxR = 6;
+constexpr int kRunFF = kRunRows * kThreads * (int)sizeof(float2);                  // float-float sums
+constexpr int kRunX = kWarps * 2 * 32 * 4 * (int)sizeof(Pair2);                    // staged x, two chunks
+constexpr int kRunRed = kWarps * 32 * kRunMaxR * (int)sizeof(double);              // one run's warp sums
+constexpr int kRunSmem = kRunFF + kRunX + kRunRed;
+
+__device__ __forceinline__ void copy16_async(void *smem, const void *gmem)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+
+// xp: column 0 of the segment's x values (pair h at xp + h * xs)
+template <int R, int NR>
+__device__ __forceinline__ void leaf_segment_runs(const float *__restrict__ col0, int64_t M,
+                                                  const Pair2 *__restrict__ xp, int64_t xs, int ca, int cb, bool last_ok,
+                                                  Pair2 *sx, float2 *ff)
+{
+    constexpr int H = NR / 2, U = 4;
+    const int lane = threadIdx.x & 31;
+    uint64_t a[R * NR];
+#pragma unroll
+    for (int i = 0; i < R * NR; ++i) a[i] = 0ull;
+    auto stage = [&](int c0, int buf) {   // one group of copies per chunk, empty past the end
+        if (c0 + lane < cb)
+#pragma unroll
+            for (int h = 0; h < H; ++h) copy16_async(&sx[buf * 32 * H + lane * H + h], xp + h * xs + c0 + lane);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float kn[U][R];
+    auto load = [&](int c) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                kn[u][i] = (c + u < cb && (i < R - 1 || last_ok)) ? __ldg(col0 + (int64_t)(c + u) * M + 32 * i) : 0.f;
+    };
+    __syncwarp();   // the last segment's chunks have been read
+    stage(ca, 0);
+    load(ca);
+    int buf = 0;
+    for (int c0 = ca; c0 < cb; c0 += 32, buf ^= 1) {
+        stage(c0 + 32, buf ^ 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();   // this chunk is in, from every lane
+        const Pair2 *x0 = sx + buf * 32 * H;
+        const int n = min(32, cb - c0);
+        for (int c = 0; c < n; c += U) {
+            float k[U][R];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int i = 0; i < R; ++i) k[u][i] = kn[u][i];
+            load(c0 + c + U);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (u > 0 && c + u >= n) break;   // uniform
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    const Pair2 x = x0[(c + u) * H + h];
+#pragma unroll
+                    for (int i = 0; i < R; ++i) {
+                        const uint64_t kk = pack2(k[u][i], k[u][i]);
+                        fma2(a[i * NR + 2 * h], kk, x.x);
+                        fma2(a[i * NR + 2 * h + 1], kk, x.y);
+                    }
+                }
+            }
+        }
+        __syncwarp();   // the chunk has been read: the next but one goes there
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < R * NR; ++i) {
+        const float2 v = unpack2(a[i]), f = ff[i * kThreads];
+        FF t = ff_add(FF{f.x, f.y}, FF{v.x, 0.f});
+        t = ff_add(t, FF{v.y, 0.f});
+        ff[i * kThreads] = make_float2(t.hi, t.lo);
+    }
+}
+
+template <int R, int NR>
+__device__ __forceinline__ void leaf_range_runs(const BlkDesc *desc, const int *wpre, int nq, int64_t lo, int64_t hi,
+                                                int pr0, int prow, const float *__restrict__ data,
+                                                const Pair2 *__restrict__ xg, const Pair2 *__restrict__ Tg,
+                                                int64_t N, int64_t t_rows, Pair2 *sx, float2 *ff)
+{
+    const int lane = threadIdx.x & 31;
+    const bool last_ok = lane + 32 * (R - 1) < prow;
+    int q = 0;
+    while (q < nq && wpre[q + 1] <= lo) ++q;
+    for (; q < nq && wpre[q] < hi; ++q) {
+        const BlkDesc d = desc[q];
+        const int ca = (int)max((int64_t)0, lo - wpre[q]);
+        const int cb = (int)min((int64_t)d.w, hi - wpre[q]);
+        if (ca >= cb) continue;
+        leaf_segment_runs<R, NR>(data + d.off + d.row0 + pr0 + lane, d.M, (d.dense ? xg : Tg) + d.x0,
+                                 d.dense ? 2 * N : t_rows, ca, cb, last_ok, sx, ff);
+    }
+}
+
+template <int NR>
+__device__ __forceinline__ void leaf_rows_runs(const float *__restrict__ data, const int64_t *__restrict__ off,
+                                               const int64_t *__restrict__ blk, const int32_t *__restrict__ rank,
+                                               int64_t p0, int64_t p1, int64_t q0, int64_t q1,
+                                               const int32_t *__restrict__ leaf_blocks, const int64_t *__restrict__ perm,
+                                               const Pair2 *__restrict__ xg, const Pair2 *__restrict__ Tg,
+                                               const int64_t *__restrict__ t_off, int64_t t_rows, int64_t N, int runs,
+                                               const int32_t *__restrict__ run, double *__restrict__ Y, BlkDesc *desc,
+                                               int *wpre, char *smem)
+{
+    constexpr int kR = kRunRows / NR < kRunMaxR ? kRunRows / NR : kRunMaxR;
+    constexpr int kPass = 32 * kR;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float2 *ff = reinterpret_cast<float2 *>(smem) + threadIdx.x;
+    Pair2 *sx = reinterpret_cast<Pair2 *>(smem + kRunFF) + wid * 2 * 32 * 4;
+    double *red = reinterpret_cast<double *>(smem + kRunFF + kRunX);
+    const int rows = 3 * (int)(p1 - p0);
+    for (int pr0 = 0; pr0 < rows; pr0 += kPass) {
+        const int prow = min(kPass, rows - pr0);
+        const int R = (prow + 31) / 32;
+        for (int i = 0; i < kR * NR; ++i) ff[i * kThreads] = make_float2(0.f, 0.f);
+        for (int64_t qs = q0; qs < q1; qs += kMaxLeafBlocks) {
+            const int nq = (int)min((int64_t)kMaxLeafBlocks, q1 - qs);
+            load_leaf_blocks(desc, wpre, nq, qs, p0, off, blk, rank, leaf_blocks, t_off);
+            const int64_t W = wpre[nq];
+            const int64_t lo = W * wid / kWarps, hi = W * (wid + 1) / kWarps;
+            if (R == 1) leaf_range_runs<1, NR>(desc, wpre, nq, lo, hi, pr0, prow, data, xg, Tg, N, t_rows, sx, ff);
+            else if (R == 2) leaf_range_runs<2, NR>(desc, wpre, nq, lo, hi, pr0, prow, data, xg, Tg, N, t_rows, sx, ff);
+            else if (R == 3 || kR == 3) leaf_range_runs<3, NR>(desc, wpre, nq, lo, hi, pr0, prow, data, xg, Tg, N, t_rows, sx, ff);
+            else if (R == 4) leaf_range_runs<kR < 4 ? kR : 4, NR>(desc, wpre, nq, lo, hi, pr0, prow, data, xg, Tg, N, t_rows, sx, ff);
+            else if (R == 5) leaf_range_runs<kR < 5 ? kR : 5, NR>(desc, wpre, nq, lo, hi, pr0, prow, data, xg, Tg, N, t_rows, sx, ff);
+            else leaf_range_runs<kR, NR>(desc, wpre, nq, lo, hi, pr0, prow, data, xg, Tg, N, t_rows, sx, ff);
+        }
+        for (int j = 0; j < runs; ++j) {
+            __syncthreads();
+            for (int i = 0; i < kR; ++i) {
+                const float2 f = ff[(i * NR + j) * kThreads];
+                red[wid * kPass + lane + 32 * i] = (double)f.x + (double)f.y;
+            }
+            __syncthreads();
+            double *Yr = Y + (int64_t)run[j] * 3 * N;
+            for (int lr = threadIdx.x; lr < prow; lr += kThreads) {
+                double s = 0.0;
+#pragma unroll
+                for (int w = 0; w < kWarps; ++w) s += red[w * kPass + lr];
+                const int row = pr0 + lr;
+                Yr[3 * perm[p0 + row / 3] + row % 3] = s;
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
+leaf_rows_runs_kernel(const float *__restrict__ data, const int64_t *__restrict__ off, const int64_t *__restrict__ blk,
+                      const int32_t *__restrict__ rank, const int64_t *__restrict__ leaf,
+                      const int64_t *__restrict__ leaf_ptr, const int32_t *__restrict__ leaf_blocks,
+                      const int64_t *__restrict__ perm, const Pair2 *__restrict__ Xs, const Pair2 *__restrict__ T,
+                      const int64_t *__restrict__ t_off, int64_t t_rows, int64_t N, int ngroups,
+                      const int32_t *__restrict__ list, double *__restrict__ Y)
+{
+    extern __shared__ __align__(16) char smem_runs[];
+    __shared__ BlkDesc desc[kMaxLeafBlocks];
+    __shared__ int wpre[kMaxLeafBlocks + 1];
+    const int L = (int)(blockIdx.x / (unsigned)ngroups), grp = (int)(blockIdx.x % (unsigned)ngroups);
+    const int left = list[0] - 8 * grp;
+    if (left <= 0) return;   // uniform per CTA
+    const int w = group_width(left), runs = min(left, 8);
+    const Pair2 *xg = Xs + 4 * grp * 2 * N, *Tg = T + 4 * grp * t_rows;
+    const int32_t *run = list + 1 + 8 * grp;
+    const int64_t p0 = leaf[2 * L], p1 = leaf[2 * L + 1], q0 = leaf_ptr[L], q1 = leaf_ptr[L + 1];
+    if (w == 8)
+        leaf_rows_runs<8>(data, off, blk, rank, p0, p1, q0, q1, leaf_blocks, perm, xg, Tg, t_off, t_rows, N, runs, run, Y, desc,
+                          wpre, smem_runs);
+    else if (w == 4)
+        leaf_rows_runs<4>(data, off, blk, rank, p0, p1, q0, q1, leaf_blocks, perm, xg, Tg, t_off, t_rows, N, runs, run, Y, desc,
+                          wpre, smem_runs);
+    else
+        leaf_rows_runs<2>(data, off, blk, rank, p0, p1, q0, q1, leaf_blocks, perm, xg, Tg, t_off, t_rows, N, runs, run, Y, desc,
+                          wpre, smem_runs);
 }
 
 }  // namespace hm
@@ -953,10 +1352,41 @@ extern "C" int pq3d_hmat_apply_masked(const pq3d_hmat *H, const double *X, int B
     clear_error();
     PQ3D_REQUIRE(H && X && Y && workspace && B >= 1, "pq3d_hmat_apply: bad arguments");
     const int64_t N = H->N;
-    const size_t need = (size_t)B * 2 * N * sizeof(float2) + (size_t)H->t_rows * B * sizeof(float2);
+    const size_t need = pq3d_hmat_workspace_bytes(H, B);
     PQ3D_REQUIRE(workspace_bytes >= need && aligned16(workspace), "pq3d_hmat_apply: workspace too small (%zu < %zu)",
                  workspace_bytes, need);
     cudaStream_t st = (cudaStream_t)stream;
+    const int64_t nshort = H->t_rows - H->t_nlong;
+    const int64_t short_ctas = (H->t_ngrp + kTWarps * kTGroupsPerWarp - 1) / (kTWarps * kTGroupsPerWarp);
+    if (B > 1) {
+        const int64_t slots = run_slots(B);
+        const int ngroups = (B + 7) / 8;
+        Pair2 *Xs = (Pair2 *)workspace, *T = Xs + (size_t)(slots / 2) * 2 * N;
+        int32_t *list = (int32_t *)(T + (size_t)(slots / 2) * H->t_rows);
+        static thread_local int smem_dev = -1;
+        int dev;
+        PQ3D_CUDA_TRY(cudaGetDevice(&dev));
+        if (smem_dev != dev) {
+            PQ3D_CUDA_TRY(cudaFuncSetAttribute(leaf_rows_runs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               kRunSmem));
+            smem_dev = dev;
+        }
+        PQ3D_REQUIRE((short_ctas + H->t_nlong) * 2 * ngroups < (int64_t)INT32_MAX &&
+                         (int64_t)H->nleaves * ngroups < (int64_t)INT32_MAX && ngroups < 65536,
+                     "pq3d_hmat_apply: too many rank rows or leaves x runs");
+        run_list_kernel<<<1, 32, 0, st>>>(B, run_active, active_stride, list);
+        permute_split_runs_kernel<<<dim3((unsigned)((2 * N + 255) / 256), (unsigned)ngroups), 256, 0, st>>>(
+            X, H->perm, N, list, Xs);
+        if (H->t_rows > 0)
+            lowrank_T_runs_kernel<<<(unsigned)((short_ctas + H->t_nlong) * 2 * ngroups), kTWarps * 32, 0, st>>>(
+                H->data, (const longlong2 *)H->t_info, H->t_sched, (const longlong2 *)H->t_grp, H->t_ngrp, nshort,
+                H->t_nlong, short_ctas, Xs, N, H->t_rows, 2 * ngroups, T, list);
+        leaf_rows_runs_kernel<<<(unsigned)(H->nleaves * ngroups), kThreads, kRunSmem, st>>>(
+            H->data, H->off, H->blk, H->rank, H->leaf, H->leaf_ptr, H->leaf_blocks, H->perm, Xs, T, H->t_off, H->t_rows,
+            N, ngroups, list, Y);
+        PQ3D_CUDA_TRY(cudaGetLastError());
+        return PQ3D_OK;
+    }
     float2 *Xs = (float2 *)workspace;
     float2 *T = (float2 *)((char *)workspace + (size_t)B * 2 * N * sizeof(float2));
     dim3 g1((unsigned)((2 * N + 255) / 256), (unsigned)B);
@@ -964,8 +1394,6 @@ extern "C" int pq3d_hmat_apply_masked(const pq3d_hmat *H, const double *X, int B
     // all runs in one launch, run fastest in the block index; a run's result
     // does not depend on B
     if (H->t_rows > 0) {
-        const int64_t nshort = H->t_rows - H->t_nlong;
-        const int64_t short_ctas = (H->t_ngrp + kTWarps * kTGroupsPerWarp - 1) / (kTWarps * kTGroupsPerWarp);
         const int64_t nT = (short_ctas + H->t_nlong) * B;
         PQ3D_REQUIRE(nT < (int64_t)INT32_MAX, "pq3d_hmat_apply: too many rank rows x runs");
         lowrank_T_kernel<<<(unsigned)nT, kTWarps * 32, 0, st>>>(H->data, (const longlong2 *)H->t_info, H->t_sched,
@@ -991,5 +1419,7 @@ extern "C" int pq3d_hmat_apply(const pq3d_hmat *H, const double *X, int B, doubl
 extern "C" size_t pq3d_hmat_workspace_bytes(const pq3d_hmat *H, int B)
 {
     if (!H || B < 1) return 0;
-    return (size_t)B * 2 * H->N * sizeof(float2) + (size_t)H->t_rows * B * sizeof(float2);
+    // x and T values of every run slot, then the list of runs (B > 1)
+    return (size_t)run_slots(B) * (2 * (size_t)H->N + (size_t)H->t_rows) * sizeof(float2) +
+           (B > 1 ? ((size_t)B + 1) * sizeof(int32_t) : 0);
 }
