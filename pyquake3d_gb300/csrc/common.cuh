@@ -52,8 +52,11 @@ __device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned *gen, uns
             __threadfence();
             atomicAdd(gen, 1u);
         } else {
-            unsigned it = 0;
+            // short looks first (a barrier of resident blocks takes a few
+            // microseconds), then ~1 us each up to the limit
+            unsigned it = 0, looks = 0;
             while (*((volatile unsigned *)gen) == my_gen) {
+                if (looks < 256) { ++looks; __nanosleep(32); continue; }
                 if (++it > limit) { ok = false; break; }
                 __nanosleep(1000);
             }

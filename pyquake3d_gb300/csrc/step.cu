@@ -42,14 +42,15 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
-// One warp: out[3i+c] for c = 0..2.  K rows have N double2 (strike, dip).
+// One warp: rows 3i + c, c = 0..2, over the sources [j0, j1).  K rows have N
+// double2 (strike, dip).
 __device__ __forceinline__ void rows3_f64(const double2 *__restrict__ K, const double2 *__restrict__ v, int64_t N,
-                                          int64_t i, int lane, double acc[3])
+                                          int64_t i, int64_t j0, int64_t j1, int lane, double acc[3])
 {
     const double2 *r0 = K + (3 * i) * N, *r1 = r0 + N, *r2 = r1 + N;
     double a0 = 0.0, a1 = 0.0, a2 = 0.0, b0 = 0.0, b1 = 0.0, b2 = 0.0;
-    int64_t j = lane;
-    for (; j + 32 < N; j += 64) {
+    int64_t j = j0 + lane;
+    for (; j + 32 < j1; j += 64) {
         const double2 x0 = __ldg(v + j), x1 = __ldg(v + j + 32);
         const double2 k00 = __ldcs(r0 + j), k10 = __ldcs(r1 + j), k20 = __ldcs(r2 + j);
         const double2 k01 = __ldcs(r0 + j + 32), k11 = __ldcs(r1 + j + 32), k21 = __ldcs(r2 + j + 32);
@@ -60,7 +61,7 @@ __device__ __forceinline__ void rows3_f64(const double2 *__restrict__ K, const d
         b1 = fma(k11.x, x1.x, b1); b1 = fma(k11.y, x1.y, b1);
         b2 = fma(k21.x, x1.x, b2); b2 = fma(k21.y, x1.y, b2);
     }
-    for (; j < N; j += 32) {
+    for (; j < j1; j += 32) {
         const double2 x0 = __ldg(v + j);
         const double2 k00 = __ldcs(r0 + j), k10 = __ldcs(r1 + j), k20 = __ldcs(r2 + j);
         a0 = fma(k00.x, x0.x, a0); a0 = fma(k00.y, x0.y, a0);
@@ -102,12 +103,12 @@ __device__ __forceinline__ float4 split_v(double v1, double v2)
 }
 
 __device__ __forceinline__ void rows3_f32(const float2 *__restrict__ K, const float4 *__restrict__ v, int64_t N,
-                                          int64_t i, int lane, double acc[3])
+                                          int64_t i, int64_t j0, int64_t j1, int lane, double acc[3])
 {
     const float2 *r0 = K + (3 * i) * N, *r1 = r0 + N, *r2 = r1 + N;
     Acc2 a0{0.f, 0.f}, a1{0.f, 0.f}, a2{0.f, 0.f};
-    int64_t j = lane;
-    for (; j + 32 < N; j += 64) {
+    int64_t j = j0 + lane;
+    for (; j + 32 < j1; j += 64) {
         const float4 x0 = __ldg(v + j), x1 = __ldg(v + j + 32);
         const float2 k00 = __ldcs(r0 + j), k10 = __ldcs(r1 + j), k20 = __ldcs(r2 + j);
         const float2 k01 = __ldcs(r0 + j + 32), k11 = __ldcs(r1 + j + 32), k21 = __ldcs(r2 + j + 32);
@@ -118,7 +119,7 @@ __device__ __forceinline__ void rows3_f32(const float2 *__restrict__ K, const fl
         acc2_add(a1, k11.x, x1.x, x1.z); acc2_add(a1, k11.y, x1.y, x1.w);
         acc2_add(a2, k21.x, x1.x, x1.z); acc2_add(a2, k21.y, x1.y, x1.w);
     }
-    for (; j < N; j += 32) {
+    for (; j < j1; j += 32) {
         const float4 x0 = __ldg(v + j);
         const float2 k00 = __ldcs(r0 + j), k10 = __ldcs(r1 + j), k20 = __ldcs(r2 + j);
         acc2_add(a0, k00.x, x0.x, x0.z); acc2_add(a0, k00.y, x0.y, x0.w);
@@ -130,18 +131,48 @@ __device__ __forceinline__ void rows3_f32(const float2 *__restrict__ K, const fl
     acc[2] = warp_sum((double)a2.s + (double)a2.c);
 }
 
-template <bool kF32>
+// The three sums of receiver i by S neighbouring warps of a block of 8 (each a
+// contiguous part of the sources, the parts added in order); valid in lane 0
+// of the first.  A warp has two rounds of loads in flight, so a small operator
+// (in L2) needs more than N warps to keep the FP64 pipe fed: N = 1,600 with S =
+// 1 (11 warps per SM) 46.9 us, S = 2 XX us, against 24.5 us of multiply-adds.
+template <bool kF32, int S>
+__device__ __forceinline__ void receiver_rows(const void *K, const void *v, int64_t N, int64_t i, double acc[3])
+{
+    __shared__ double part[8][3];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, p = w % S;
+    const int64_t len = (N + 32 * S - 1) / (32 * S) * 32, j0 = p * len, j1 = min(N, j0 + len);
+    if (i < N) {
+        if (kF32) rows3_f32((const float2 *)K, (const float4 *)v, N, i, j0, j1, lane, acc);
+        else rows3_f64((const double2 *)K, (const double2 *)v, N, i, j0, j1, lane, acc);
+    }
+    if (S == 1) return;
+    if (lane == 0) { part[w][0] = acc[0]; part[w][1] = acc[1]; part[w][2] = acc[2]; }
+    __syncthreads();
+    if (p == 0)
+        for (int q = 1; q < S; ++q)
+            for (int c = 0; c < 3; ++c) acc[c] += part[w + q][c];
+}
+
+// warps per receiver: at least 16 warps per SM where the mesh is too small for that
+static int receiver_warps(int64_t N, int sms)
+{
+    int s = 1;
+    while (s < 8 && N * s < 16 * (int64_t)sms) s *= 2;
+    return s;
+}
+
+template <bool kF32, int S>
 __global__ void __launch_bounds__(256) matvec_kernel(const void *__restrict__ K, const void *__restrict__ v,
                                                      int64_t N, double *__restrict__ out)
 {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t i = warp; i < N; i += nwarps) {
-        double acc[3];
-        if (kF32) rows3_f32((const float2 *)K, (const float4 *)v, N, i, lane, acc);
-        else rows3_f64((const double2 *)K, (const double2 *)v, N, i, lane, acc);
-        if (lane == 0) { out[3 * i] = acc[0]; out[3 * i + 1] = acc[1]; out[3 * i + 2] = acc[2]; }
+    const int64_t i = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) / S;
+    double acc[3];
+    receiver_rows<kF32, S>(K, v, N, i, acc);
+    if (i < N && (threadIdx.x & 31) == 0 && (threadIdx.x >> 5) % S == 0) {
+        out[3 * i] = acc[0];
+        out[3 * i + 1] = acc[1];
+        out[3 * i + 2] = acc[2];
     }
 }
 
@@ -216,25 +247,18 @@ __global__ void __launch_bounds__(256) vprime_kernel(pq3d_dense_sim S)
     else reinterpret_cast<double2 *>(S.vprime)[i] = make_double2(v1, v2);
 }
 
-// (1) traction rates of one step (src/QDsim_gpu.py:948-957): a warp per
-// receiver, the normal component with the normal loading added (or the
-// loading alone with fix_Tn)
-template <bool kF32>
-__global__ void __launch_bounds__(256) step_rates_kernel(pq3d_dense_sim S)
+// (1) traction rates of one step (src/QDsim_gpu.py:948-957): the normal
+// component with the normal loading added (or the loading alone with fix_Tn)
+template <bool kF32, int S>
+__global__ void __launch_bounds__(256) step_rates_kernel(pq3d_dense_sim D)
 {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int64_t N = S.N;
-    for (int64_t i = warp; i < N; i += nwarps) {
-        double acc[3];
-        if (kF32) rows3_f32((const float2 *)S.K32, (const float4 *)S.vprime, N, i, lane, acc);
-        else rows3_f64((const double2 *)S.K64, (const double2 *)S.vprime, N, i, lane, acc);
-        if (lane == 0) {
-            S.rates[3 * i] = acc[0];
-            S.rates[3 * i + 1] = acc[1];
-            S.rates[3 * i + 2] = S.fix_Tn ? S.normal_loading[i] : acc[2] + S.normal_loading[i];
-        }
+    const int64_t i = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) / S;
+    double acc[3];
+    receiver_rows<kF32, S>(kF32 ? (const void *)D.K32 : (const void *)D.K64, D.vprime, D.N, i, acc);
+    if (i < D.N && (threadIdx.x & 31) == 0 && (threadIdx.x >> 5) % S == 0) {
+        D.rates[3 * i] = acc[0];
+        D.rates[3 * i + 1] = acc[1];
+        D.rates[3 * i + 2] = D.fix_Tn ? D.normal_loading[i] : acc[2] + D.normal_loading[i];
     }
 }
 
@@ -242,12 +266,20 @@ __global__ void __launch_bounds__(256) step_rates_kernel(pq3d_dense_sim S)
 // until one is accepted (grid barrier per attempt for the error norms; every
 // thread takes the same decision), the state update with v' for the next
 // product, the dilatancy step.  `step` indexes h_hist / t_hist / h_force.
+//
+// Bound (small meshes): one chain of FP64 latency per cell.  N = 1,600: 133 us
+// with the reference formula's 15 divisions and 6 exponentials per right-hand
+// side, two pow calls by every thread of the grid (16 warps per SM through a
+// pipe of 2 lanes per clock) and a microsecond between looks at the barrier;
+// XX us with the reciprocal form, the pow calls by two threads of a block and
+// one block per SM (a second one's warps would share its FP64 pipe).
 template <bool kF32>
 __global__ void __launch_bounds__(256) dense_attempt_kernel(pq3d_dense_sim S, int step, double *h_hist, double *t_hist,
                                                             const double *h_force)
 {
     __shared__ unsigned long long red[32];
     __shared__ double dil_cp[kMaxDepth], dil_inv[kMaxDepth];
+    __shared__ double s_c[2], s_hn[2];
     pq3d_step_ctrl *C = S.ctrl;
     // read before the first grid barrier (the lead changes them only after it)
     if (*(volatile int32_t *)&C->status != PQ3D_OK) return;   // same for every block
@@ -277,7 +309,7 @@ __global__ void __launch_bounds__(256) dense_attempt_kernel(pq3d_dense_sim S, in
                          S.P ? S.P[i] : 0.0, S.dPdt ? S.dPdt[i] : 0.0};
             const double y[4] = {S.Tno[i], S.Tt1o[i], S.Tt2o[i], S.state[i]};
             double yo[4], e1, e2;
-            dp_attempt(c, S.V0, S.eta, h, y, yo, e1, e2);
+            dp_attempt<true>(c, S.V0, S.eta, h, y, yo, e1, e2);
             reinterpret_cast<double4_16a *>(S.cand)[i] = make_double4_16a(yo[0], yo[1], yo[2], yo[3]);
             m1 = (isnan(m1) || isnan(e1)) ? NAN : fmax(m1, e1);
             m2 = (isnan(m2) || isnan(e2)) ? NAN : fmax(m2, e2);
@@ -289,8 +321,13 @@ __global__ void __launch_bounds__(256) dense_attempt_kernel(pq3d_dense_sim S, in
             atomicMax((unsigned long long *)&C->err_slot[2 * slot + 1], b2);
         }
         if (!grid_barrier(bc, bg, nb)) { if (threadIdx.x == 0) C->status = PQ3D_ERR_TIMEOUT; return; }
-        const double err1 = __longlong_as_double((long long)*((volatile unsigned long long *)&C->err_slot[2 * slot])) + 1e-10;
-        const double err2 = __longlong_as_double((long long)*((volatile unsigned long long *)&C->err_slot[2 * slot + 1])) + 1e-10;
+        if (threadIdx.x < 2) {
+            const double err =
+                __longlong_as_double((long long)*((volatile unsigned long long *)&C->err_slot[2 * slot + threadIdx.x])) + 1e-10;
+            s_c[threadIdx.x] = err / kRelTol;
+            s_hn[threadIdx.x] = h * 0.9 * pow(kRelTol / err, 0.2);
+        }
+        __syncthreads();
         if (lead) {
             // the slot of the attempt before this one: every thread has read it
             const int z = (int)((attempt + 2) % 3);
@@ -299,9 +336,7 @@ __global__ void __launch_bounds__(256) dense_attempt_kernel(pq3d_dense_sim S, in
             C->attempts += 1;
         }
         ++attempt;
-        const double c1 = err1 / kRelTol, c2 = err2 / kRelTol;
-        const double hn1 = h * 0.9 * pow(kRelTol / err1, 0.2);
-        const double hn2 = h * 0.9 * pow(kRelTol / err2, 0.2);
+        const double c1 = s_c[0], c2 = s_c[1], hn1 = s_hn[0], hn2 = s_hn[1];
         if (h_force || (fmax(c1, c2) < 1.0 && !(isnan(c1) || isnan(c2)))) {
             dtnext = pymin(1.5 * h, pymin(hn1, hn2));
             break;
@@ -334,7 +369,9 @@ __global__ void __launch_bounds__(256) dense_attempt_kernel(pq3d_dense_sim S, in
         S.slip1[i] = s1; S.slip2[i] = s2;
         S.slip[i] = sqrt(s1 * s1 + s2 * s2);
         S.fric[i] = S.P ? S.Tt[i] / (Tno - S.P[i] * 1e-6) : S.Tt[i] / Tno;   // pressure before its update
-        const double w1 = v1 - S.Vpl * cos(S.rake0[i]), w2 = v2 - S.Vpl * sin(S.rake0[i]);
+        double sr, cr;
+        sincos(S.rake0[i], &sr, &cr);
+        const double w1 = v1 - S.Vpl * cr, w2 = v2 - S.Vpl * sr;
         if (kF32) vs[i] = split_v(w1, w2);
         else vp[i] = make_double2(w1, w2);
     }
@@ -343,14 +380,20 @@ __global__ void __launch_bounds__(256) dense_attempt_kernel(pq3d_dense_sim S, in
     // (3b) pore-pressure diffusion of every cell with the new state and
     // slip rate (src/QDsim_gpu.py:628-671, after the update 1119-1120)
     if (S.Parr) dilatancy_step(S, h, dil_cp, dil_inv, cell0, cell1);
-    if (!grid_barrier(bc, bg, nb)) { if (threadIdx.x == 0) C->status = PQ3D_ERR_TIMEOUT; return; }
-    if (lead) {
-        if (h_hist) h_hist[step] = h;
-        if (t_hist) t_hist[step] = time + h;
-        C->steps_done += 1;
-        C->dttry = dtnext;
-        C->time = time + h;
-        C->maxv = __longlong_as_double((long long)C->maxv_bits);
+    // the last block to get here closes the step (no barrier: nobody waits;
+    // bar_count is 0 again since the attempt's barrier)
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(bc, 1u) + 1u == nb) {
+            __threadfence();
+            *(volatile unsigned *)bc = 0u;
+            if (h_hist) h_hist[step] = h;
+            if (t_hist) t_hist[step] = time + h;
+            C->steps_done += 1;
+            C->dttry = dtnext;
+            C->time = time + h;
+            C->maxv = __longlong_as_double((long long)*(volatile unsigned long long *)&C->maxv_bits);
+        }
     }
 }
 
@@ -400,11 +443,11 @@ namespace step {
 
 struct LaunchCfg {
     int device = -1;
-    int grid64 = 0, grid32 = 0;
+    int sms = 0, grid64 = 0, grid32 = 0;
 };
 static thread_local LaunchCfg g_cfg;
 
-static int coop_grid(bool f32, int *grid)
+static int launch_cfg(LaunchCfg **out)
 {
     int dev;
     PQ3D_CUDA_TRY(cudaGetDevice(&dev));
@@ -417,11 +460,39 @@ static int coop_grid(bool f32, int *grid)
         PQ3D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b32, dense_attempt_kernel<true>, 256, 0));
         if (b64 < 1 || b32 < 1) return set_error(PQ3D_ERR_UNSUPPORTED, "stepper kernel does not fit on an SM");
         g_cfg.device = dev;
+        g_cfg.sms = sms;
         g_cfg.grid64 = sms * b64;
         g_cfg.grid32 = sms * b32;
     }
-    *grid = f32 ? g_cfg.grid32 : g_cfg.grid64;
+    *out = &g_cfg;
     return PQ3D_OK;
+}
+
+// Blocks of the attempt kernel: one per SM while its 256 threads hold the
+// SM's cells, else all that are resident.
+static int attempt_grid(const LaunchCfg &c, bool f32, int64_t N)
+{
+    return N <= 256 * (int64_t)c.sms ? c.sms : (f32 ? c.grid32 : c.grid64);
+}
+
+template <bool kF32>
+static void launch_rates(const pq3d_dense_sim &S, int s, cudaStream_t st)
+{
+    const unsigned blocks = (unsigned)((S.N * s + 7) / 8);
+    if (s == 1) step_rates_kernel<kF32, 1><<<blocks, 256, 0, st>>>(S);
+    else if (s == 2) step_rates_kernel<kF32, 2><<<blocks, 256, 0, st>>>(S);
+    else if (s == 4) step_rates_kernel<kF32, 4><<<blocks, 256, 0, st>>>(S);
+    else step_rates_kernel<kF32, 8><<<blocks, 256, 0, st>>>(S);
+}
+
+template <bool kF32>
+static void launch_matvec(const void *K, const void *v, int64_t N, int s, double *out, cudaStream_t st)
+{
+    const unsigned blocks = (unsigned)((N * s + 7) / 8);
+    if (s == 1) matvec_kernel<kF32, 1><<<blocks, 256, 0, st>>>(K, v, N, out);
+    else if (s == 2) matvec_kernel<kF32, 2><<<blocks, 256, 0, st>>>(K, v, N, out);
+    else if (s == 4) matvec_kernel<kF32, 4><<<blocks, 256, 0, st>>>(K, v, N, out);
+    else matvec_kernel<kF32, 8><<<blocks, 256, 0, st>>>(K, v, N, out);
 }
 
 }  // namespace step
@@ -436,11 +507,12 @@ static int matvec(const void *K, int64_t N, const void *v, double *out, void *st
     PQ3D_REQUIRE(N > 0 && K && v && out, "pq3d_dense_matvec: bad arguments");
     PQ3D_REQUIRE(aligned16(v) && (f32 ? ((uintptr_t)K & 7u) == 0 : aligned16(K)),
                  "pq3d_dense_matvec: K and v must be aligned (16 bytes for FP64, 8 for FP32)");
-    const int threads = 256;
-    const int64_t warps = N;
-    const unsigned blocks = (unsigned)((warps * 32 + threads - 1) / threads);
-    if (f32) matvec_kernel<true><<<blocks, threads, 0, (cudaStream_t)stream>>>(K, v, N, out);
-    else matvec_kernel<false><<<blocks, threads, 0, (cudaStream_t)stream>>>(K, v, N, out);
+    LaunchCfg *cfg;
+    const int rc = launch_cfg(&cfg);
+    if (rc) return rc;
+    const int s = receiver_warps(N, cfg->sms);
+    if (f32) launch_matvec<true>(K, v, N, s, out, (cudaStream_t)stream);
+    else launch_matvec<false>(K, v, N, s, out, (cudaStream_t)stream);
     PQ3D_CUDA_TRY(cudaGetLastError());
     return PQ3D_OK;
 }
@@ -469,15 +541,15 @@ extern "C" int pq3d_dense_step(const pq3d_dense_sim *sim, int nsteps, double *h_
                      "pq3d_dense_step: dilatancy needs P, dPdt, dila and 2 <= ndepth <= %d", kMaxDepth);
     if (nsteps == 0) return PQ3D_OK;
     const bool f32 = sim->K32 != nullptr;
-    int grid = 0;
-    int rc = coop_grid(f32, &grid);
+    LaunchCfg *cfg;
+    const int rc = launch_cfg(&cfg);
     if (rc) return rc;
+    const int grid = attempt_grid(*cfg, f32, sim->N), s = receiver_warps(sim->N, cfg->sms);
     // clear the reduction slots and the barrier counter of the control block
     cudaStream_t st = (cudaStream_t)stream;
     PQ3D_CUDA_TRY(cudaMemsetAsync(&sim->ctrl->err_slot[0], 0, sizeof(uint64_t) * 7 + sizeof(uint32_t), st));
     pq3d_dense_sim S = *sim;
     const unsigned cell_blocks = (unsigned)((sim->N + 255) / 256);
-    const unsigned warp_blocks = (unsigned)((sim->N * 32 + 255) / 256);
     if (f32) vprime_kernel<true><<<cell_blocks, 256, 0, st>>>(S);
     else vprime_kernel<false><<<cell_blocks, 256, 0, st>>>(S);
     PQ3D_CUDA_TRY(cudaGetLastError());
@@ -485,11 +557,11 @@ extern "C" int pq3d_dense_step(const pq3d_dense_sim *sim, int nsteps, double *h_
     void *args[] = {(void *)&S, (void *)&step, (void *)&h_hist, (void *)&t_hist, (void *)&h_force};
     for (; step < nsteps; ++step) {
         if (f32) {
-            step_rates_kernel<true><<<warp_blocks, 256, 0, st>>>(S);
+            launch_rates<true>(S, s, st);
             PQ3D_CUDA_TRY(cudaGetLastError());
             PQ3D_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)dense_attempt_kernel<true>, grid, 256, args, 0, st));
         } else {
-            step_rates_kernel<false><<<warp_blocks, 256, 0, st>>>(S);
+            launch_rates<false>(S, s, st);
             PQ3D_CUDA_TRY(cudaGetLastError());
             PQ3D_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)dense_attempt_kernel<false>, grid, 256, args, 0, st));
         }
