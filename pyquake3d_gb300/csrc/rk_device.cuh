@@ -882,6 +882,44 @@ __device__ __forceinline__ void dp_attempt(const Cell &c, double V0, double eta,
     e2 = (isnan(ea) || isnan(eb) || isnan(ec)) ? NAN : fmax(fmax(ea, eb), ec);
 }
 
+// The attempt with dp_attempt<true>'s values, operation by operation, by four
+// neighbouring lanes per cell: lane v integrates variable v of (tau1, tau2,
+// psi, sigma), so the stage sums are one chain a lane, and the four
+// exponentials of a right-hand side (tau1, tau2, -psi/a, (f0 - psi)/b), like the
+// quotients of the two tractions, are one instruction stream.  For meshes with
+// so few cells per SM that a single warp's FP64 latency sets the time.  A1: the
+// lane's traction rate K.v' (v < 2).  All 32 lanes of a warp take part.
+__device__ __forceinline__ void dp_attempt_quad(const Cell &c, int v, double A, double V0, double eta, double h,
+                                                double y, double &yo, double &err)
+{
+    const CellRecip kr = cell_recip(c, V0);
+    const double ds = c.dsig - c.dPdt, dn = c.dsig * 1e-6;
+    auto f = [&](double yl) {
+        const double sig = __shfl_sync(0xffffffffu, yl, 3, 4), st = __shfl_sync(0xffffffffu, yl, 2, 4);
+        const double Tn = sig * 1e6 - c.P, T = yl * 1e6;
+        const double iTn = 1.0 / Tn, iaTn = kr.ia * iTn;
+        const double arg = v < 2 ? T * iaTn : (v == 2 ? -st * kr.ia : (c.f0 - st) * kr.ib);
+        const double e = exp(clip700(arg)), em = 1.0 / e;
+        const double es = __shfl_sync(0xffffffffu, e, 2, 4), ed = __shfl_sync(0xffffffffu, e, 3, 4);
+        const double ch = (e + em) * 0.5, sh = (e - em) * 0.5;
+        const double ct = 2.0 * V0 * iaTn * es, cs = kr.v0ia2 * es;
+        const double dVdtau = ct * ch, dVdsigma = -ct * (T * iTn) * ch, dVdstate = -cs * sh;
+        const double dstate = kr.bdc * (V0 * ed - c.slipv);
+        const double t = (-A + c.shear - eta * (dVdsigma * ds + dVdstate * dstate)) / (1.0 + eta * dVdtau);
+        return v < 2 ? t * 1e-6 : (v == 2 ? dstate : dn);
+    };
+    const double k1 = f(y);
+    const double k2 = f(y + h * B21 * k1);
+    const double k3 = f(y + h * (B31 * k1 + B32 * k2));
+    const double k4 = f(y + h * (B41 * k1 + B42 * k2 + B43 * k3));
+    const double k5 = f(y + h * (B51 * k1 + B52 * k2 + B53 * k3 + B54 * k4));
+    const double k6 = f(y + h * (B61 * k1 + B62 * k2 + B63 * k3 + B64 * k4 + B65 * k5));
+    yo = y + h * (B71 * k1 + B73 * k3 + B74 * k4 + B75 * k5 + B76 * k6);
+    const double k7 = f(yo);
+    const double y8 = y + h * (B81 * k1 + B83 * k3 + B84 * k4 + B85 * k5 + B86 * k6 + B87 * k7);
+    err = fabs(fabs(y8 - yo) / y8);
+}
+
 // max over non-negative doubles (and NaN, which wins) through their bit
 // patterns: for such values unsigned order is numeric order and a NaN's
 // pattern lies above +inf's, so a NaN wins as in numpy's max

@@ -135,7 +135,7 @@ __device__ __forceinline__ void rows3_f32(const float2 *__restrict__ K, const fl
 // contiguous part of the sources, the parts added in order); valid in lane 0
 // of the first.  A warp has two rounds of loads in flight, so a small operator
 // (in L2) needs more than N warps to keep the FP64 pipe fed: N = 1,600 with S =
-// 1 (11 warps per SM) 46.9 us, S = 2 XX us, against 24.5 us of multiply-adds.
+// 1 (11 warps per SM) 46.9 us, S = 2 39.1 us, against 24.5 us of multiply-adds.
 template <bool kF32, int S>
 __device__ __forceinline__ void receiver_rows(const void *K, const void *v, int64_t N, int64_t i, double acc[3])
 {
@@ -271,9 +271,11 @@ __global__ void __launch_bounds__(256) step_rates_kernel(pq3d_dense_sim D)
 // with the reference formula's 15 divisions and 6 exponentials per right-hand
 // side, two pow calls by every thread of the grid (16 warps per SM through a
 // pipe of 2 lanes per clock) and a microsecond between looks at the barrier;
-// XX us with the reciprocal form, the pow calls by two threads of a block and
-// one block per SM (a second one's warps would share its FP64 pipe).
-template <bool kF32>
+// 77 us with the reciprocal form, the pow calls by two threads of a block and
+// one block per SM (a second one's warps would share its FP64 pipe); 42 us with
+// four lanes per cell (kQuad: one cell per four threads, its candidate state
+// in their registers).
+template <bool kF32, bool kQuad>
 __global__ void __launch_bounds__(256) dense_attempt_kernel(pq3d_dense_sim S, int step, double *h_hist, double *t_hist,
                                                             const double *h_force)
 {
@@ -297,12 +299,30 @@ __global__ void __launch_bounds__(256) dense_attempt_kernel(pq3d_dense_sim S, in
     const int64_t cell0 = (int64_t)blockIdx.x * chunk, cell1 = cell0 + chunk < N ? cell0 + chunk : N;
     if (lead) C->maxv_bits = 0ull;   // the update's atomicMax comes after at least one grid barrier
 
+    // kQuad: this thread's cell and variable (tau1, tau2, psi, sigma); lanes
+    // past the last cell shadow it
+    const int var = threadIdx.x & 3;
+    const int64_t ic = cell0 + (threadIdx.x >> 2);
+    const bool mine = ic < cell1;
+    const int64_t iq = mine ? ic : (cell1 > cell0 ? cell1 - 1 : 0);
+    double *const state_of = var == 0 ? S.Tt1o : (var == 1 ? S.Tt2o : (var == 2 ? S.state : S.Tno));
+    double yq = 0.0;
+
     // (2) attempts until one is accepted
     double h = h_force ? h_force[step] : dttry, dtnext = 0.0;
     int nrjct = 0;
     for (;;) {
         const int slot = (int)(attempt % 3);
         double m1 = 0.0, m2 = 0.0;
+        if (kQuad) {
+            if ((threadIdx.x & ~31) < 4 * (cell1 - cell0)) {   // warps with a cell
+                const Cell c{S.a[iq], S.b[iq], S.dc[iq], S.f0[iq], S.shear_loading[iq], S.slipv[iq], 0.0, 0.0,
+                             S.rates[3 * iq + 2], S.P ? S.P[iq] : 0.0, S.dPdt ? S.dPdt[iq] : 0.0};
+                double e;
+                dp_attempt_quad(c, var, var < 2 ? S.rates[3 * iq + var] : 0.0, S.V0, S.eta, h, state_of[iq], yq, e);
+                if (mine) (var == 2 ? m1 : m2) = e;
+            }
+        } else
         for (int64_t i = cell0 + threadIdx.x; i < cell1; i += blockDim.x) {
             const Cell c{S.a[i], S.b[i], S.dc[i], S.f0[i], S.shear_loading[i], S.slipv[i],
                          S.rates[3 * i], S.rates[3 * i + 1], S.rates[3 * i + 2],
@@ -351,6 +371,47 @@ __global__ void __launch_bounds__(256) dense_attempt_kernel(pq3d_dense_sim S, in
 
     // (3) state update (src/QDsim_gpu.py:994-1027)
     double vmax = 0.0;
+    if (kQuad) {
+        if ((threadIdx.x & ~31) < 4 * (cell1 - cell0)) {
+            const double st = __shfl_sync(0xffffffffu, yq, 2, 4), Tno = __shfl_sync(0xffffffffu, yq, 3, 4);
+            const double a = S.a[iq];
+            const double vk = (2.0 * S.V0) * exp(-st / a) * sinh(yq / Tno / a);   // lanes 0, 1
+            const double T1 = __shfl_sync(0xffffffffu, yq, 0, 4), T2 = __shfl_sync(0xffffffffu, yq, 1, 4);
+            const double v1 = __shfl_sync(0xffffffffu, vk, 0, 4), v2 = __shfl_sync(0xffffffffu, vk, 1, 4);
+            // |tau| and |V| on two lanes; the slips and their length
+            const double p = var == 0 ? T1 : v1, q = var == 0 ? T2 : v2;
+            const double len = sqrt(p * p + q * q);
+            const double Tt = __shfl_sync(0xffffffffu, len, 0, 4);
+            double v = __shfl_sync(0xffffffffu, len, 1, 4);
+            if (v < 1e-30) v = 1e-30;
+            double *const slip_of = var == 0 ? S.slip1 : S.slip2;
+            const double sk = var < 2 ? slip_of[iq] + vk * h : 0.0;
+            const double s1 = __shfl_sync(0xffffffffu, sk, 0, 4), s2 = __shfl_sync(0xffffffffu, sk, 1, 4);
+            double sr, cr;
+            sincos(S.rake0[iq], &sr, &cr);
+            const double wk = vk - S.Vpl * (var == 0 ? cr : sr);
+            const double w1 = __shfl_sync(0xffffffffu, wk, 0, 4), w2 = __shfl_sync(0xffffffffu, wk, 1, 4);
+            if (mine) {
+                state_of[iq] = yq;
+                if (var < 2) {
+                    (var == 0 ? S.slipv1 : S.slipv2)[iq] = vk;
+                    slip_of[iq] = sk;
+                }
+                if (var == 0) {
+                    S.slipv[iq] = v;
+                    S.slip[iq] = sqrt(s1 * s1 + s2 * s2);
+                    if (kF32) vs[iq] = split_v(w1, w2);
+                    else vp[iq] = make_double2(w1, w2);
+                } else if (var == 1) {
+                    S.Tt[iq] = Tt;
+                    S.fric[iq] = S.P ? Tt / (Tno - S.P[iq] * 1e-6) : Tt / Tno;   // pressure before its update
+                } else if (var == 2) {
+                    S.rake[iq] = atan2(v2, v1);
+                }
+                vmax = isnan(v) ? NAN : v;
+            }
+        }
+    } else
     for (int64_t i = cell0 + threadIdx.x; i < cell1; i += blockDim.x) {
         const double4_16a y = reinterpret_cast<const double4_16a *>(S.cand)[i];
         const double Tno = y.x, T1 = y.y, T2 = y.z, st = y.w, a = S.a[i];
@@ -456,9 +517,12 @@ static int launch_cfg(LaunchCfg **out)
         PQ3D_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         PQ3D_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
         if (!coop) return set_error(PQ3D_ERR_UNSUPPORTED, "device has no cooperative launch");
-        PQ3D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b64, dense_attempt_kernel<false>, 256, 0));
-        PQ3D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b32, dense_attempt_kernel<true>, 256, 0));
-        if (b64 < 1 || b32 < 1) return set_error(PQ3D_ERR_UNSUPPORTED, "stepper kernel does not fit on an SM");
+        int q64 = 0, q32 = 0;
+        PQ3D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b64, dense_attempt_kernel<false, false>, 256, 0));
+        PQ3D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b32, dense_attempt_kernel<true, false>, 256, 0));
+        PQ3D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q64, dense_attempt_kernel<false, true>, 256, 0));
+        PQ3D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q32, dense_attempt_kernel<true, true>, 256, 0));
+        if (b64 < 1 || b32 < 1 || q64 < 1 || q32 < 1) return set_error(PQ3D_ERR_UNSUPPORTED, "stepper kernel does not fit on an SM");
         g_cfg.device = dev;
         g_cfg.sms = sms;
         g_cfg.grid64 = sms * b64;
@@ -474,6 +538,11 @@ static int attempt_grid(const LaunchCfg &c, bool f32, int64_t N)
 {
     return N <= 256 * (int64_t)c.sms ? c.sms : (f32 ? c.grid32 : c.grid64);
 }
+
+// Four lanes per cell up to this many cells per SM (one block's 256 threads
+// would hold 64): there a warp per SM and cell count of 32 is as much work for
+// the FP64 pipe as four warps of quads, whose chains are three times shorter.
+constexpr int64_t kQuadCells = 32;
 
 template <bool kF32>
 static void launch_rates(const pq3d_dense_sim &S, int s, cudaStream_t st)
@@ -553,18 +622,18 @@ extern "C" int pq3d_dense_step(const pq3d_dense_sim *sim, int nsteps, double *h_
     if (f32) vprime_kernel<true><<<cell_blocks, 256, 0, st>>>(S);
     else vprime_kernel<false><<<cell_blocks, 256, 0, st>>>(S);
     PQ3D_CUDA_TRY(cudaGetLastError());
+    const bool quad = S.N <= kQuadCells * cfg->sms;
+    const void *attempt = f32 ? (quad ? (const void *)dense_attempt_kernel<true, true>
+                                      : (const void *)dense_attempt_kernel<true, false>)
+                              : (quad ? (const void *)dense_attempt_kernel<false, true>
+                                      : (const void *)dense_attempt_kernel<false, false>);
     int step = 0;
     void *args[] = {(void *)&S, (void *)&step, (void *)&h_hist, (void *)&t_hist, (void *)&h_force};
     for (; step < nsteps; ++step) {
-        if (f32) {
-            launch_rates<true>(S, s, st);
-            PQ3D_CUDA_TRY(cudaGetLastError());
-            PQ3D_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)dense_attempt_kernel<true>, grid, 256, args, 0, st));
-        } else {
-            launch_rates<false>(S, s, st);
-            PQ3D_CUDA_TRY(cudaGetLastError());
-            PQ3D_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)dense_attempt_kernel<false>, grid, 256, args, 0, st));
-        }
+        if (f32) launch_rates<true>(S, s, st);
+        else launch_rates<false>(S, s, st);
+        PQ3D_CUDA_TRY(cudaGetLastError());
+        PQ3D_CUDA_TRY(cudaLaunchCooperativeKernel(attempt, grid, 256, args, 0, st));
     }
     return PQ3D_OK;
 }
