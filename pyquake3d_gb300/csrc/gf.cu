@@ -12,8 +12,7 @@
 //                                     tractions -> FP64 K (+ FP32 copy) with
 //                                     16-byte stores
 //   assemble_dense_hs                 half space: one pair per thread
-//   points_one_source / point_many_sources
-//                                     the two host-pointer entry points of the
+//   points_full / points_hs           the two host-pointer entry points of the
 //                                     reference TDstressFS_C.so
 //   half-space (jud_halfspace / halfspace != 0): per-source image record and
 //   free-surface side table (setup_hs), the pair evaluated by
@@ -340,111 +339,224 @@ assemble_dense_hs_kernel(const double *__restrict__ src, const double *__restric
     }
 }
 
-__global__ void points_one_source_hs_kernel(SrcVal s, SrcVal si, FscVal g, const double *__restrict__ X,
-                                            const double *__restrict__ Y, const double *__restrict__ Z, int64_t n,
-                                            double bx, double by, double bz, double mu, double lam, double nu,
-                                            double k, double *__restrict__ stress, double *__restrict__ strain)
+// ---------------------------------------------------------------------------
+// Point kernels (host-pointer calls): strain and stress of n pairs -- one
+// source at n receivers (kMany = false, records by value), or n sources at one
+// receiver (kMany = true, the thread sets its source up).  The calls are short:
+// what counts is the chain of FP64 latency of one pair (a half-space pair by
+// one thread: ~200 us), so a pair's parts are shared out over the warps of a
+// block of 32 pairs: half space -- three warps with a side of the free-surface
+// correction each, a fourth with the main and the image dislocation; full space
+// -- a warp per angular dislocation.  The parts are added in order through
+// shared memory, and the 12 results per pair stored as one contiguous piece.
+struct PointArgs {
+    const double *A, *B, *C;      // receivers X, Y, Z, or the sources' vertices [n][3]
+    double X, Y, Z;               // the one receiver (kMany)
+    int64_t n;
+    double bx, by, bz, mu, lam, nu, k;
+    double *stress, *strain;      // [n][6]
+};
+constexpr int kPointPairs = 32;
+
+template <bool kMany>
+struct PointPair {
+    double a[3], b[3], c[3], x, y, z;
+    __device__ PointPair(const PointArgs &P, int64_t i)
+    {
+        if (kMany) {
+            for (int q = 0; q < 3; ++q) { a[q] = P.A[3 * i + q]; b[q] = P.B[3 * i + q]; c[q] = P.C[3 * i + q]; }
+            x = P.X; y = P.Y; z = P.Z;
+        } else {
+            x = P.A[i]; y = P.B[i]; z = P.C[i];
+        }
+    }
+};
+
+// The parts' sum e of pair t (thread t of the first warp) to the outputs; all
+// threads of the block.
+__device__ __forceinline__ void store_points(const PointArgs &P, int64_t i0, const double e[6], double (*out)[kPointPairs][6])
 {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const ValSrc F{s.f}, Fi{si.f}, G{g.f};
-    double e[6], sg[6];
-    point_strain_hs(F, Fi, G, X[i], Y[i], Z[i], bx, by, bz, nu, k, e);
-    hooke(e, mu, lam, sg);
-    for (int c = 0; c < 6; ++c) { stress[6 * i + c] = sg[c]; strain[6 * i + c] = e[c]; }
+    const int t = threadIdx.x;
+    if (t < kPointPairs) {
+        double s[6];
+        hooke(e, P.mu, P.lam, s);
+        for (int q = 0; q < 6; ++q) { out[0][t][q] = s[q]; out[1][t][q] = e[q]; }
+    }
+    __syncthreads();
+    const int n = 6 * (int)min((int64_t)kPointPairs, P.n - i0);
+    for (int q = t; q < n; q += blockDim.x) {
+        P.stress[6 * i0 + q] = (&out[0][0][0])[q];
+        P.strain[6 * i0 + q] = (&out[1][0][0])[q];
+    }
 }
 
-__global__ void point_many_sources_hs_kernel(double X, double Y, double Z, const double *__restrict__ P1,
-                                             const double *__restrict__ P2, const double *__restrict__ P3,
-                                             int64_t ns, double bx, double by, double bz, double mu, double lam,
-                                             double nu, double k, double *__restrict__ stress,
-                                             double *__restrict__ strain)
+template <bool kMany>
+__global__ void __launch_bounds__(128) points_hs_kernel(SrcVal s, SrcVal si, FscVal g, PointArgs P)
 {
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= ns) return;
-    double f[kSrcStride], fi[kSrcStride], g[kFscStride];
-    double a[3] = {P1[3 * j], P1[3 * j + 1], P1[3 * j + 2]};
-    double b[3] = {P2[3 * j], P2[3 * j + 1], P2[3 * j + 2]};
-    double c[3] = {P3[3 * j], P3[3 * j + 1], P3[3 * j + 2]};
-    double am[3] = {a[0], a[1], -a[2]}, bm[3] = {b[0], b[1], -b[2]}, cm[3] = {c[0], c[1], -c[2]};
-    setup_source(a, b, c, f, 1);
-    setup_source(am, bm, cm, fi, 1);
-    setup_fsc(a, b, c, g, 1);
-    const ValSrc F{f}, Fi{fi}, G{g};
-    double e[6], sg[6];
-    point_strain_hs(F, Fi, G, X, Y, Z, bx, by, bz, nu, k, e);
-    hooke(e, mu, lam, sg);
-    for (int q = 0; q < 6; ++q) { stress[6 * j + q] = sg[q]; strain[6 * j + q] = e[q]; }
+    __shared__ double part[5][kPointPairs][6], out[2][kPointPairs][6];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t i0 = (int64_t)blockIdx.x * kPointPairs, i = i0 + lane;
+    if (i < P.n) {
+        const PointPair<kMany> p(P, i);
+        if (w < 3) {
+            double f[S_COUNT];
+            if (kMany) setup_fsc_side(p.a, p.b, p.c, w, f, 1);
+            point_strain_side(ValSrc{kMany ? f : g.f + w * S_COUNT}, p.x, p.y, p.z, P.bx, P.by, P.bz, P.nu, part[w][lane]);
+        } else {
+            for (int q = 0; q < 2; ++q) {
+                double f[kSrcStride];
+                const double sg = q ? -1.0 : 1.0;
+                if (kMany) {
+                    const double a[3] = {p.a[0], p.a[1], sg * p.a[2]}, b[3] = {p.b[0], p.b[1], sg * p.b[2]},
+                                 c[3] = {p.c[0], p.c[1], sg * p.c[2]};
+                    setup_source<false>(a, b, c, f, 1);
+                }
+                point_strain_full(ValSrc{kMany ? f : (q ? si.f : s.f)}, p.x, p.y, p.z, P.bx, P.by, P.bz, P.nu, P.k,
+                                  part[3 + q][lane]);
+            }
+            image_signs(kMany ? fsc_surface(p.a, p.b, p.c) : g.f[kFscSurface], part[4][lane]);
+        }
+    }
+    __syncthreads();
+    double e[6];
+    if (threadIdx.x < kPointPairs && i < P.n)
+        for (int q = 0; q < 6; ++q)
+            e[q] = part[3][lane][q] + ((part[0][lane][q] + part[1][lane][q] + part[2][lane][q]) + part[4][lane][q]);
+    store_points(P, i0, e, out);
 }
 
-__global__ void points_one_source_kernel(SrcVal s, const double *__restrict__ X, const double *__restrict__ Y,
-                                         const double *__restrict__ Z, int64_t n, double bx, double by, double bz,
-                                         double mu, double lam, double nu, double k, double *__restrict__ stress,
-                                         double *__restrict__ strain)
+// W warps per 32 pairs: 3 (a vertex each) or 1.
+template <bool kMany, int W>
+__global__ void __launch_bounds__(32 * W) points_full_kernel(SrcVal s, PointArgs P)
 {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const ValSrc F{s.f};
-    double x, y, z, E[6], e[6], sg[6];
-    tdcs_point(F, X[i], Y[i], Z[i], x, y, z);
-    tdcs_strain_general(F, x, y, z, bx, by, bz, nu, k, E);
-    tdcs_to_efcs(F, E, e);
-    hooke(e, mu, lam, sg);
-    for (int c = 0; c < 6; ++c) { stress[6 * i + c] = sg[c]; strain[6 * i + c] = e[c]; }
-}
-
-__global__ void point_many_sources_kernel(double X, double Y, double Z, const double *__restrict__ P1,
-                                          const double *__restrict__ P2, const double *__restrict__ P3, int64_t ns,
-                                          double bx, double by, double bz, double mu, double lam, double nu, double k,
-                                          double *__restrict__ stress, double *__restrict__ strain)
-{
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= ns) return;
+    __shared__ double part[W][kPointPairs][6], out[2][kPointPairs][6];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t i0 = (int64_t)blockIdx.x * kPointPairs, i = i0 + lane;
     double f[kSrcStride];
-    double a[3] = {P1[3 * j], P1[3 * j + 1], P1[3 * j + 2]};
-    double b[3] = {P2[3 * j], P2[3 * j + 1], P2[3 * j + 2]};
-    double c[3] = {P3[3 * j], P3[3 * j + 1], P3[3 * j + 2]};
-    setup_source(a, b, c, f, 1);
-    const ValSrc F{f};
-    double x, y, z, E[6], e[6], sg[6];
-    tdcs_point(F, X, Y, Z, x, y, z);
-    tdcs_strain_general(F, x, y, z, bx, by, bz, nu, k, E);
-    tdcs_to_efcs(F, E, e);
-    hooke(e, mu, lam, sg);
-    for (int q = 0; q < 6; ++q) { stress[6 * j + q] = sg[q]; strain[6 * j + q] = e[q]; }
+    const ValSrc F{kMany ? f : s.f};
+    double E[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (i < P.n) {
+        const PointPair<kMany> p(P, i);
+        if (kMany) setup_source<false>(p.a, p.b, p.c, f, 1);
+        double x, y, z;
+        tdcs_point(F, p.x, p.y, p.z, x, y, z);
+        const int m = tdcs_mode(F, x, y, z);
+        if (m != 0)
+            for (int v = W > 1 ? w : 0; v < (W > 1 ? w + 1 : 3); ++v)
+                tdcs_vertex_general(F, m, v, x, y, z, P.bx, P.by, P.bz, P.nu, P.k, E);
+        for (int q = 0; q < 6; ++q) part[w][lane][q] = E[q];
+    }
+    __syncthreads();
+    double e[6];
+    if (threadIdx.x < kPointPairs && i < P.n) {
+        for (int q = 0; q < 6; ++q) {
+            E[q] = part[0][lane][q];
+            for (int v = 1; v < W; ++v) E[q] += part[v][lane][q];
+        }
+        tdcs_to_efcs(F, E, e);
+    }
+    store_points(P, i0, e, out);
+}
+
+// A source per thread costs its set-up once more for every warp that shares
+// the pair: beyond this many pairs (the SMs hold their warps) one warp takes
+// all three vertices (40,000 sources: 282 us by three warps, 184 us by one).
+constexpr size_t kPointShare = 4096;
+
+template <bool kMany>
+static void launch_points_full(const SrcVal &s, const PointArgs &P, size_t n, cudaStream_t st)
+{
+    const unsigned blocks = (unsigned)((n + kPointPairs - 1) / kPointPairs);
+    if (!kMany || n <= kPointShare) points_full_kernel<kMany, 3><<<blocks, 96, 0, st>>>(s, P);
+    else points_full_kernel<kMany, 1><<<blocks, 32, 0, st>>>(s, P);
 }
 
 static inline double poisson(double mu, double lam) { return 1.0 / (1.0 + lam / mu) / 2.0; }
 static inline double kfac(double nu) { return 1.0 / (8.0 * kPi * (1.0 - nu)); }
 
 // ---------------------------------------------------------------------------
-// host-pointer context: one stream and one growing device buffer per host thread
+// host-pointer context: one stream, one growing device buffer and one bounded
+// page-locked buffer per host thread, given back when the thread ends
 struct HostCtx {
     int device = -1;
     cudaStream_t stream = nullptr;
     double *buf = nullptr;
     size_t cap = 0;   // doubles
+    double *pin = nullptr, *pin_dev = nullptr;   // host and device address
+    void drop()
+    {
+        if (device < 0) return;
+        if (stream) cudaStreamDestroy(stream);
+        if (buf) cudaFree(buf);
+        if (pin) cudaFreeHost(pin);
+        (void)cudaGetLastError();
+        device = -1;
+        stream = nullptr;
+        buf = pin = pin_dev = nullptr;
+        cap = 0;
+    }
+    ~HostCtx() { drop(); }
 };
 static thread_local HostCtx g_ctx;
 
-static int host_ctx(size_t need_doubles, HostCtx **out)
+// Calls of up to kPinDoubles doubles in and out go through page-locked memory
+// that the kernel reads and writes itself: one launch and one wait, where five
+// copies of a few KB each cost more than the kernel (64 points: 61 -> 44 us a
+// call, 4,000: 128 -> 106 us; 12,000 sources: 295 -> 351 us).  Above, the copies' own rate counts.
+constexpr size_t kPinDoubles = 1 << 16;
+
+static int host_ctx(size_t need_doubles, bool *pinned, HostCtx **out)
 {
     int dev = 0;
     PQ3D_CUDA_TRY(cudaGetDevice(&dev));
     HostCtx &c = g_ctx;
     if (c.device != dev) {
-        c = HostCtx();
-        c.device = dev;
+        c.drop();
         PQ3D_CUDA_TRY(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
+        c.device = dev;
+    }
+    *out = &c;
+    *pinned = need_doubles <= kPinDoubles;
+    if (*pinned) {
+        if (!c.pin) {
+            PQ3D_CUDA_TRY(cudaHostAlloc(&c.pin, kPinDoubles * sizeof(double), cudaHostAllocMapped));
+            void *d = nullptr;
+            PQ3D_CUDA_TRY(cudaHostGetDevicePointer(&d, c.pin, 0));
+            c.pin_dev = (double *)d;
+        }
+        return PQ3D_OK;
     }
     if (c.cap < need_doubles) {
         if (c.buf) cudaFree(c.buf);
         c.buf = nullptr;
+        c.cap = 0;
         size_t cap = std::max<size_t>(need_doubles, 1 << 16);
         PQ3D_CUDA_TRY(cudaMalloc(&c.buf, cap * sizeof(double)));
         c.cap = cap;
     }
-    *out = &c;
+    return PQ3D_OK;
+}
+
+// n doubles into the call's buffer at offset `at` (doubles); the address the kernel reads
+static int put(HostCtx *c, bool pinned, size_t at, const double *src, size_t n)
+{
+    if (pinned) memcpy(c->pin + at, src, n * sizeof(double));
+    else PQ3D_CUDA_TRY(cudaMemcpyAsync(c->buf + at, src, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    return PQ3D_OK;
+}
+
+// the two results of n doubles each from offset `at`, once the kernel is done
+static int take(HostCtx *c, bool pinned, size_t at, size_t n, double *stress, double *strain)
+{
+    if (!pinned) {
+        PQ3D_CUDA_TRY(cudaMemcpyAsync(stress, c->buf + at, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+        PQ3D_CUDA_TRY(cudaMemcpyAsync(strain, c->buf + at + n, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    }
+    PQ3D_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if (pinned) {
+        memcpy(stress, c->pin + at, n * sizeof(double));
+        memcpy(strain, c->pin + at + n, n * sizeof(double));
+    }
     return PQ3D_OK;
 }
 
@@ -473,34 +585,29 @@ static int points_one_source(const double *X, const double *Y, const double *Z, 
     PQ3D_REQUIRE(X && Y && Z && P1 && P2 && P3 && stress && strain, "TDstressFS_C: null pointer");
     if (half) warn_halfspace_z(X, Y, Z, n, P1, P2, P3);
     HostCtx *c;
-    int rc = host_ctx(15 * n, &c);
+    bool pinned;
+    int rc = host_ctx(15 * n, &pinned, &c);
+    const double *in[3] = {X, Y, Z};
+    for (int q = 0; q < 3 && !rc; ++q) rc = put(c, pinned, q * n, in[q], n);
     if (rc) return rc;
-    double *dX = c->buf, *dY = dX + n, *dZ = dY + n, *dS = dZ + n, *dE = dS + 6 * n;
-    PQ3D_CUDA_TRY(cudaMemcpyAsync(dX, X, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    PQ3D_CUDA_TRY(cudaMemcpyAsync(dY, Y, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    PQ3D_CUDA_TRY(cudaMemcpyAsync(dZ, Z, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    SrcVal s;
+    double *dX = pinned ? c->pin_dev : c->buf, *dY = dX + n, *dZ = dY + n, *dS = dZ + n, *dE = dS + 6 * n;
+    SrcVal s, si;
+    FscVal g;
     double a[3] = {P1[0], P1[1], P1[2]}, b[3] = {P2[0], P2[1], P2[2]}, cc[3] = {P3[0], P3[1], P3[2]};
     setup_source(a, b, cc, s.f, 1);
     const double nu = poisson(mu, lam);
-    const int threads = 128;
+    const PointArgs P{dX, dY, dZ, 0.0, 0.0, 0.0, (int64_t)n, Ts, Ss, Ds, mu, lam, nu, kfac(nu), dS, dE};
+    const unsigned blocks = (unsigned)((n + kPointPairs - 1) / kPointPairs);
     if (half) {
-        SrcVal si;
-        FscVal g;
         double am[3] = {a[0], a[1], -a[2]}, bm[3] = {b[0], b[1], -b[2]}, cm[3] = {cc[0], cc[1], -cc[2]};
         setup_source(am, bm, cm, si.f, 1);
         setup_fsc(a, b, cc, g.f, 1);
-        points_one_source_hs_kernel<<<(unsigned)((n + threads - 1) / threads), threads, 0, c->stream>>>(
-            s, si, g, dX, dY, dZ, (int64_t)n, Ts, Ss, Ds, mu, lam, nu, kfac(nu), dS, dE);
+        points_hs_kernel<false><<<blocks, 128, 0, c->stream>>>(s, si, g, P);
     } else {
-        points_one_source_kernel<<<(unsigned)((n + threads - 1) / threads), threads, 0, c->stream>>>(
-            s, dX, dY, dZ, (int64_t)n, Ts, Ss, Ds, mu, lam, nu, kfac(nu), dS, dE);
+        launch_points_full<false>(s, P, n, c->stream);
     }
     PQ3D_CUDA_TRY(cudaGetLastError());
-    PQ3D_CUDA_TRY(cudaMemcpyAsync(stress, dS, 6 * n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    PQ3D_CUDA_TRY(cudaMemcpyAsync(strain, dE, 6 * n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    PQ3D_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    return PQ3D_OK;
+    return take(c, pinned, 3 * n, 6 * n, stress, strain);
 }
 
 static int point_many_sources(double x, double y, double z, const double *P1, const double *P2, const double *P3,
@@ -512,25 +619,19 @@ static int point_many_sources(double x, double y, double z, const double *P1, co
     PQ3D_REQUIRE(P1 && P2 && P3 && stress && strain, "TDstressEachSourceAtReceiver_C: null pointer");
     if (half) warn_halfspace_z(&x, &y, &z, 1, nullptr, nullptr, nullptr);
     HostCtx *c;
-    int rc = host_ctx(21 * ns, &c);
+    bool pinned;
+    int rc = host_ctx(21 * ns, &pinned, &c);
+    const double *in[3] = {P1, P2, P3};
+    for (int q = 0; q < 3 && !rc; ++q) rc = put(c, pinned, 3 * q * ns, in[q], 3 * ns);
     if (rc) return rc;
-    double *d1 = c->buf, *d2 = d1 + 3 * ns, *d3 = d2 + 3 * ns, *dS = d3 + 3 * ns, *dE = dS + 6 * ns;
-    PQ3D_CUDA_TRY(cudaMemcpyAsync(d1, P1, 3 * ns * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    PQ3D_CUDA_TRY(cudaMemcpyAsync(d2, P2, 3 * ns * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    PQ3D_CUDA_TRY(cudaMemcpyAsync(d3, P3, 3 * ns * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    double *d1 = pinned ? c->pin_dev : c->buf, *d2 = d1 + 3 * ns, *d3 = d2 + 3 * ns, *dS = d3 + 3 * ns, *dE = dS + 6 * ns;
     const double nu = poisson(mu, lam);
-    const int threads = 128;
-    if (half)
-        point_many_sources_hs_kernel<<<(unsigned)((ns + threads - 1) / threads), threads, 0, c->stream>>>(
-            x, y, z, d1, d2, d3, (int64_t)ns, Ts, Ss, Ds, mu, lam, nu, kfac(nu), dS, dE);
-    else
-        point_many_sources_kernel<<<(unsigned)((ns + threads - 1) / threads), threads, 0, c->stream>>>(
-            x, y, z, d1, d2, d3, (int64_t)ns, Ts, Ss, Ds, mu, lam, nu, kfac(nu), dS, dE);
+    const PointArgs P{d1, d2, d3, x, y, z, (int64_t)ns, Ts, Ss, Ds, mu, lam, nu, kfac(nu), dS, dE};
+    const unsigned blocks = (unsigned)((ns + kPointPairs - 1) / kPointPairs);
+    if (half) points_hs_kernel<true><<<blocks, 128, 0, c->stream>>>(SrcVal(), SrcVal(), FscVal(), P);
+    else launch_points_full<true>(SrcVal(), P, ns, c->stream);
     PQ3D_CUDA_TRY(cudaGetLastError());
-    PQ3D_CUDA_TRY(cudaMemcpyAsync(stress, dS, 6 * ns * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    PQ3D_CUDA_TRY(cudaMemcpyAsync(strain, dE, 6 * ns * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    PQ3D_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    return PQ3D_OK;
+    return take(c, pinned, 9 * ns, 6 * ns, stress, strain);
 }
 
 // Workspace: source table [kSrcStride][N], receiver table [N][kRecvStride],

@@ -88,6 +88,10 @@ __host__ __device__ inline double cube_im(double sy, double sz)
 }
 
 // Source setup (src/TDstressFS_C.cpp:291-396).  f[i * fstride] receives field i.
+// kAngles: through the vertex angles, as the reference (and the tables); else
+// their cosines and sines from the unit side vectors' products (no acos, sin
+// and cos: for a kernel that sets up a source per thread).
+template <bool kAngles = true>
 __host__ __device__ inline void setup_source(const double P1[3], const double P2[3], const double P3[3],
                                              double *f, int fstride)
 {
@@ -112,16 +116,26 @@ __host__ __device__ inline void setup_source(const double P1[3], const double P2
     double e13[3] = {p3[0] - p1[0], p3[1] - p1[1], p3[2] - p1[2]};
     double e23[3] = {p3[0], p3[1], p3[2]};
     unit3(e12); unit3(e13); unit3(e23);
-    const double A = acos(e12[0] * e13[0] + e12[1] * e13[1] + e12[2] * e13[2]);
-    const double B = acos(-e12[0] * e23[0] - e12[1] * e23[1] - e12[2] * e23[2]);
-    const double C = acos(e23[0] * e13[0] + e23[1] * e13[1] + e23[2] * e13[2]);
-    const double Am = -kPi + A, Bm = -kPi + B, Cm = -kPi + C;
+    const double dA = e12[0] * e13[0] + e12[1] * e13[1] + e12[2] * e13[2];
+    const double dB = -e12[0] * e23[0] - e12[1] * e23[1] - e12[2] * e23[2];
+    const double dC = e23[0] * e13[0] + e23[1] * e13[1] + e23[2] * e13[2];
+    double ca, sa, cb, sb, cc, sc;   // of (angle - pi)
+    if (kAngles) {
+        const double Am = -kPi + acos(dA), Bm = -kPi + acos(dB), Cm = -kPi + acos(dC);
+        ca = cos(Am); sa = sin(Am);
+        cb = cos(Bm); sb = sin(Bm);
+        cc = cos(Cm); sc = sin(Cm);
+    } else {
+        ca = -dA; sa = -fabs(e12[1] * e13[2] - e12[2] * e13[1]);
+        cb = -dB; sb = -fabs(e12[1] * e23[2] - e12[2] * e23[1]);
+        cc = -dC; sc = -fabs(e23[1] * e13[2] - e23[2] * e13[1]);
+    }
     const double vals[F_COUNT] = {
         P2[0], P2[1], P2[2], n[0], n[1], n[2], s[0], s[1], s[2], d[0], d[1], d[2],
         p1[1], p1[2], p3[1], p3[2],
         -p3[2] * (p1[1] - p3[1]) + p3[1] * (p1[2] - p3[2]),
         e13[1], e13[2], e12[1], e12[2], e23[1], e23[2],
-        cos(Am), sin(Am), cos(Bm), sin(Bm), cos(Cm), sin(Cm),
+        ca, sa, cb, sb, cc, sc,
         e13[2] * e13[2] - e13[1] * e13[1], 2.0 * (e13[1] * e13[2]),
         e12[2] * e12[2] - e12[1] * e12[1], 2.0 * (e12[1] * e12[2]),
         e23[2] * e23[2] - e23[1] * e23[1], 2.0 * (e23[1] * e23[2]),
@@ -252,6 +266,63 @@ __device__ __forceinline__ float d2f_rn_bits(double x)
     return __uint_as_float(f);
 }
 #endif
+
+#ifdef __CUDACC__
+// Positive v truncated to FP32 by the bit layout (three integer operations:
+// GB300 runs FP64 <-> FP32 conversions on its FP64 pipe); NaN where v is not
+// within 2^-120 .. 2^120.
+__device__ __forceinline__ float seed_f32(double v)
+{
+    const unsigned hw = (unsigned)__double2hiint(v);
+    const unsigned f = __funnelshift_l((unsigned)__double2loint(v), hw, 3) - (896u << 23);
+    return __uint_as_float(hw - (903u << 20) < (240u << 20) ? f : 0x7fc00000u);
+}
+// A normal FP32 value (or NaN, inf) widened by the bit layout.
+__device__ __forceinline__ double widen_seed(float s)
+{
+    const unsigned u = __float_as_uint(s);
+    const unsigned hi = (u >> 3) + (896u << 20);
+    return __hiloint2double((int)(s < 3.0e38f ? hi : 0x7ff80000u), (int)(u << 29));
+}
+// 1/p and 1/sqrt(q), r = sqrt(q): one third-order step from the FP32 value
+// (1 + e + e^2 and 1 + e/2 + 3 e^2/8 times the seed, e its FP64 residual,
+// below 2^-22: the cubic term is below 2^-66): 3 and 6 FP64 operations.
+__device__ __forceinline__ double seg_rcp(double p)
+{
+    const double s = widen_seed(__frcp_rn(seed_f32(p)));
+    const double e = fma(-p, s, 1.0);
+    return fma(s, fma(e, e, e), s);
+}
+__device__ __forceinline__ void seg_rsqrt(double q, double &r, double &ir)
+{
+    const double s = widen_seed(rsqrtf(seed_f32(q)));
+    const double e = fma(-q * s, s, 1.0);
+    ir = fma(s * e, fma(0.375, e, 0.5), s);
+    r = q * ir;
+}
+#endif
+// 1/x and sqrt(q) with its reciprocal: by those steps where they apply, else
+// (zero, not finite, beyond 2^+-120) the plain quotient and root.  The root
+// takes one residual more: an ulp of it comes times cot^2 beta near a vertical
+// side (q ir alone moved a strain there by 2e-10).
+__device__ __forceinline__ double reciprocal(double x)
+{
+#ifdef __CUDACC__
+    const double r = seg_rcp(x);
+    if (isfinite_t(r)) return r;
+#endif
+    return 1.0 / x;
+}
+__device__ __forceinline__ void root_and_reciprocal(double q, double &r, double &ir)
+{
+#ifdef __CUDACC__
+    seg_rsqrt(q, r, ir);
+    r = fma(fma(-r, r, q), 0.5 * ir, r);
+    if (isfinite_t(r)) return;
+#endif
+    r = sqrt(q);
+    ir = 1.0 / r;
+}
 
 // Shared geometric terms of one angular dislocation at (x, y, z) of its own
 // frame, opening angle with cos/sin (ca, sa).
@@ -500,36 +571,49 @@ __device__ __forceinline__ bool tdcs_strain_sd2k(const Src &F, T x, T y, T z, do
     return true;
 }
 
-// General Burgers vector (bx = Ts, by = Ss, bz = Ds) strain in the triangle system.
+// General Burgers vector (bx = Ts, by = Ss, bz = Ds): the angular dislocation
+// of vertex v (configuration m = +-1), added to the strain E in the triangle
+// system.
+template <class Src>
+__device__ __forceinline__ void tdcs_vertex_general(const Src &F, int m, int v, double x, double y, double z, double bx,
+                                                    double by, double bz, double nu, double k, double E[6])
+{
+    const double sg = (m == 1) ? 1.0 : -1.0;
+    double vy, vz, sy, sz, ca, sa;
+    if (v == 0) { vy = F(F_P1Y); vz = F(F_P1Z); sy = -sg * F(F_E13Y); sz = -sg * F(F_E13Z); ca = F(F_CA); sa = F(F_SA); }
+    else if (v == 1) { vy = 0.0; vz = 0.0; sy = sg * F(F_E12Y); sz = sg * F(F_E12Z); ca = F(F_CB); sa = F(F_SB); }
+    else { vy = F(F_P3Y); vz = F(F_P3Z); sy = sg * F(F_E23Y); sz = sg * F(F_E23Z); ca = F(F_CC); sa = F(F_SC); }
+    const double ty = y - vy, tz = z - vz;
+    AdGeom<double> g;
+    ad_geom<double>(x, sz * ty - sy * tz, sy * ty + sz * tz, ca, sa, nu, g);
+    double Ey[6], Ez[6], Ex[6];
+    ad_parts_yz<double>(g, nu, k, Ey, Ez);
+    const double by1 = sz * by - sy * bz, bz1 = sy * by + sz * bz;
+    double t[6];
+    if (bx != 0.0) {
+        ad_part_x(g, nu, k, Ex);
+        for (int i = 0; i < 6; ++i) t[i] = bx * Ex[i] + by1 * Ey[i] + bz1 * Ez[i];
+    } else {
+        for (int i = 0; i < 6; ++i) t[i] = by1 * Ey[i] + bz1 * Ez[i];
+    }
+    add_rot_x(E, t, sy, sz, sz * sz - sy * sy, 2.0 * (sy * sz));
+}
+
+template <class Src>
+__device__ __forceinline__ int tdcs_mode(const Src &F, double x, double y, double z)
+{
+    return tri_mode<double>(x, y, z, F(F_P1Y), F(F_P1Z), F(F_P3Y), F(F_P3Z), F(F_DEN));
+}
+
 template <class Src>
 __device__ __forceinline__ void tdcs_strain_general(const Src &F, double x, double y, double z, double bx, double by,
                                                     double bz, double nu, double k, double E[6])
 {
 #pragma unroll
     for (int i = 0; i < 6; ++i) E[i] = 0.0;
-    const int m = tri_mode<double>(x, y, z, F(F_P1Y), F(F_P1Z), F(F_P3Y), F(F_P3Z), F(F_DEN));
+    const int m = tdcs_mode(F, x, y, z);
     if (m == 0) return;
-    const double sg = (m == 1) ? 1.0 : -1.0;
-    for (int v = 0; v < 3; ++v) {
-        double vy, vz, sy, sz, ca, sa;
-        if (v == 0) { vy = F(F_P1Y); vz = F(F_P1Z); sy = -sg * F(F_E13Y); sz = -sg * F(F_E13Z); ca = F(F_CA); sa = F(F_SA); }
-        else if (v == 1) { vy = 0.0; vz = 0.0; sy = sg * F(F_E12Y); sz = sg * F(F_E12Z); ca = F(F_CB); sa = F(F_SB); }
-        else { vy = F(F_P3Y); vz = F(F_P3Z); sy = sg * F(F_E23Y); sz = sg * F(F_E23Z); ca = F(F_CC); sa = F(F_SC); }
-        const double ty = y - vy, tz = z - vz;
-        AdGeom<double> g;
-        ad_geom<double>(x, sz * ty - sy * tz, sy * ty + sz * tz, ca, sa, nu, g);
-        double Ey[6], Ez[6], Ex[6];
-        ad_parts_yz<double>(g, nu, k, Ey, Ez);
-        const double by1 = sz * by - sy * bz, bz1 = sy * by + sz * bz;
-        double t[6];
-        if (bx != 0.0) {
-            ad_part_x(g, nu, k, Ex);
-            for (int i = 0; i < 6; ++i) t[i] = bx * Ex[i] + by1 * Ey[i] + bz1 * Ez[i];
-        } else {
-            for (int i = 0; i < 6; ++i) t[i] = by1 * Ey[i] + bz1 * Ez[i];
-        }
-        add_rot_x(E, t, sy, sz, sz * sz - sy * sy, 2.0 * (sy * sz));
-    }
+    for (int v = 0; v < 3; ++v) tdcs_vertex_general(F, m, v, x, y, z, bx, by, bz, nu, k, E);
 }
 
 // T_EFCS = A^T T A with A rows (n, s, d) of the source system.

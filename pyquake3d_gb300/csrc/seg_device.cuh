@@ -78,47 +78,15 @@ __device__ __forceinline__ double flip_sign(double v, unsigned s)   // v with it
     return __hiloint2double((int)((unsigned)__double2hiint(v) ^ s), __double2loint(v));
 }
 __device__ __forceinline__ unsigned sign_bit(double v) { return (unsigned)__double2hiint(v) & 0x80000000u; }
-// Positive v truncated to FP32 by the bit layout (three integer operations:
-// GB300 runs FP64 <-> FP32 conversions on its FP64 pipe); NaN where v is not
-// within 2^-120 .. 2^120.
-__device__ __forceinline__ float seed_f32(double v)
-{
-    const unsigned hw = (unsigned)__double2hiint(v);
-    const unsigned f = __funnelshift_l((unsigned)__double2loint(v), hw, 3) - (896u << 23);
-    return __uint_as_float(hw - (903u << 20) < (240u << 20) ? f : 0x7fc00000u);
-}
-// A normal FP32 value (or NaN, inf) widened by the bit layout.
-__device__ __forceinline__ double widen_seed(float s)
-{
-    const unsigned u = __float_as_uint(s);
-    const unsigned hi = (u >> 3) + (896u << 20);
-    return __hiloint2double((int)(s < 3.0e38f ? hi : 0x7ff80000u), (int)(u << 29));
-}
-// 1/p and 1/sqrt(q), r = sqrt(q): one third-order step from the FP32 value
-// (1 + e + e^2 and 1 + e/2 + 3 e^2/8 times the seed, e its FP64 residual,
-// below 2^-22: the cubic term is below 2^-66): 3 and 6 FP64 operations.
-__device__ __forceinline__ double seg_rcp(double p)
-{
-    const double s = widen_seed(__frcp_rn(seed_f32(p)));
-    const double e = fma(-p, s, 1.0);
-    return fma(s, fma(e, e, e), s);
-}
-__device__ __forceinline__ void seg_rsqrt(double q, double &r, double &ir)
-{
-    const double s = widen_seed(rsqrtf(seed_f32(q)));
-    const double e = fma(-q * s, s, 1.0);
-    ir = fma(s * e, fma(0.375, e, 0.5), s);
-    r = q * ir;
-}
 __device__ __forceinline__ double seg_nan() { return __hiloint2double(0x7ff80000, 0); }
 __device__ __forceinline__ float seg_small(double v) { return (float)seed_f32(v); }
 #else
 inline double flip_sign(double v, unsigned s) { return s ? -v : v; }
 inline unsigned sign_bit(double v) { return std::signbit(v) ? 0x80000000u : 0u; }
-inline double seg_rcp(double p) { return 1.0 / p; }
-inline void seg_rsqrt(double q, double &r, double &ir) { r = sqrt(q); ir = 1.0 / r; }
 inline double seg_nan() { return NAN; }
 inline float seg_small(double v) { return (float)v; }
+inline double seg_rcp(double p) { return 1.0 / p; }
+inline void seg_rsqrt(double q, double &r, double &ir) { r = sqrt(q); ir = 1.0 / r; }
 #endif
 
 // R: receiver record (centroid, e1, e2, n).
