@@ -11,12 +11,13 @@
 //                                     pair per thread, both unit slips, 6
 //                                     tractions -> FP64 K (+ FP32 copy) with
 //                                     16-byte stores
-//   assemble_dense_hs                 half space: one pair per thread
+//   assemble_hs                       half space: the same, with the edge's image
+//                                     and its free-surface correction
 //   points_full / points_hs           the two host-pointer entry points of the
 //                                     reference TDstressFS_C.so
 //   half-space (jud_halfspace / halfspace != 0): per-source image record and
-//   free-surface side table (setup_hs), the pair evaluated by
-//   pair_tractions_hs / point_strain_hs (hs_device.cuh)
+//   free-surface side table (setup_hs) for single pairs (pair_tractions_hs,
+//   hs_device.cuh), per-edge records (setup_tiles) for the assembly
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -92,11 +93,35 @@ struct Tile {
 };
 constexpr int kSegDoubles = (int)(sizeof(Tile) / sizeof(double));
 static_assert(sizeof(Tile) % 16 == 0, "tiles start 16-byte aligned");
+// Half space: the geometric fields of the edges' free-surface record (those of
+// setup_fsc_side before the Burgers vectors, and 1 / sin beta), one row a field.
+constexpr int kHsFields = S_BN0 + 1;
+struct TileHs {
+    double f[kHsFields][kTileItems];
+};
+constexpr int kHsDoubles = (int)(sizeof(TileHs) / sizeof(double));
+struct TileSide {   // the record of one edge
+    const double *f;
+    __device__ __forceinline__ double operator()(int i) const
+    {
+        return __ldg(f + (i == S_ISIN ? kHsFields - 1 : i) * kTileItems);
+    }
+};
 
-inline int64_t tile_count(int64_t N) { return (N + kTileMax - 1) / kTileMax; }
+// (half space: 240 triangles, so that the matrices of 720 edges that none
+// share leave room for two blocks per SM)
+constexpr int kTileMaxHs = 240;
+inline int64_t tile_count(int64_t N, bool half = false)
+{
+    const int most = half ? kTileMaxHs : kTileMax;
+    return (N + most - 1) / most;
+}
 // equal tiles: the last one of N = 1,600 would hold 64 of 256 triangles, and
 // its blocks would idle while the others finish
-inline int tile_size(int64_t N) { return (int)((N + tile_count(N) - 1) / tile_count(N)); }
+inline int tile_size(int64_t N, bool half = false)
+{
+    return (int)((N + tile_count(N, half) - 1) / tile_count(N, half));
+}
 
 // One block per tile: the node ids and the node pairs go into hash tables in
 // shared memory; the thread that places a key takes the next local index.
@@ -105,7 +130,7 @@ inline int tile_size(int64_t N) { return (int)((N + tile_count(N) - 1) / tile_co
 constexpr int kHash = 2048;
 __global__ void __launch_bounds__(kTileMax)
 setup_tiles_kernel(const double *__restrict__ nodes, const int64_t *__restrict__ tris, int64_t N, int ts,
-                   Tile *__restrict__ tiles)
+                   Tile *__restrict__ tiles, TileHs *__restrict__ hs)
 {
     __shared__ unsigned long long vkey[kHash], ekey[kHash];
     __shared__ uint16_t vidx[kHash], eidx[kHash];
@@ -157,6 +182,13 @@ setup_tiles_kernel(const double *__restrict__ nodes, const int64_t *__restrict__
             if (eown[q]) {
                 const SegEdge r = seg_edge_record(nodes + 3 * (id[q] - 1), nodes + 3 * (id[n] - 1));
                 T.edge[e] = TileEdge{r.L, r.iL, r.near2, vidx[vs[rev ? n : q]], vidx[vs[rev ? q : n]]};
+                if (hs) {
+                    const double *A = nodes + 3 * (id[rev ? n : q] - 1), *B = nodes + 3 * (id[rev ? q : n] - 1);
+                    double f[S_COUNT];
+                    setup_fsc_side(A, B, nodes + 3 * (id[(q + 2) % 3] - 1), 0, f, 1);
+                    f[kHsFields - 1] = f[S_ISIN];
+                    for (int i = 0; i < kHsFields; ++i) hs[blockIdx.x].f[i][e] = f[i];
+                }
             }
             tri.e[q] = (uint16_t)(e | (rev ? 0x8000 : 0));
         }
@@ -299,42 +331,147 @@ assemble_seg_kernel(const Tile *__restrict__ tiles, int ts, const double *__rest
     }
 }
 
-constexpr int kTJ = 128;   // half space: sources per block (one per thread)
-constexpr int kTI = 32;    // receivers per block (looped by every thread)
+// ---------------------------------------------------------------------------
+// Half-space dense assembly from the tiles: per receiver (1) every edge's
+// matrices -- that of the edge with its free-surface correction, and that of
+// its mirror image, whose triangles slip along axes of their own -- and (2) the
+// triangles' sums.  The correction of an edge walked the other way is its
+// negative, so that it too serves both triangles of an edge.
+//
+// Bound: the FP64 pipe, with the correction's two end points 85 % of an edge's
+// ~1,700 operations; an edge per item instead of three sides per pair is 1.7
+// instead of 3 of them on a structured mesh (N = 2,500: 67.8 ms with a thread
+// per pair, 35.3 ms; 102 ms with the derivatives in nine variables, a thread per pair).
+constexpr int kHsThreads = 128;   // 255 registers, two blocks per SM
+constexpr int kHsRecv = 16;       // receivers of a block at most
+constexpr int kHsMatD = 18;
+constexpr int kHsSmem = 3 * kTileMaxHs * kHsMatD * (int)sizeof(double);
 
-// Half-space variant: main record in shared memory, image record and side
-// table read from their structure-of-arrays tables (coalesced over sources).
-template <bool kWrite32>
-__global__ void __launch_bounds__(kTJ)
-assemble_dense_hs_kernel(const double *__restrict__ src, const double *__restrict__ recv,
-                         const double *__restrict__ img, const double *__restrict__ fsc, int64_t N, int64_t row0,
-                         int64_t row1, double nu, double k, double two_mu, double lam, double *__restrict__ K64,
-                         float *__restrict__ K32)
+// The pair by its angular dislocations (receivers on an edge of the source or
+// of its image; sources in the surface).
+__device__ __noinline__ void pair_angular_hs(const double *src, const double *img, const double *fsc, int64_t N,
+                                             const double *R, double nu, double k, double two_mu, double lam,
+                                             double ts[3], double td[3])
 {
-    __shared__ double s_src[F_COUNT * kTJ];
-    __shared__ double s_rcv[kTI * kRecvStride];
-    const int t = threadIdx.x;
-    const int64_t j0 = (int64_t)blockIdx.x * kTJ;
-    const int64_t i0 = row0 + (int64_t)blockIdx.y * kTI;
-    const int64_t j = j0 + t;
-    for (int f = 0; f < F_COUNT; ++f) s_src[f * kTJ + t] = (j < N) ? src[f * N + j] : 0.0;
-    const int nrec = (int)((row1 - i0) < kTI ? (row1 - i0) : kTI);
-    for (int q = t; q < nrec * kRecvStride; q += kTJ) s_rcv[q] = recv[i0 * kRecvStride + q];
-    __syncthreads();
-    if (j >= N) return;
-    const SoaSrc F{s_src + t, kTJ};
-    const SoaSrc Fi{img + j, (int)N};
-    const SoaSrc G{fsc + j, (int)N};
-    const int64_t ld = 2 * N;
-    for (int ii = 0; ii < nrec; ++ii) {
-        double ts[3], td[3];
-        pair_tractions_hs(F, Fi, G, s_rcv + ii * kRecvStride, nu, k, two_mu, lam, ts, td);
-        const int64_t r = 3 * (i0 + ii - row0);
+    const SoaSrc F{src, (int)N}, Fi{img, (int)N}, G{fsc, (int)N};
+    pair_tractions_hs(F, Fi, G, R, nu, k, two_mu, lam, ts, td);
+}
+
+// The correction of one edge as a matrix like seg_matrix's, added to M.
+__device__ __forceinline__ void fsc_matrix(const TileSide &F, const double *R, double nu, double two_mu, double lam,
+                                           double M[9])
+{
+    double U[3][6];
+    if (!fsc_side_strains(F, R[0], R[1], R[2], nu, U)) return;
+    const double c1 = F(S_C1), s1 = F(S_S1);
+    // in units of mu/(4 pi): the strains' factor 1/(4 pi (1 - nu)) times 2 mu, lambda
+    const double c2 = 2.0 / (1.0 - nu), cl = c2 * lam / two_mu;
+    double r[3][3];   // the receiver's axes in the side's frame
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double *e = R + 3 + 3 * a;
+        r[a][0] = e[0] * c1 + e[1] * s1;
+        r[a][1] = e[0] * s1 - e[1] * c1;
+        r[a][2] = -e[2];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const double *e = U[k];
+        const double h3 = 0.5 * e[3], h4 = 0.5 * e[4], h5 = 0.5 * e[5];
+        const double u0 = e[0] * r[2][0] + h3 * r[2][1] + h4 * r[2][2];
+        const double u1 = h3 * r[2][0] + e[1] * r[2][1] + h5 * r[2][2];
+        const double u2 = h4 * r[2][0] + h5 * r[2][1] + e[2] * r[2][2];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            *reinterpret_cast<double2 *>(K64 + (r + c) * ld + 2 * j) = make_double2(ts[c], td[c]);
-            if (kWrite32)
-                *reinterpret_cast<float2 *>(K32 + (r + c) * ld + 2 * j) = make_float2(d2f_rn_bits(ts[c]), d2f_rn_bits(td[c]));
+            double t = c2 * (r[c][0] * u0 + r[c][1] * u1 + r[c][2] * u2);
+            if (c == 2) t += cl * (e[0] + e[1] + e[2]);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) M[3 * c + a] += t * r[a][k];
+        }
+    }
+}
+
+template <bool kWrite32>
+__global__ void __launch_bounds__(kHsThreads, 2)
+assemble_hs_kernel(const Tile *__restrict__ tiles, const TileHs *__restrict__ hs, int ts,
+                   const double *__restrict__ src, const double *__restrict__ recv, const double *__restrict__ img,
+                   const double *__restrict__ fsc, int64_t N, int64_t row0, int64_t row1, int nr, SegMat mat, double nu,
+                   double k, double two_mu, double lam, double *__restrict__ K64, float *__restrict__ K32)
+{
+    extern __shared__ double s_buf[];
+    __shared__ double s_rcv[kHsRecv * kRecvStride];
+    const int t = threadIdx.x;
+    const Tile &T = tiles[blockIdx.x];
+    const int ne = T.ne;
+    const int64_t i0 = row0 + (int64_t)blockIdx.y * nr;
+    const int nrec = (int)((row1 - i0) < nr ? (row1 - i0) : nr);
+    for (int q = t; q < nrec * kRecvStride; q += kHsThreads) s_rcv[q] = recv[i0 * kRecvStride + q];
+    const int batch = min(nrec, kHsSmem / (int)sizeof(double) / (ne * kHsMatD));
+    const int64_t j0 = (int64_t)blockIdx.x * ts, ld = 2 * N;
+    const int nt = (int)((N - j0) < ts ? (N - j0) : ts);
+    for (int b0 = 0; b0 < nrec; b0 += batch) {
+        const int nb = min(batch, nrec - b0);
+        __syncthreads();   // the receivers are in; the last batch's readers are done
+        for (int q = t; q < nb * ne; q += kHsThreads) {
+            const int r = q / ne, e = q - r * ne;
+            const double *R = s_rcv + (b0 + r) * kRecvStride;
+            const TileEdge ed = T.edge[e];
+            const double *A = T.vert[ed.a], *B = T.vert[ed.b];
+            double *o = s_buf + q * kHsMatD;
+            double M[9];
+            seg_matrix(seg_terms(seg_vertex(R, A[0], A[1], -A[2]), seg_vertex(R, B[0], B[1], -B[2]), ed.L, ed.iL,
+                                 ed.near2, mat.kap), mat.kap, mat.ci, M);
+#pragma unroll
+            for (int c = 0; c < 9; ++c) o[9 + c] = M[c];
+            seg_matrix(seg_terms(seg_vertex(R, A[0], A[1], A[2]), seg_vertex(R, B[0], B[1], B[2]), ed.L, ed.iL,
+                                 ed.near2, mat.kap), mat.kap, mat.ci, M);
+            fsc_matrix(TileSide{&hs[blockIdx.x].f[0][e]}, R, nu, two_mu, lam, M);
+#pragma unroll
+            for (int c = 0; c < 9; ++c) o[c] = M[c];
+        }
+        __syncthreads();
+        for (int q = t; q < nt; q += kHsThreads) {
+            const int64_t j = j0 + q;
+            const TileTri tri = T.tri[q];
+            const bool surface = fsc[kFscSurface * N + j] != 0.0;
+            for (int r = 0; r < nb; ++r) {
+                const double *R = s_rcv + (b0 + r) * kRecvStride, *Mr = s_buf + r * ne * kHsMatD;
+                double ts3[3] = {0.0, 0.0, 0.0}, td3[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {   // the edges with the correction, the image
+                    const double *tab = p ? img : src;
+                    double vs[3], vd[3];
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        vs[a] = mat.scale * (R[3 + 3 * a] * tab[F_SX * N + j] + R[4 + 3 * a] * tab[F_SY * N + j] +
+                                             R[5 + 3 * a] * tab[F_SZ * N + j]);
+                        vd[a] = mat.scale * (R[3 + 3 * a] * tab[F_DX * N + j] + R[4 + 3 * a] * tab[F_DY * N + j] +
+                                             R[5 + 3 * a] * tab[F_DZ * N + j]);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) {
+                            double m = 0.0;
+#pragma unroll
+                            for (int v = 0; v < 3; ++v)
+                                m += flip_sign(Mr[(tri.e[v] & 0x7fff) * kHsMatD + 9 * p + 3 * c + a],
+                                               (unsigned)(tri.e[v] & 0x8000) << 16);
+                            ts3[c] += m * vs[a];
+                            td3[c] += m * vd[a];
+                        }
+                }
+                if (surface || seg_bad(ts3[0]))
+                    pair_angular_hs(src + j, img + j, fsc + j, N, R, nu, k, two_mu, lam, ts3, td3);
+                const int64_t row = 3 * (i0 + b0 + r - row0);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    *reinterpret_cast<double2 *>(K64 + (row + c) * ld + 2 * j) = make_double2(ts3[c], td3[c]);
+                    if (kWrite32)
+                        *reinterpret_cast<float2 *>(K32 + (row + c) * ld + 2 * j) =
+                            make_float2(d2f_rn_bits(ts3[c]), d2f_rn_bits(td3[c]));
+                }
+            }
         }
     }
 }
@@ -635,13 +772,18 @@ static int point_many_sources(double x, double y, double z, const double *P1, co
 }
 
 // Workspace: source table [kSrcStride][N], receiver table [N][kRecvStride],
-// then for the half space the image table [kImgStride][N] and the side table
-// [kFscStride][N], for the full space (from an even offset) the tiles.
-static size_t tiles_offset(int64_t N) { return ((size_t)N * (kSrcStride + kRecvStride) + 1) & ~(size_t)1; }
+// for the half space the image table [kImgStride][N] and the side table
+// [kFscStride][N], then (from an even offset) the tiles, and for the half space
+// their edges' surface records.
+static size_t tables_doubles(int64_t N, bool half)
+{
+    return (size_t)N * (kSrcStride + kRecvStride + (half ? kImgStride + kFscStride : 0));
+}
+static size_t tiles_offset(int64_t N, bool half) { return (tables_doubles(N, half) + 1) & ~(size_t)1; }
 static size_t ws_bytes(int64_t N, bool half)
 {
-    const size_t h = (size_t)N * (kSrcStride + kRecvStride + kImgStride + kFscStride);
-    return (half ? h : tiles_offset(N) + (size_t)tile_count(N) * kSegDoubles) * sizeof(double);
+    return (tiles_offset(N, half) + (size_t)tile_count(N, half) * (kSegDoubles + (half ? kHsDoubles : 0))) *
+           sizeof(double);
 }
 
 static void setup_elements(const double *nodes, const int64_t *tris, int64_t N, double *src, double *recv,
@@ -652,13 +794,13 @@ static void setup_elements(const double *nodes, const int64_t *tris, int64_t N, 
 }
 
 // Receivers per block: the grid's tail costs up to one block's time, so the
-// count (16 .. kSegRecv) with the fewest receivers on a slot's path wins; one
-// extra receiver stands for a block's start.
-static int seg_receivers(int64_t tiles, int64_t rows, int64_t slots)
+// count (a quarter of the most .. the most) with the fewest receivers on a
+// slot's path wins; one extra receiver stands for a block's start.
+static int seg_receivers(int most, int64_t tiles, int64_t rows, int64_t slots)
 {
-    int best = kSegRecv;
+    int best = most;
     int64_t cost = INT64_MAX;
-    for (int nr = kSegRecv; nr >= 16; --nr) {
+    for (int nr = most; nr >= most / 4; --nr) {
         const int64_t waves = (tiles * ((rows + nr - 1) / nr) + slots - 1) / slots;
         const int64_t c = waves * (nr + 1);
         if (c < cost) { cost = c; best = nr; }
@@ -677,11 +819,12 @@ static int seg_config(int *sms)
     int dev;
     PQ3D_CUDA_TRY(cudaGetDevice(&dev));
     if (g_seg.device != dev) {
+        const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
         PQ3D_CUDA_TRY(cudaDeviceGetAttribute(&g_seg.sms, cudaDevAttrMultiProcessorCount, dev));
-        PQ3D_CUDA_TRY(cudaFuncSetAttribute(assemble_seg_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           kSegSmem));
-        PQ3D_CUDA_TRY(cudaFuncSetAttribute(assemble_seg_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           kSegSmem));
+        PQ3D_CUDA_TRY(cudaFuncSetAttribute(assemble_seg_kernel<true>, a, kSegSmem));
+        PQ3D_CUDA_TRY(cudaFuncSetAttribute(assemble_seg_kernel<false>, a, kSegSmem));
+        PQ3D_CUDA_TRY(cudaFuncSetAttribute(assemble_hs_kernel<true>, a, kHsSmem));
+        PQ3D_CUDA_TRY(cudaFuncSetAttribute(assemble_hs_kernel<false>, a, kHsSmem));
         g_seg.device = dev;
     }
     *sms = g_seg.sms;
@@ -694,41 +837,41 @@ static int assemble_rows(const double *nodes, const int64_t *tris, int64_t N, in
 {
     double *src = ws, *recv = src + (size_t)kSrcStride * N;
     double *img = recv + (size_t)kRecvStride * N, *fsc = img + (size_t)kImgStride * N;
-    Tile *tiles = (Tile *)(ws + tiles_offset(N));
-    const int ts = tile_size(N);
+    Tile *tiles = (Tile *)(ws + tiles_offset(N, half));
+    TileHs *hs = half ? (TileHs *)(tiles + tile_count(N, true)) : nullptr;
+    const int ts = tile_size(N, half);
     const int64_t nt = (N + ts - 1) / ts;
     if (do_setup) {
         const int th = 128;
         setup_elements(nodes, tris, N, src, recv, st);
         if (half) setup_hs_kernel<<<(unsigned)((N + th - 1) / th), th, 0, st>>>(nodes, tris, N, img, fsc);
-        else setup_tiles_kernel<<<(unsigned)nt, kTileMax, 0, st>>>(nodes, tris, N, ts, tiles);
+        setup_tiles_kernel<<<(unsigned)nt, kTileMax, 0, st>>>(nodes, tris, N, ts, tiles, hs);
         PQ3D_CUDA_TRY(cudaGetLastError());
     }
     if (row0 == row1) return PQ3D_OK;
-    const double nu = poisson(mu, lam);
-    if (half) {
-        dim3 grid((unsigned)((N + kTJ - 1) / kTJ), (unsigned)((row1 - row0 + kTI - 1) / kTI));
-        if (K32)
-            assemble_dense_hs_kernel<true><<<grid, kTJ, 0, st>>>(src, recv, img, fsc, N, row0, row1, nu, kfac(nu),
-                                                                2.0 * mu, lam, K64, K32);
-        else
-            assemble_dense_hs_kernel<false><<<grid, kTJ, 0, st>>>(src, recv, img, fsc, N, row0, row1, nu, kfac(nu),
-                                                                 2.0 * mu, lam, K64, K32);
-        PQ3D_CUDA_TRY(cudaGetLastError());
-        return PQ3D_OK;
-    }
     int sms = 0;
     const int rc = seg_config(&sms);
     if (rc) return rc;
-    const int nr = seg_receivers(nt, row1 - row0, 2 * (int64_t)sms);
+    const double nu = poisson(mu, lam);
     const SegMat mat = seg_material(nu, 2.0 * mu, lam);
-    dim3 grid((unsigned)nt, (unsigned)((row1 - row0 + nr - 1) / nr));
-    if (K32)
+    const int nr = seg_receivers(half ? kHsRecv : kSegRecv, nt, row1 - row0, 2 * (int64_t)sms);
+    const dim3 grid((unsigned)nt, (unsigned)((row1 - row0 + nr - 1) / nr));
+    if (half) {
+        if (K32)
+            assemble_hs_kernel<true><<<grid, kHsThreads, kHsSmem, st>>>(tiles, hs, ts, src, recv, img, fsc, N, row0,
+                                                                        row1, nr, mat, nu, kfac(nu), 2.0 * mu, lam, K64,
+                                                                        K32);
+        else
+            assemble_hs_kernel<false><<<grid, kHsThreads, kHsSmem, st>>>(tiles, hs, ts, src, recv, img, fsc, N, row0,
+                                                                         row1, nr, mat, nu, kfac(nu), 2.0 * mu, lam,
+                                                                         K64, nullptr);
+    } else if (K32) {
         assemble_seg_kernel<true><<<grid, kSegThreads, kSegSmem, st>>>(tiles, ts, src, recv, N, row0, row1, nr, mat, nu,
                                                                        kfac(nu), 2.0 * mu, lam, K64, K32);
-    else
+    } else {
         assemble_seg_kernel<false><<<grid, kSegThreads, kSegSmem, st>>>(tiles, ts, src, recv, N, row0, row1, nr, mat,
                                                                         nu, kfac(nu), 2.0 * mu, lam, K64, nullptr);
+    }
     PQ3D_CUDA_TRY(cudaGetLastError());
     return PQ3D_OK;
 }
@@ -894,7 +1037,8 @@ extern "C" int pq3d_assemble_dense_host(const double *nodes_host, int64_t n_node
     }
     const size_t ld = 2 * (size_t)N;
     // rows per block: about 256 MB of FP64 output per block
-    int64_t rb = std::max<int64_t>(kTI, ((int64_t)(256u << 20) / (int64_t)(3 * ld * sizeof(double))) / kTI * kTI);
+    int64_t rb = std::max<int64_t>(kSegRecv,
+                                   ((int64_t)(256u << 20) / (int64_t)(3 * ld * sizeof(double))) / kSegRecv * kSegRecv);
     rb = std::min<int64_t>(rb, N);
     double *d_nodes = nullptr, *d_ws = nullptr, *d_K64[2] = {nullptr, nullptr};
     float *d_K32[2] = {nullptr, nullptr};
@@ -985,9 +1129,8 @@ extern "C" int pq3d_gf_setup(const double *nodes, const int64_t *tris, int64_t N
 {
     clear_error();
     PQ3D_REQUIRE(nodes && tris && workspace && N > 0, "pq3d_gf_setup: bad arguments");
-    PQ3D_REQUIRE(workspace_bytes >= (halfspace ? ws_bytes(N, true)
-                                               : (size_t)N * (kSrcStride + kRecvStride) * sizeof(double)) &&
-                     aligned16(workspace), "pq3d_gf_setup: workspace too small");
+    PQ3D_REQUIRE(workspace_bytes >= tables_doubles(N, halfspace != 0) * sizeof(double) && aligned16(workspace),
+                 "pq3d_gf_setup: workspace too small");
     double *src = (double *)workspace;
     double *recv = src + (size_t)kSrcStride * N;
     setup_elements(nodes, tris, N, src, recv, (cudaStream_t)stream);
