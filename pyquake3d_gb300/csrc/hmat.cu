@@ -666,10 +666,14 @@ lowrank_T_kernel(const float *__restrict__ data, const longlong2 *__restrict__ t
 // columns of a pair are four full lines (with all 8 runs of a column together,
 // its loads touched every line of 2 KB four times over).
 //
-// Bound: FP32 issue (2 FMAs per entry and run, one packed f32x2 FMA) beside
-// HBM.  N = 30,000, B = 16: 2.17 ms with a CTA per (leaf, run) -- 16 walks over
-// the blocks from L2, 19 instructions per 192 products -- against 0.27 ms of
-// FMAs and 0.2 ms of HBM.
+// Bound: L2 in the rank rows (the entries once per 4 runs and the x values:
+// 8.3 TB/s), FP32 issue in the leaf rows (2 FMAs per entry and run, one packed
+// f32x2 FMA; 47 % of the FMA pipe) -- beside 0.2 ms of HBM.  N = 30,000,
+// B = 16: 2.17 ms with a CTA per (leaf, run) -- 16 walks over the blocks from L2,
+// 19 instructions per 192 products -- 1.46 ms with 8 runs per entry (rank rows
+// 0.58, leaf rows 0.85), 1.06 ms with the loads kept in flight, the float-float
+// sums of two runs in one instruction and the row passes on two CTAs (0.35 and
+// 0.69).  A second set of registers for the next entries spills: 1.50 ms.
 
 __host__ __device__ inline int group_width(int left) { return left > 4 ? 8 : (left > 2 ? 4 : 2); }
 // slots of n runs (B > 1)
@@ -709,7 +713,49 @@ __device__ __forceinline__ void fma2(uint64_t &acc, uint64_t k, uint64_t x)
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(k), "l"(x));
 }
 
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 typedef ulonglong2 Pair2;   // (hi, lo) of two runs, as f32x2 operands
+
+// ff_add of two runs at once (hi and lo of the two side by side), and with an
+// addend without a low part
+struct __align__(16) FFPair {
+    uint64_t hi, lo;
+};
+__device__ __forceinline__ uint64_t two_sum2(uint64_t a, uint64_t b, uint64_t &e)
+{
+    const uint64_t s = add2(a, b), bb = sub2(s, a);
+    e = add2(sub2(a, sub2(s, bb)), sub2(b, bb));
+    return s;
+}
+__device__ __forceinline__ FFPair ff_close2(uint64_t s, uint64_t l)
+{
+    const uint64_t h = add2(s, l);
+    return FFPair{h, sub2(l, sub2(h, s))};
+}
+__device__ __forceinline__ FFPair ff_add2p(FFPair a, FFPair b)
+{
+    uint64_t e;
+    const uint64_t s = two_sum2(a.hi, b.hi, e);
+    return ff_close2(s, add2(add2(a.lo, b.lo), e));
+}
+__device__ __forceinline__ FFPair ff_add2p(FFPair a, uint64_t b)
+{
+    uint64_t e;
+    const uint64_t s = two_sum2(a.hi, b, e);
+    return ff_close2(s, add2(a.lo, e));
+}
 
 __global__ void permute_split_runs_kernel(const double *__restrict__ X, const int64_t *__restrict__ perm, int64_t N,
                                           const int32_t *__restrict__ list, Pair2 *__restrict__ Xs)
@@ -727,38 +773,47 @@ __global__ void permute_split_runs_kernel(const double *__restrict__ X, const in
     }
 }
 
-// t_row_group for NR runs (pair h of the x values at x + h * xs, of the sums at T + h * ts).  The 4 NR sums
-// are reduced together: at each step of the butterfly a lane keeps half of
-// them (16 additions for 16 sums instead of 80; every sum is added in
-// warp_sum_ff's tree, and the two-sum is symmetric in its operands).
+// t_row_group for NR runs (pair h of the x values at x + h * xs, of the sums at
+// T + h * ts); kept: 2 NR float-float sums a lane in shared memory, stride 32,
+// for rows of more than 1024 columns.  An entry's register takes the column 128
+// further on as soon as it is used, so that loads are always in flight without a
+// second set of registers.  The 4 NR sums are reduced together: at each step
+// of the butterfly a lane keeps half of them (16 additions for 16 sums instead
+// of 80; every sum is added in warp_sum_ff's tree, and the two-sum is symmetric
+// in its operands), two runs in one instruction.
 template <int NR>
 __device__ __forceinline__ void t_row_group_runs(const float *__restrict__ v, int nc, int g, const Pair2 *__restrict__ x,
-                                                 int64_t xs, int lane, Pair2 *__restrict__ T, int64_t ts)
+                                                 int64_t xs, int lane, Pair2 *__restrict__ T, int64_t ts, FFPair *kept)
 {
-    FF sum[4 * NR];
+    constexpr int U = 4, P = 2 * NR;   // columns a lane per step; pairs of sums
+    const float *row[4];               // rows past the group's last repeat it; their sums are not stored
 #pragma unroll
-    for (int q = 0; q < 4 * NR; ++q) sum[q] = FF{0.f, 0.f};
+    for (int j = 0; j < 4; ++j) row[j] = v + (int64_t)min(j, g - 1) * nc + lane;
+    x += lane;
+    float k[U][4];
+    auto load = [&](int u, int c) {   // entries of the column c + lane (past the last: that one, its x is zero)
+        const int cc = min(c, nc - 1 - lane);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) k[u][j] = __ldg(row[j] + cc);
+    };
+    FFPair sum[P];
+#pragma unroll
+    for (int u = 0; u < U; ++u) load(u, 32 * u);
     for (int c0k = 0; c0k < nc; c0k += 1024) {
-        uint64_t a[4 * NR];
+        uint64_t a[2 * P];
 #pragma unroll
-        for (int q = 0; q < 4 * NR; ++q) a[q] = 0ull;
+        for (int q = 0; q < 2 * P; ++q) a[q] = 0ull;
         const int cend = min(nc, c0k + 1024);
-        constexpr int U = 4;   // columns per lane in flight
-        for (int col = c0k + lane; col - lane < cend; col += 32 * U) {
+        for (int c = c0k; c < cend; c += 32 * U) {
+            const bool whole = c + 32 * U <= cend;
             Pair2 xv[U][NR / 2];
-            float k[U][4];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int c = col + 32 * u;
-                const bool ok = c < cend;
-#pragma unroll
-                for (int h = 0; h < NR / 2; ++h)
-                    xv[u][h] = ok ? x[h * xs + c] : make_ulonglong2(0ull, 0ull);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) k[u][j] = (ok && j < g) ? __ldg(v + (int64_t)j * nc + c) : 0.f;
-            }
 #pragma unroll
             for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int h = 0; h < NR / 2; ++h)
+                    xv[u][h] = whole || c + lane + 32 * u < cend ? x[h * xs + c + 32 * u] : make_ulonglong2(0ull, 0ull);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const uint64_t kk = pack2(k[u][j], k[u][j]);
@@ -768,36 +823,53 @@ __device__ __forceinline__ void t_row_group_runs(const float *__restrict__ v, in
                         fma2(a[j * NR + 2 * h + 1], kk, xv[u][h].y);
                     }
                 }
+                load(u, c + 32 * (U + u));
+            }
         }
 #pragma unroll
-        for (int q = 0; q < 4 * NR; ++q) {
-            const float2 p = unpack2(a[q]);
-            sum[q] = ff_add(sum[q], FF{p.x, 0.f});
-            sum[q] = ff_add(sum[q], FF{p.y, 0.f});
+        for (int q = 0; q < P; ++q) {
+            const float2 p0 = unpack2(a[2 * q]), p1 = unpack2(a[2 * q + 1]);
+            const uint64_t s = pack2(p0.x, p1.x), c = pack2(p0.y, p1.y);
+            if (c0k == 0) {
+                sum[q].hi = two_sum2(s, c, sum[q].lo);   // what adding both to zero gives
+            } else {
+                sum[q] = ff_add2p(ff_add2p(kept[32 * q], s), c);
+            }
+            if (cend < nc) kept[32 * q] = sum[q];
         }
     }
     int idx = 0, o = 16;
 #pragma unroll
-    for (int n = 2 * NR; n >= 1; n >>= 1, o >>= 1) {   // n sums stay
+    for (int n = P / 2; n >= 1; n >>= 1, o >>= 1) {   // n pairs stay
         const bool up = (lane & o) != 0;
 #pragma unroll
         for (int q = 0; q < n; ++q) {
-            const FF keep = up ? sum[q + n] : sum[q], give = up ? sum[q] : sum[q + n];
-            FF other;
+            const FFPair keep = up ? sum[q + n] : sum[q], give = up ? sum[q] : sum[q + n];
+            FFPair other;
             other.hi = __shfl_xor_sync(0xffffffffu, give.hi, o);
             other.lo = __shfl_xor_sync(0xffffffffu, give.lo, o);
-            sum[q] = ff_add(keep, other);
+            sum[q] = ff_add2p(keep, other);
         }
         idx = 2 * idx + (up ? 1 : 0);
     }
-    for (int p = o; p > 0; p >>= 1) {
+    FF one;   // the last pair: a run to each half
+    {
+        const bool up = (lane & o) != 0;
+        const float2 h = unpack2(sum[0].hi), l = unpack2(sum[0].lo);
         FF other;
-        other.hi = __shfl_xor_sync(0xffffffffu, sum[0].hi, p);
-        other.lo = __shfl_xor_sync(0xffffffffu, sum[0].lo, p);
-        sum[0] = ff_add(sum[0], other);
+        other.hi = __shfl_xor_sync(0xffffffffu, up ? h.x : h.y, o);
+        other.lo = __shfl_xor_sync(0xffffffffu, up ? l.x : l.y, o);
+        one = ff_add(FF{up ? h.y : h.x, up ? l.y : l.x}, other);
+        idx = 2 * idx + (up ? 1 : 0);
     }
-    if ((lane & (2 * o - 1)) == 0 && idx / NR < g)
-        reinterpret_cast<float2 *>(T + (idx % NR / 2) * ts + idx / NR)[idx & 1] = make_float2(sum[0].hi, sum[0].lo);
+    for (int p = o >> 1; p > 0; p >>= 1) {
+        FF other;
+        other.hi = __shfl_xor_sync(0xffffffffu, one.hi, p);
+        other.lo = __shfl_xor_sync(0xffffffffu, one.lo, p);
+        one = ff_add(one, other);
+    }
+    if ((lane & (o - 1)) == 0 && idx / NR < g)
+        reinterpret_cast<float2 *>(T + (idx % NR / 2) * ts + idx / NR)[idx & 1] = make_float2(one.hi, one.lo);
 }
 
 __global__ void __launch_bounds__(kTWarps * 32, 4)
@@ -807,6 +879,7 @@ lowrank_T_runs_kernel(const float *__restrict__ data, const longlong2 *__restric
                       int64_t t_rows, int nquads, Pair2 *__restrict__ T, const int32_t *__restrict__ list)
 {
     __shared__ FF part[kTWarps];
+    __shared__ FFPair kept[kTWarps][8 * 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int quad = (int)(blockIdx.x % (unsigned)nquads), grp = quad >> 1, half = quad & 1;
     const int64_t cta = blockIdx.x / (unsigned)nquads;
@@ -817,8 +890,8 @@ lowrank_T_runs_kernel(const float *__restrict__ data, const longlong2 *__restric
     Pair2 *Tg = T + (4 * grp + 2 * half) * t_rows;
     if (cta < short_ctas) {
         const int64_t g0 = (cta * kTWarps + wid) * kTGroupsPerWarp;
-        if (g0 >= ngrp) return;
         const int64_t g1 = min(ngrp, g0 + kTGroupsPerWarp);
+        if (g0 >= ngrp) return;
         longlong2 nrec = t_grp[g0];
         for (int64_t gi = g0; gi < g1; ++gi) {
             const longlong2 rec = nrec;
@@ -827,8 +900,8 @@ lowrank_T_runs_kernel(const float *__restrict__ data, const longlong2 *__restric
             const int nc = (int)((rec.x >> 40) & 0xffff), g = (int)(rec.x >> 56);
             const int64_t w0 = (int64_t)((uint64_t)rec.y >> 32);
             const Pair2 *x = xg + (rec.y & 0xffffffffll);
-            if (nr == 4) t_row_group_runs<4>(data + off, nc, g, x, 2 * N, lane, Tg + w0, t_rows);
-            else t_row_group_runs<2>(data + off, nc, g, x, 2 * N, lane, Tg + w0, t_rows);
+            if (nr == 4) t_row_group_runs<4>(data + off, nc, g, x, 2 * N, lane, Tg + w0, t_rows, &kept[wid][lane]);
+            else t_row_group_runs<2>(data + off, nc, g, x, 2 * N, lane, Tg + w0, t_rows, &kept[wid][lane]);
         }
         return;
     }
@@ -1028,11 +1101,14 @@ leaf_rows_kernel(const float *__restrict__ data, const int64_t *__restrict__ off
 // runs), the work columns in the same 8 ranges.  Lanes own up to kRunRows / NR
 // rows (24 f32x2 accumulators a lane).  The x values of 32 columns come into
 // shared memory by asynchronous copies (a lane takes its column's pairs), the
-// next 32 while these are used; the entries of the next 4 columns are loaded
-// while 4 are used; the float-float sums, touched once per block segment, live
-// in shared memory.
+// next 32 while these are used; an entry's register takes the column 8 further
+// on (4 in wide passes) as soon as it is used; the float-float sums, touched
+// once per block segment, live in shared memory.  The row passes of a leaf are
+// independent: two CTAs take every other one (N = 30,000: 512 leaves are 1,024
+// CTAs for 304 places, whose last round was half empty).
 constexpr int kRunRows = 24;
 constexpr int kRunMaxR = 6;
+constexpr int kRunPasses = 2;   // CTAs of a leaf and run group
 constexpr int kRunFF = kRunRows * kThreads * (int)sizeof(float2);                  // float-float sums
 constexpr int kRunX = kWarps * 2 * 32 * 4 * (int)sizeof(Pair2);                    // staged x, two chunks
 constexpr int kRunRed = kWarps * 32 * kRunMaxR * (int)sizeof(double);              // one run's warp sums
@@ -1044,13 +1120,14 @@ __device__ __forceinline__ void copy16_async(void *smem, const void *gmem)
                  : "memory");
 }
 
-// xp: column 0 of the segment's x values (pair h at xp + h * xs)
+// xp: column 0 of the segment's x values (pair h at xp + h * xs); row: offset
+// of the lane's last row in a column (a lane without one repeats the leaf's last)
 template <int R, int NR>
-__device__ __forceinline__ void leaf_segment_runs(const float *__restrict__ col0, int64_t M,
-                                                  const Pair2 *__restrict__ xp, int64_t xs, int ca, int cb, bool last_ok,
-                                                  Pair2 *sx, float2 *ff)
+__device__ __forceinline__ void leaf_segment_runs(const float *__restrict__ col0, int row, int M,
+                                                  const Pair2 *__restrict__ xp, int64_t xs, int ca, int cb, Pair2 *sx,
+                                                  FFPair *ff)
 {
-    constexpr int H = NR / 2, U = 4;
+    constexpr int H = NR / 2, U = R <= 3 ? 8 : 4;   // columns in flight (24 entries a lane)
     const int lane = threadIdx.x & 31;
     uint64_t a[R * NR];
 #pragma unroll
@@ -1061,17 +1138,32 @@ __device__ __forceinline__ void leaf_segment_runs(const float *__restrict__ col0
             for (int h = 0; h < H; ++h) copy16_async(&sx[buf * 32 * H + lane * H + h], xp + h * xs + c0 + lane);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float kn[U][R];
-    auto load = [&](int c) {
+    float k[U][R];
+    const float *coll = col0 + row;
+    auto load = [&](int u, int c) {   // entries of column c (past the last: that one, unused)
+        const int64_t o = min(c, cb - 1) * (int64_t)M;
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int i = 0; i < R - 1; ++i) k[u][i] = __ldg(col0 + o + 32 * i);
+        k[u][R - 1] = __ldg(coll + o);
+    };
+    auto column = [&](int u, const Pair2 *x0) {
+        uint64_t kk[R];
 #pragma unroll
-            for (int i = 0; i < R; ++i)
-                kn[u][i] = (c + u < cb && (i < R - 1 || last_ok)) ? __ldg(col0 + (int64_t)(c + u) * M + 32 * i) : 0.f;
+        for (int i = 0; i < R; ++i) kk[i] = pack2(k[u][i], k[u][i]);
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+            const Pair2 x = x0[h];
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                fma2(a[i * NR + 2 * h], kk[i], x.x);
+                fma2(a[i * NR + 2 * h + 1], kk[i], x.y);
+            }
+        }
     };
     __syncwarp();   // the last segment's chunks have been read
     stage(ca, 0);
-    load(ca);
+#pragma unroll
+    for (int u = 0; u < U; ++u) load(u, ca + u);
     int buf = 0;
     for (int c0 = ca; c0 < cb; c0 += 32, buf ^= 1) {
         stage(c0 + 32, buf ^ 1);
@@ -1079,37 +1171,23 @@ __device__ __forceinline__ void leaf_segment_runs(const float *__restrict__ col0
         __syncwarp();   // this chunk is in, from every lane
         const Pair2 *x0 = sx + buf * 32 * H;
         const int n = min(32, cb - c0);
-        for (int c = 0; c < n; c += U) {
-            float k[U][R];
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-#pragma unroll
-                for (int i = 0; i < R; ++i) k[u][i] = kn[u][i];
-            load(c0 + c + U);
+        int c = 0;
+        for (; c + U <= n; c += U)
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                if (u > 0 && c + u >= n) break;   // uniform
-#pragma unroll
-                for (int h = 0; h < H; ++h) {
-                    const Pair2 x = x0[(c + u) * H + h];
-#pragma unroll
-                    for (int i = 0; i < R; ++i) {
-                        const uint64_t kk = pack2(k[u][i], k[u][i]);
-                        fma2(a[i * NR + 2 * h], kk, x.x);
-                        fma2(a[i * NR + 2 * h + 1], kk, x.y);
-                    }
-                }
+                column(u, x0 + (c + u) * H);
+                load(u, c0 + c + U + u);
             }
-        }
+#pragma unroll
+        for (int u = 0; u < U - 1; ++u)   // the segment's last columns
+            if (c + u < n) column(u, x0 + (c + u) * H);
         __syncwarp();   // the chunk has been read: the next but one goes there
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < R * NR; ++i) {
-        const float2 v = unpack2(a[i]), f = ff[i * kThreads];
-        FF t = ff_add(FF{f.x, f.y}, FF{v.x, 0.f});
-        t = ff_add(t, FF{v.y, 0.f});
-        ff[i * kThreads] = make_float2(t.hi, t.lo);
+    for (int i = 0; i < R * H; ++i) {
+        const float2 v0 = unpack2(a[2 * i]), v1 = unpack2(a[2 * i + 1]);
+        ff[i * kThreads] = ff_add2p(ff_add2p(ff[i * kThreads], pack2(v0.x, v1.x)), pack2(v0.y, v1.y));
     }
 }
 
@@ -1117,10 +1195,10 @@ template <int R, int NR>
 __device__ __forceinline__ void leaf_range_runs(const BlkDesc *desc, const int *wpre, int nq, int64_t lo, int64_t hi,
                                                 int pr0, int prow, const float *__restrict__ data,
                                                 const Pair2 *__restrict__ xg, const Pair2 *__restrict__ Tg,
-                                                int64_t N, int64_t t_rows, Pair2 *sx, float2 *ff)
+                                                int64_t N, int64_t t_rows, Pair2 *sx, FFPair *ff)
 {
     const int lane = threadIdx.x & 31;
-    const bool last_ok = lane + 32 * (R - 1) < prow;
+    const int row = min(32 * (R - 1), prow - 1 - lane);
     int q = 0;
     while (q < nq && wpre[q + 1] <= lo) ++q;
     for (; q < nq && wpre[q] < hi; ++q) {
@@ -1128,8 +1206,8 @@ __device__ __forceinline__ void leaf_range_runs(const BlkDesc *desc, const int *
         const int ca = (int)max((int64_t)0, lo - wpre[q]);
         const int cb = (int)min((int64_t)d.w, hi - wpre[q]);
         if (ca >= cb) continue;
-        leaf_segment_runs<R, NR>(data + d.off + d.row0 + pr0 + lane, d.M, (d.dense ? xg : Tg) + d.x0,
-                                 d.dense ? 2 * N : t_rows, ca, cb, last_ok, sx, ff);
+        leaf_segment_runs<R, NR>(data + d.off + d.row0 + pr0 + lane, row, d.M, (d.dense ? xg : Tg) + d.x0,
+                                 d.dense ? 2 * N : t_rows, ca, cb, sx, ff);
     }
 }
 
@@ -1140,20 +1218,20 @@ __device__ __forceinline__ void leaf_rows_runs(const float *__restrict__ data, c
                                                const int32_t *__restrict__ leaf_blocks, const int64_t *__restrict__ perm,
                                                const Pair2 *__restrict__ xg, const Pair2 *__restrict__ Tg,
                                                const int64_t *__restrict__ t_off, int64_t t_rows, int64_t N, int runs,
-                                               const int32_t *__restrict__ run, double *__restrict__ Y, BlkDesc *desc,
+                                               const int32_t *__restrict__ run, double *__restrict__ Y, int pass0, BlkDesc *desc,
                                                int *wpre, char *smem)
 {
     constexpr int kR = kRunRows / NR < kRunMaxR ? kRunRows / NR : kRunMaxR;
     constexpr int kPass = 32 * kR;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    float2 *ff = reinterpret_cast<float2 *>(smem) + threadIdx.x;
+    FFPair *ff = reinterpret_cast<FFPair *>(smem) + threadIdx.x;
     Pair2 *sx = reinterpret_cast<Pair2 *>(smem + kRunFF) + wid * 2 * 32 * 4;
     double *red = reinterpret_cast<double *>(smem + kRunFF + kRunX);
     const int rows = 3 * (int)(p1 - p0);
-    for (int pr0 = 0; pr0 < rows; pr0 += kPass) {
+    for (int pr0 = pass0 * kPass; pr0 < rows; pr0 += kRunPasses * kPass) {
         const int prow = min(kPass, rows - pr0);
         const int R = (prow + 31) / 32;
-        for (int i = 0; i < kR * NR; ++i) ff[i * kThreads] = make_float2(0.f, 0.f);
+        for (int i = 0; i < kR * NR / 2; ++i) ff[i * kThreads] = FFPair{0ull, 0ull};
         for (int64_t qs = q0; qs < q1; qs += kMaxLeafBlocks) {
             const int nq = (int)min((int64_t)kMaxLeafBlocks, q1 - qs);
             load_leaf_blocks(desc, wpre, nq, qs, p0, off, blk, rank, leaf_blocks, t_off);
@@ -1169,8 +1247,9 @@ __device__ __forceinline__ void leaf_rows_runs(const float *__restrict__ data, c
         for (int j = 0; j < runs; ++j) {
             __syncthreads();
             for (int i = 0; i < kR; ++i) {
-                const float2 f = ff[(i * NR + j) * kThreads];
-                red[wid * kPass + lane + 32 * i] = (double)f.x + (double)f.y;
+                const FFPair f = ff[(i * NR + j) / 2 * kThreads];
+                const float2 h = unpack2(f.hi), l = unpack2(f.lo);
+                red[wid * kPass + lane + 32 * i] = j & 1 ? (double)h.y + (double)l.y : (double)h.x + (double)l.x;
             }
             __syncthreads();
             double *Yr = Y + (int64_t)run[j] * 3 * N;
@@ -1196,7 +1275,9 @@ leaf_rows_runs_kernel(const float *__restrict__ data, const int64_t *__restrict_
     extern __shared__ __align__(16) char smem_runs[];
     __shared__ BlkDesc desc[kMaxLeafBlocks];
     __shared__ int wpre[kMaxLeafBlocks + 1];
-    const int L = (int)(blockIdx.x / (unsigned)ngroups), grp = (int)(blockIdx.x % (unsigned)ngroups);
+    const int grp = (int)(blockIdx.x % (unsigned)ngroups);
+    const unsigned lp = blockIdx.x / (unsigned)ngroups;
+    const int L = (int)(lp / kRunPasses), pass0 = (int)(lp % kRunPasses);
     const int left = list[0] - 8 * grp;
     if (left <= 0) return;   // uniform per CTA
     const int w = group_width(left), runs = min(left, 8);
@@ -1204,14 +1285,14 @@ leaf_rows_runs_kernel(const float *__restrict__ data, const int64_t *__restrict_
     const int32_t *run = list + 1 + 8 * grp;
     const int64_t p0 = leaf[2 * L], p1 = leaf[2 * L + 1], q0 = leaf_ptr[L], q1 = leaf_ptr[L + 1];
     if (w == 8)
-        leaf_rows_runs<8>(data, off, blk, rank, p0, p1, q0, q1, leaf_blocks, perm, xg, Tg, t_off, t_rows, N, runs, run, Y, desc,
-                          wpre, smem_runs);
+        leaf_rows_runs<8>(data, off, blk, rank, p0, p1, q0, q1, leaf_blocks, perm, xg, Tg, t_off, t_rows, N, runs, run, Y, pass0,
+                          desc, wpre, smem_runs);
     else if (w == 4)
-        leaf_rows_runs<4>(data, off, blk, rank, p0, p1, q0, q1, leaf_blocks, perm, xg, Tg, t_off, t_rows, N, runs, run, Y, desc,
-                          wpre, smem_runs);
+        leaf_rows_runs<4>(data, off, blk, rank, p0, p1, q0, q1, leaf_blocks, perm, xg, Tg, t_off, t_rows, N, runs, run, Y, pass0,
+                          desc, wpre, smem_runs);
     else
-        leaf_rows_runs<2>(data, off, blk, rank, p0, p1, q0, q1, leaf_blocks, perm, xg, Tg, t_off, t_rows, N, runs, run, Y, desc,
-                          wpre, smem_runs);
+        leaf_rows_runs<2>(data, off, blk, rank, p0, p1, q0, q1, leaf_blocks, perm, xg, Tg, t_off, t_rows, N, runs, run, Y, pass0,
+                          desc, wpre, smem_runs);
 }
 
 }  // namespace hm
@@ -1372,7 +1453,7 @@ extern "C" int pq3d_hmat_apply_masked(const pq3d_hmat *H, const double *X, int B
             smem_dev = dev;
         }
         PQ3D_REQUIRE((short_ctas + H->t_nlong) * 2 * ngroups < (int64_t)INT32_MAX &&
-                         (int64_t)H->nleaves * ngroups < (int64_t)INT32_MAX && ngroups < 65536,
+                         (int64_t)H->nleaves * ngroups * kRunPasses < (int64_t)INT32_MAX && ngroups < 65536,
                      "pq3d_hmat_apply: too many rank rows or leaves x runs");
         run_list_kernel<<<1, 32, 0, st>>>(B, run_active, active_stride, list);
         permute_split_runs_kernel<<<dim3((unsigned)((2 * N + 255) / 256), (unsigned)ngroups), 256, 0, st>>>(
@@ -1381,7 +1462,7 @@ extern "C" int pq3d_hmat_apply_masked(const pq3d_hmat *H, const double *X, int B
             lowrank_T_runs_kernel<<<(unsigned)((short_ctas + H->t_nlong) * 2 * ngroups), kTWarps * 32, 0, st>>>(
                 H->data, (const longlong2 *)H->t_info, H->t_sched, (const longlong2 *)H->t_grp, H->t_ngrp, nshort,
                 H->t_nlong, short_ctas, Xs, N, H->t_rows, 2 * ngroups, T, list);
-        leaf_rows_runs_kernel<<<(unsigned)(H->nleaves * ngroups), kThreads, kRunSmem, st>>>(
+        leaf_rows_runs_kernel<<<(unsigned)(H->nleaves * ngroups * kRunPasses), kThreads, kRunSmem, st>>>(
             H->data, H->off, H->blk, H->rank, H->leaf, H->leaf_ptr, H->leaf_blocks, H->perm, Xs, T, H->t_off, H->t_rows,
             N, ngroups, list, Y);
         PQ3D_CUDA_TRY(cudaGetLastError());
