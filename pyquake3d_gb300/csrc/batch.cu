@@ -114,7 +114,7 @@ __global__ void prepare_kernel(pq3d_batch_sim S)
             const int64_t stride = (int64_t)S.B * S.N;
             store_base_constants(pb, stride, S.a[idx], S.b[idx], S.dc[idx], S.f0[idx]);
             MixedBase m;
-            store_base_state(pb, stride, S.Tno[idx], S.Tt1o[idx], S.Tt2o[idx], S.state[idx],
+            store_base_state(pb, stride, load_base_constants(pb, stride), S.Tno[idx], S.Tt1o[idx], S.Tt2o[idx], S.state[idx],
                              ff_split(log_eta_v0(S)), m);
             pb[19 * stride] = (float)S.slipv[idx];
         }
@@ -295,11 +295,60 @@ __device__ __forceinline__ void ff_partials(const pq3d_batch_sim &S, int r, int6
 // ---------------------------------------------------------------------------
 // attempt / decide / update
 
+// The mixed attempt of cell i of run r: its inputs as the last update left them
+// (read before chain_wait, from L2), the attempt with the rates of the product,
+// and the accepted state's part of the update: the new constants, the slip rate.
+struct MixedCell {
+    double y[4];
+    float shear, normal;
+    MixedBase m;
+};
+__device__ __forceinline__ MixedCell load_mixed(const pq3d_batch_sim &S, int64_t idx)
+{
+    MixedCell c;
+    c.y[0] = __ldcg(S.Tno + idx); c.y[1] = __ldcg(S.Tt1o + idx); c.y[2] = __ldcg(S.Tt2o + idx); c.y[3] = __ldcg(S.state + idx);
+    c.shear = (float)__ldcg(S.shear_loading + idx);
+    c.normal = (float)__ldcg(S.normal_loading + idx);
+    c.m = load_base(S.base + idx, (int64_t)S.B * S.N);
+    return c;
+}
+__device__ __forceinline__ void attempt_mixed(const pq3d_batch_sim &S, int r, int64_t i, MixedCell &c, float h, float V0,
+                                              double yo[4], float &f1, float &f2)
+{
+    FF q[3];
+    ff_partials(S, r, i, q);
+    const float dsig = S.fix_Tn ? c.normal : (q[2].hi + (q[2].lo + c.normal));
+    c.m.V0 = V0;
+    c.m.dsf = dsig;
+    c.m.L[0] = (c.shear - q[0].hi) - q[0].lo;
+    c.m.L[1] = (c.shear - q[1].hi) - q[1].lo;
+    dp_attempt_mixed(c.m, dsig, h, c.y, yo, f1, f2);
+}
+__device__ __forceinline__ void update_mixed(const pq3d_batch_sim &S, int64_t idx, const BaseConst &k, const double y[4],
+                                             FF c0, float inv_eta, double &v1, double &v2, double &v)
+{
+    float *pb = S.base + idx;
+    const int64_t stride = (int64_t)S.B * S.N;
+    MixedBase m;
+    store_base_state(pb, stride, k, y[0], y[1], y[2], y[3], c0, m);
+    const float f1 = base_slip_rate(m, 0, inv_eta), f2 = base_slip_rate(m, 1, inv_eta);
+    // |V| without under/overflow of the squares
+    const float p = fmaxf(fabsf(f1), fabsf(f2)), q = fminf(fabsf(f1), fabsf(f2));
+    const float t = p > 0.f ? q / p : 0.f;
+    const float vf = fmaxf(p * sqrtf(fmaf(t, t, 1.f)), 1e-30f);
+    pb[19 * stride] = vf;
+    v1 = f1; v2 = f2; v = vf;
+}
+
 // kFF: the float-float attempt (attempt64 = 2), with its own launch bounds
 // (3 CTAs per SM: its float-float chains are latency bound, not register bound)
 template <bool kMixed, bool kFF = false>
 __global__ void __launch_bounds__(256, kMixed ? 4 : (kFF ? 3 : 2)) attempt_kernel(pq3d_batch_sim S)
 {
+    // What the previous iteration left (the product that runs before this
+    // kernel has waited for it) is read while the product ends; its rates after.
+    // All reads before chain_wait go to L2 (__ldcg).
+    chain_release();
     __shared__ unsigned long long red[32];
     __shared__ int act;
     __shared__ double hs;
@@ -309,8 +358,8 @@ __global__ void __launch_bounds__(256, kMixed ? 4 : (kFF ? 3 : 2)) attempt_kerne
     const int r = blockIdx.y;
     pq3d_run_ctrl *C = S.ctrl + r;
     if (threadIdx.x == 0) {
-        act = C->active;
-        hs = C->h;
+        act = __ldcg(&C->active);
+        hs = __ldcg(&C->h);
         if (kMixed) {
             hsf = (float)hs;
             V0f = (float)S.V0;
@@ -320,36 +369,35 @@ __global__ void __launch_bounds__(256, kMixed ? 4 : (kFF ? 3 : 2)) attempt_kerne
     }
     if (kFF && threadIdx.x < 64) etab[threadIdx.x] = ffv(kExp2Tab.v[threadIdx.x]);
     __syncthreads();
-    if (!act) return;
+    if (!act) { chain_wait(); return; }   // no kernel of the chain ends before the one ahead of it
     const int64_t N = S.N;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t idx = (int64_t)r * N + (i < N ? i : N - 1);
+    const int Bp = padded_runs(S.B);
+    double y[4], normal;
+    MixedCell mc;
+    Cell c;
+    if (kMixed) {
+        mc = load_mixed(S, idx);
+    } else {
+        y[0] = __ldcg(S.Tno + idx); y[1] = __ldcg(S.Tt1o + idx); y[2] = __ldcg(S.Tt2o + idx); y[3] = __ldcg(S.state + idx);
+        normal = __ldcg(S.normal_loading + idx);
+        c = Cell{__ldcg(S.a + idx), __ldcg(S.b + idx), __ldcg(S.dc + idx), __ldcg(S.f0 + idx),
+                 __ldcg(S.shear_loading + idx), __ldcg(S.slipv + idx), 0.0, 0.0, 0.0, 0.0, 0.0};
+    }
+    chain_wait();
     double m1 = 0.0, m2 = 0.0;
     float f1 = 0.f, f2 = 0.f;
     if (i < N) {
-        const int64_t idx = (int64_t)r * N + i;
-        const int Bp = padded_runs(S.B);
-        const double y[4] = {S.Tno[idx], S.Tt1o[idx], S.Tt2o[idx], S.state[idx]};
         double yo[4];
         if (kMixed) {
-            FF q[3];
-            ff_partials(S, r, i, q);
-            MixedBase m = load_base(S.base + idx, (int64_t)S.B * N);
-            const float shear = (float)S.shear_loading[idx];
-            const float dsig = S.fix_Tn ? (float)S.normal_loading[idx]
-                                        : (q[2].hi + (q[2].lo + (float)S.normal_loading[idx]));
-            m.V0 = V0f;
-            m.dsf = dsig;
-            m.L[0] = (shear - q[0].hi) - q[0].lo;
-            m.L[1] = (shear - q[1].hi) - q[1].lo;
-            dp_attempt_mixed(m, dsig, hsf, y, yo, f1, f2);
+            attempt_mixed(S, r, i, mc, hsf, V0f, yo, f1, f2);
         } else if (kFF) {
             // float-float attempt: the rates stay float-float (no FP64 sums)
             FF q[3];
             ff_partials(S, r, i, q);
-            const FF nl = ff_split_fast(S.normal_loading[idx]);
+            const FF nl = ff_split_fast(normal);
             const FFRates fr{q[0], q[1], S.fix_Tn ? nl : ff_add2(q[2], nl)};
-            const Cell c{S.a[idx], S.b[idx], S.dc[idx], S.f0[idx], S.shear_loading[idx], S.slipv[idx], 0.0, 0.0, 0.0,
-                         0.0, 0.0};
             dp_attempt_ff(c, fr, S.V0, lnev, hs, y, yo, m1, m2, etab);
         } else {
             double q0 = 0.0, q1 = 0.0, q2 = 0.0;
@@ -372,9 +420,9 @@ __global__ void __launch_bounds__(256, kMixed ? 4 : (kFF ? 3 : 2)) attempt_kerne
                     q0 += p[0]; q1 += p[1]; q2 += p[2];
                 }
             }
-            const double dsig = S.fix_Tn ? S.normal_loading[idx] : q2 + S.normal_loading[idx];
-            const Cell c{S.a[idx], S.b[idx], S.dc[idx], S.f0[idx], S.shear_loading[idx], S.slipv[idx], q0, q1, dsig,
-                         0.0, 0.0};
+            c.AdotV1 = q0;
+            c.AdotV2 = q1;
+            c.dsig = S.fix_Tn ? normal : q2 + normal;
             // the FP64 precision keeps the reference formula (it is the arm the
             // others are compared with); the FP64 attempt of the mixed
             // products (attempt64 = 1) takes the reciprocal form, the
@@ -403,22 +451,24 @@ __global__ void __launch_bounds__(256, kMixed ? 4 : (kFF ? 3 : 2)) attempt_kerne
     }
 }
 
-__global__ void decide_kernel(pq3d_run_ctrl *ctrl, int B)
+// One error's part of the decision: its ratio to the tolerance and the step size
+// it asks for (a division and a pow, microseconds of FP64 latency: two lanes
+// take the two errors side by side).
+__device__ __forceinline__ void step_size(unsigned long long err_bits, double h, double &c, double &hn)
 {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= B) return;
-    pq3d_run_ctrl *C = ctrl + r;
-    if (!C->active) { C->accepted = 0; return; }
-    const double err1 = __longlong_as_double((long long)C->err1_bits) + 1e-10;
-    const double err2 = __longlong_as_double((long long)C->err2_bits) + 1e-10;
+    const double err = __longlong_as_double((long long)err_bits) + 1e-10;
+    c = err / kRelTol;
+    hn = h * 0.9 * pow(kRelTol / err, 0.2);
+}
+__device__ __forceinline__ bool accepts(double c1, double c2) { return fmax(c1, c2) < 1.0 && !(isnan(c1) || isnan(c2)); }
+
+// The control record after an attempt of an active run with the step h.
+__device__ __forceinline__ void decide(pq3d_run_ctrl *C, double h, bool accepted, double hn1, double hn2)
+{
     C->err1_bits = 0ull;
     C->err2_bits = 0ull;
-    const double h = C->h;
     C->attempts += 1;
-    const double c1 = err1 / kRelTol, c2 = err2 / kRelTol;
-    const double hn1 = h * 0.9 * pow(kRelTol / err1, 0.2);
-    const double hn2 = h * 0.9 * pow(kRelTol / err2, 0.2);
-    if (fmax(c1, c2) < 1.0 && !(isnan(c1) || isnan(c2))) {
+    if (accepted) {
         C->accepted = 1;
         C->h_last = h;
         C->time = C->time + h;
@@ -438,6 +488,22 @@ __global__ void decide_kernel(pq3d_run_ctrl *ctrl, int B)
     }
 }
 
+// two neighbouring lanes per run; the even one decides
+__global__ void __launch_bounds__(128) decide_kernel(pq3d_run_ctrl *ctrl, int B)
+{
+    chain_release();
+    chain_wait();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, r = t >> 1;
+    pq3d_run_ctrl *C = ctrl + (r < B ? r : B - 1);
+    const double h = C->h;
+    double c1, hn1;
+    step_size(t & 1 ? C->err2_bits : C->err1_bits, h, c1, hn1);
+    const double c2 = __shfl_down_sync(0xffffffffu, c1, 1), hn2 = __shfl_down_sync(0xffffffffu, hn1, 1);
+    if (r >= B || (t & 1)) return;
+    if (C->active) decide(C, h, accepts(c1, c2), hn1, hn2);
+    else C->accepted = 0;
+}
+
 // The update kernel packs the BF16x18 right-hand side itself when the packed
 // columns follow the cells (no cell order, one shard): its 256-cell blocks are
 // then two whole 256-column spans, and a rejected run keeps its packed v'.
@@ -455,6 +521,8 @@ __host__ __device__ inline bool fused_rhs_pack(const pq3d_batch_sim &S)
 template <bool kMixed>
 __global__ void __launch_bounds__(256) update_kernel(pq3d_batch_sim S)
 {
+    // constants before the wait
+    chain_release();
     __shared__ int acc;
     __shared__ double hs, lnv0;
     __shared__ float inv_eta, c0hi, c0lo;
@@ -463,8 +531,6 @@ __global__ void __launch_bounds__(256) update_kernel(pq3d_batch_sim S)
     const pq3d_run_ctrl *C = S.ctrl + r;
     const bool ffu = !kMixed && S.attempt64 == 2 && S.precision != PQ3D_BATCH_FP64;
     if (threadIdx.x == 0) {
-        acc = C->accepted;
-        hs = C->h_last;
         if (kMixed) {
             const FF c0 = ff_split(log_eta_v0(S));
             c0hi = c0.hi;
@@ -475,32 +541,29 @@ __global__ void __launch_bounds__(256) update_kernel(pq3d_batch_sim S)
         }
     }
     if (ffu && threadIdx.x < 64) etab[threadIdx.x] = ffv(kExp2Tab.v[threadIdx.x]);
-    __syncthreads();
-    if (!acc) return;
     const int64_t N = S.N;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t idx = (int64_t)r * N + (i < N ? i : N - 1);
+    chain_wait();
+    if (threadIdx.x == 0) {
+        acc = C->accepted;
+        hs = C->h_last;
+    }
+    __syncthreads();
+    if (!acc) return;
     const bool fuse = fused_rhs_pack(S);
     if (i >= N && !fuse) return;
     double p1 = 0.0, p2 = 0.0;   // the cell's v' (fused packing; zero past the last cell)
     if (i < N) {
-        const int64_t idx = (int64_t)r * N + i;
         const double h = hs;
         const double4_16a y = reinterpret_cast<const double4_16a *>(S.cand)[idx];
         const double Tno = y.x, T1 = y.y, T2 = y.z, st = y.w;
         S.Tno[idx] = Tno; S.Tt1o[idx] = T1; S.Tt2o[idx] = T2; S.state[idx] = st;
         double v1, v2, v;
         if (kMixed) {
-            float *pb = S.base + idx;
-            const int64_t stride = (int64_t)S.B * N;
-            MixedBase m;
-            store_base_state(pb, stride, Tno, T1, T2, st, FF{c0hi, c0lo}, m);
-            const float f1 = base_slip_rate(m, 0, inv_eta), f2 = base_slip_rate(m, 1, inv_eta);
-            // |V| without under/overflow of the squares
-            const float p = fmaxf(fabsf(f1), fabsf(f2)), q = fminf(fabsf(f1), fabsf(f2));
-            const float t = p > 0.f ? q / p : 0.f;
-            const float vf = fmaxf(p * sqrtf(fmaf(t, t, 1.f)), 1e-30f);
-            pb[19 * stride] = vf;
-            v1 = f1; v2 = f2; v = vf;
+            const double yn[4] = {Tno, T1, T2, st};
+            update_mixed(S, idx, load_base_constants(S.base + idx, (int64_t)S.B * N), yn, FF{c0hi, c0lo}, inv_eta, v1, v2,
+                         v);
         } else if (ffu) {
             // the float-float arm: 2 V0 e^{-psi/a} sinh(x) = sign(x) V0 e^{-psi/a + |x|} (1 - e^{-2|x|}),
             // x = tau / (a sigma), the exponent argument in FP64 (reduced), the rest float-float
@@ -521,10 +584,11 @@ __global__ void __launch_bounds__(256) update_kernel(pq3d_batch_sim S)
         S.slipv1[idx] = v1; S.slipv2[idx] = v2; S.slipv[idx] = v;
         S.slip1[idx] += v1 * h;
         S.slip2[idx] += v2 * h;
-        write_vop<!kMixed>(S, r, i, v1 - S.Vpl * S.cos_rake0[idx], v2 - S.Vpl * S.sin_rake0[idx]);
+        const double cr = S.cos_rake0[idx], sr = S.sin_rake0[idx];
+        write_vop<!kMixed>(S, r, i, v1 - S.Vpl * cr, v2 - S.Vpl * sr);
         if (fuse) {
-            p1 = fma(-S.Vpl, S.cos_rake0[idx], v1);
-            p2 = fma(-S.Vpl, S.sin_rake0[idx], v2);
+            p1 = fma(-S.Vpl, cr, v1);
+            p2 = fma(-S.Vpl, sr, v2);
         }
     }
     if (fuse) {
@@ -543,10 +607,142 @@ __global__ void __launch_bounds__(256) update_kernel(pq3d_batch_sim S)
     }
 }
 
+// Small meshes: attempt, decision and update of a run by one cluster, a cell per
+// thread, the candidate state in registers and the blocks' errors through
+// distributed shared memory.  One warp more than the cells need takes the
+// decision: the cells go on as soon as it knows whether the step is accepted,
+// while it works out the next step size (rank 0's writes the control record).
+//
+// Bound: latency (two kernel boundaries, three trips to the control record and
+// the candidate through L2 gone).  N = 2,000, B = 16, BF16X6: iteration 47.8 us
+// as three kernels, 38.9 us, of which the product takes 23.5.
+constexpr int kStepCluster = 8;   // blocks of a run at most
+constexpr int kStepCells = 512;   // cells of a block at most
+
+__device__ __forceinline__ unsigned peer_shared(const unsigned *p, int rank)
+{
+    unsigned at = (unsigned)__cvta_generic_to_shared(p), v;
+    asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(at) : "r"(rank));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+    return v;
+}
+
+template <int kCells>
+__global__ void __launch_bounds__(kCells + 32) step_cluster_kernel(pq3d_batch_sim S)
+{
+    chain_release();
+    __shared__ unsigned red[32], err[2];
+    __shared__ int act, acc;
+    __shared__ double hs;
+    __shared__ float inv_eta, c0hi, c0lo;
+    const int r = blockIdx.y, rank = blockIdx.x;   // the cluster is the row of the grid
+    const int t = threadIdx.x - kCells;            // lane of the deciding warp
+    pq3d_run_ctrl *C = S.ctrl + r;
+    if (t == 0) {
+        act = __ldcg(&C->active);
+        hs = __ldcg(&C->h);
+    }
+    if (threadIdx.x == 0) {
+        const FF c0 = ff_split(log_eta_v0(S));
+        c0hi = c0.hi;
+        c0lo = c0.lo;
+        inv_eta = (float)(1.0 / S.eta);
+    }
+    __syncthreads();
+    if (!act) {
+        chain_wait();
+        if (rank == 0 && t == 0) C->accepted = 0;
+        return;   // uniform over the cluster
+    }
+    const int64_t N = S.N;
+    const int per = (int)((N + gridDim.x - 1) / gridDim.x + 31) / 32 * 32;   // an even share of whole warps
+    const int64_t i = rank * (int64_t)per + threadIdx.x;
+    const bool on = (int)threadIdx.x < per && i < N;
+    const int64_t idx = (int64_t)r * N + (on ? i : N - 1);
+    const double h = hs;
+    MixedCell mc = load_mixed(S, idx);
+    const BaseConst k = load_base_constants(S.base + idx, (int64_t)S.B * N);
+    const double slip1 = __ldcg(S.slip1 + idx), slip2 = __ldcg(S.slip2 + idx);
+    const double cr = __ldcg(S.cos_rake0 + idx), sr = __ldcg(S.sin_rake0 + idx);
+    // errors of attempts not decided on (0 unless an iteration was begun and not ended)
+    const unsigned long long before = __ldcg((const unsigned long long *)(t & 1 ? &C->err2_bits : &C->err1_bits));
+    chain_wait();
+    double yo[4];
+    float f1 = 0.f, f2 = 0.f;
+    if (on) attempt_mixed(S, r, i, mc, (float)h, (float)S.V0, yo, f1, f2);
+    const unsigned b1 = block_max_bits32(f1, red);
+    const unsigned b2 = block_max_bits32(f2, red);
+    if (threadIdx.x == 0) { err[0] = b1; err[1] = b2; }
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    unsigned long long e = 0ull;
+    if (t >= 0) {   // even lanes the first error, odd ones the second
+        unsigned b = 0u;
+        for (int q = 0; q < (int)gridDim.x; ++q) b = max(b, peer_shared(&err[t & 1], q));
+        e = max(before, dbits((double)__uint_as_float(b)));
+        // accepts() without its quotients: err / tol rounds to less than 1 just if err < tol
+        const bool below = __longlong_as_double((long long)e) + 1e-10 < kRelTol;
+        const bool all = __all_sync(0xffffffffu, below);
+        if (t == 0) acc = all;
+    }
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");   // no block leaves while its errors are read
+    __syncthreads();
+    if (t >= 0 && rank == 0) {
+        double c1, hn1;
+        step_size(e, h, c1, hn1);
+        const double hn2 = __shfl_down_sync(0xffffffffu, hn1, 1);
+        if (t == 0) decide(C, h, acc, hn1, hn2);
+    }
+    if (acc && on) {
+        S.Tno[idx] = yo[0]; S.Tt1o[idx] = yo[1]; S.Tt2o[idx] = yo[2]; S.state[idx] = yo[3];
+        double v1, v2, v;
+        update_mixed(S, idx, k, yo, FF{c0hi, c0lo}, inv_eta, v1, v2, v);
+        if (v < 1e-30) v = 1e-30;
+        S.slipv1[idx] = v1; S.slipv2[idx] = v2; S.slipv[idx] = v;
+        S.slip1[idx] = slip1 + v1 * h;
+        S.slip2[idx] = slip2 + v2 * h;
+        write_vop<false>(S, r, i, v1 - S.Vpl * cr, v2 - S.Vpl * sr);
+    }
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
 // The Dormand-Prince attempt and update in mixed precision (FP32 stages on the
 // FP64 state), or in the reference FP64 arithmetic: always for the FP64
 // product, on request (attempt64) for the others.
 static bool mixed_attempt(const pq3d_batch_sim &S) { return S.precision != PQ3D_BATCH_FP64 && !S.attempt64; }
+
+// Blocks of a run in the one-cluster form, 0 where the three kernels are the
+// better ones: a run's blocks want SMs of their own (the FP64 conversions of a
+// cell are a third of its time), and a full chip leaves no room to place
+// clusters.  us an iteration of the BF16X6 product, cluster / three kernels:
+// N = 2,000: B = 16 45.6 / 51.5, B = 64 68.3 / 66.4, B = 200 154 / 124;
+// N = 1,000: B = 30 27.9 / 30.6, B = 38 (152 blocks) 34.6 / 32.1; N = 4,000 (512
+// cells a block): B = 9 108.8 / 114.6, B = 19 126.5 / 121.9.
+static int step_clusters(const pq3d_batch_sim &S, int sms)
+{
+    if (!mixed_attempt(S) || S.precision == PQ3D_BATCH_BF16X18 || S.N > kStepCluster * kStepCells) return 0;
+    int n = 1;
+    while (n < kStepCluster && n * (kStepCells / 2) < S.N) n *= 2;
+    return (int64_t)S.B * n <= (S.N <= n * (kStepCells / 2) ? sms * 7 / 8 : sms / 2) ? n : 0;
+}
+
+static int launch_step_cluster(const pq3d_batch_sim &S, int blocks, cudaStream_t st)
+{
+    const bool half = S.N <= blocks * (kStepCells / 2);
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)blocks;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks, (unsigned)S.B);
+    cfg.blockDim = dim3((half ? kStepCells / 2 : kStepCells) + 32);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    PQ3D_CUDA_TRY(cudaLaunchKernelEx(&cfg, half ? step_cluster_kernel<kStepCells / 2> : step_cluster_kernel<kStepCells>, S));
+    return PQ3D_OK;
+}
 
 static int check_sim(const pq3d_batch_sim *S)
 {
@@ -610,17 +806,12 @@ extern "C" int pq3d_batch_prepare(const pq3d_batch_sim *sim, void *stream)
     return PQ3D_OK;
 }
 
-extern "C" int pq3d_batch_iterate_begin(const pq3d_batch_sim *sim, void *workspace, size_t workspace_bytes,
-                                        void *stream)
+// 1. operator product of an iteration (a checked simulation)
+static int product(const pq3d_batch_sim &S, void *workspace, size_t workspace_bytes, cudaStream_t st)
 {
-    clear_error();
-    int rc = check_sim(sim);
-    if (rc) return rc;
-    cudaStream_t st = (cudaStream_t)stream;
-    const pq3d_batch_sim &S = *sim;
+    int rc;
     const int Bp = padded_runs(S.B);
     const int64_t Nt = total_cells(S);
-    // 1. operator product
     if (S.precision == PQ3D_BATCH_FP64) {
         const int64_t warps = S.N * Bp;
         gemm_f64_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, st>>>(
@@ -648,16 +839,29 @@ extern "C" int pq3d_batch_iterate_begin(const pq3d_batch_sim *sim, void *workspa
         // inactive runs (free slots, finished runs) skip the product
         rc = pq3d_hmat_apply_masked((const pq3d_hmat *)S.K, (const double *)S.vop, S.B, S.rates, &S.ctrl[0].active,
                                     (int)(sizeof(pq3d_run_ctrl) / sizeof(int32_t)), workspace, workspace_bytes,
-                                    stream);
+                                    (void *)st);
         if (rc) return rc;
     }
     PQ3D_CUDA_TRY(cudaGetLastError());
+    return PQ3D_OK;
+}
+
+extern "C" int pq3d_batch_iterate_begin(const pq3d_batch_sim *sim, void *workspace, size_t workspace_bytes,
+                                        void *stream)
+{
+    clear_error();
+    int rc = check_sim(sim);
+    if (rc) return rc;
+    cudaStream_t st = (cudaStream_t)stream;
+    const pq3d_batch_sim &S = *sim;
+    rc = product(S, workspace, workspace_bytes, st);
+    if (rc) return rc;
     // 2. attempt (FP64 arm: the reference arithmetic; mixed arms: dp_attempt_mixed)
     dim3 grid((unsigned)((S.N + 255) / 256), (unsigned)S.B);
-    if (mixed_attempt(S)) attempt_kernel<true><<<grid, 256, 0, st>>>(S);
-    else if (S.attempt64 == 2 && S.precision != PQ3D_BATCH_FP64) attempt_kernel<false, true><<<grid, 256, 0, st>>>(S);
-    else attempt_kernel<false><<<grid, 256, 0, st>>>(S);
-    PQ3D_CUDA_TRY(cudaGetLastError());
+    PQ3D_CUDA_TRY(launch_chained(mixed_attempt(S) ? attempt_kernel<true>
+                                 : S.attempt64 == 2 && S.precision != PQ3D_BATCH_FP64 ? attempt_kernel<false, true>
+                                                                                      : attempt_kernel<false>,
+                                 grid, 256, 0, st, S));
     return PQ3D_OK;
 }
 
@@ -669,11 +873,9 @@ extern "C" int pq3d_batch_iterate_end(const pq3d_batch_sim *sim, void *stream)
     cudaStream_t st = (cudaStream_t)stream;
     const pq3d_batch_sim &S = *sim;
     // 3-4. decide, update
-    decide_kernel<<<(S.B + 127) / 128, 128, 0, st>>>(S.ctrl, S.B);
+    PQ3D_CUDA_TRY(launch_chained(decide_kernel, (2 * S.B + 127) / 128, 128, 0, st, S.ctrl, S.B));
     dim3 grid((unsigned)((S.N + 255) / 256), (unsigned)S.B);
-    if (mixed_attempt(S)) update_kernel<true><<<grid, 256, 0, st>>>(S);
-    else update_kernel<false><<<grid, 256, 0, st>>>(S);
-    PQ3D_CUDA_TRY(cudaGetLastError());
+    PQ3D_CUDA_TRY(launch_chained(mixed_attempt(S) ? update_kernel<true> : update_kernel<false>, grid, 256, 0, st, S));
     if (S.precision == PQ3D_BATCH_BF16X18 && !fused_rhs_pack(S))   // v' of every run from its slip rates
         return fx::pack_rhs_from_state(S.slipv1, S.slipv2, S.cos_rake0, S.sin_rake0, S.Vpl, S.fix_order, S.N, S.B,
                                        S.vop, st);
@@ -682,6 +884,22 @@ extern "C" int pq3d_batch_iterate_end(const pq3d_batch_sim *sim, void *stream)
 
 extern "C" int pq3d_batch_iterate(const pq3d_batch_sim *sim, void *workspace, size_t workspace_bytes, void *stream)
 {
-    const int rc = pq3d_batch_iterate_begin(sim, workspace, workspace_bytes, stream);
+    clear_error();
+    int rc = check_sim(sim);
+    if (rc) return rc;
+    const pq3d_batch_sim &S = *sim;
+    static thread_local int sms_dev = -1, sms = 0;
+    int dev;
+    PQ3D_CUDA_TRY(cudaGetDevice(&dev));
+    if (sms_dev != dev) {
+        PQ3D_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        sms_dev = dev;
+    }
+    const int blocks = step_clusters(S, sms);
+    if (blocks > 0) {
+        rc = product(S, workspace, workspace_bytes, (cudaStream_t)stream);
+        return rc ? rc : launch_step_cluster(S, blocks, (cudaStream_t)stream);
+    }
+    rc = pq3d_batch_iterate_begin(sim, workspace, workspace_bytes, stream);
     return rc ? rc : pq3d_batch_iterate_end(sim, stream);
 }

@@ -29,6 +29,32 @@ void clear_error();
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Launch that may start before the stream's previous kernel has ended, if that
+// kernel lets it (chain_release by all its blocks); the kernel must call
+// chain_wait, in every block, before it touches anything an earlier kernel
+// reads or writes: the previous kernel is then complete, and with it everything
+// before it.  A small batched iteration is four kernels of 5-10 us, so launch
+// latency and prologues are a visible part of it.
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+
 // Iteration cap of every device-side spin wait (each iteration sleeps ~1 us,
 // so a wait gives up after roughly two seconds).
 constexpr unsigned kSpinLimit = 1u << 21;

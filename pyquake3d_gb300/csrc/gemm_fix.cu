@@ -222,6 +222,8 @@ gemm_fix_kernel(const uint8_t *__restrict__ Kp, const uint8_t *__restrict__ Vp, 
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = *(volatile uint32_t *)tmem_slot;
+    chain_wait();
+    chain_release();   // from here on the previous iteration is complete: the attempt may read its state
 
     if (warp == 0) {
         if (lane == 0) {
@@ -529,9 +531,8 @@ int gemm_bf16x18(const void *Kpacked, const void *Vpacked, int64_t N, int B, int
         balanced = bal_owner((t + 1) * KB - 1, W, G) - bal_owner(t * KB, W, G) + 1 <= nsplit;
     const FixSched sc{KB, balanced ? W : 0, nsplit};
     const dim3 grid = balanced ? dim3((unsigned)G) : dim3((unsigned)tiles, (unsigned)nsplit);
-    gemm_fix_kernel<<<grid, kThreads, smem, stream>>>((const uint8_t *)Kpacked, (const uint8_t *)Vpacked, N, Bq, Bo,
-                                                      sc, out, (int *)workspace, stages);
-    PQ3D_CUDA_TRY(cudaGetLastError());
+    PQ3D_CUDA_TRY(launch_chained(gemm_fix_kernel, grid, kThreads, smem, stream, (const uint8_t *)Kpacked,
+                                 (const uint8_t *)Vpacked, N, Bq, Bo, sc, out, (int *)workspace, stages));
     return PQ3D_OK;
 }
 

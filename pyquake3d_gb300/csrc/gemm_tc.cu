@@ -89,15 +89,30 @@ gemm_bf16x6_kernel(const uint8_t *__restrict__ Kp, const uint8_t *__restrict__ V
     tc_fence_after();
     const uint32_t tmem = *(volatile uint32_t *)tmem_slot;
 
+    // the first stages' operator images, which no kernel of an iteration writes,
+    // come in while the previous kernel ends
+    const int early = nkb < stages ? nkb : stages;
+    if (warp == 0 && lane == 0)
+        for (int it = 0; it < early; ++it) {
+            mbar_expect_tx(full0 + 8 * it, stage_bytes);
+            bulk_g2s(smem_u32(smem + (size_t)it * stage_bytes), Kp + (size_t)(mt * KB + kb0 + it) * a_bytes, a_bytes,
+                     full0 + 8 * it);
+        }
+    __syncwarp();
+    chain_wait();
+    chain_release();   // from here on the previous iteration is complete: the attempt may read its state
+
     if (warp == 0 && lane == 0) {
         // producer: two bulk copies per stage
         for (int it = 0; it < nkb; ++it) {
             const int st = it % stages, use = it / stages;
-            if (!mbar_wait(empty0 + 8 * st, (use & 1) ^ 1)) { atomicExch(err, 1); break; }
             const uint32_t sa = smem_u32(smem + (size_t)st * stage_bytes);
             const int64_t kb = kb0 + it;
-            mbar_expect_tx(full0 + 8 * st, stage_bytes);
-            bulk_g2s(sa, Kp + (size_t)(mt * KB + kb) * a_bytes, a_bytes, full0 + 8 * st);
+            if (it >= early) {
+                if (!mbar_wait(empty0 + 8 * st, (use & 1) ^ 1)) { atomicExch(err, 1); break; }
+                mbar_expect_tx(full0 + 8 * st, stage_bytes);
+                bulk_g2s(sa, Kp + (size_t)(mt * KB + kb) * a_bytes, a_bytes, full0 + 8 * st);
+            }
             bulk_g2s(sa + a_bytes, Vp + (size_t)kb * b_bytes, b_bytes, full0 + 8 * st);
         }
     } else if (warp == 1 && lane == 0) {
@@ -241,9 +256,8 @@ int gemm_bf16x6(const void *Kpacked, const void *Vpacked, int64_t N, int Bp, int
     const size_t stage_bytes = (size_t)kPieces * (kImageA + (size_t)Bp * kBlockK * 2);
     const size_t smem = (size_t)stages * stage_bytes + 16 * (size_t)stages + 16;
     dim3 grid((unsigned)m_tiles(N), (unsigned)nsplit);
-    gemm_bf16x6_kernel<<<grid, 128, smem, stream>>>((const uint8_t *)Kpacked, (const uint8_t *)Vpacked, N, Bp, nsplit,
-                                                     out, (int *)workspace, stages);
-    PQ3D_CUDA_TRY(cudaGetLastError());
+    PQ3D_CUDA_TRY(launch_chained(gemm_bf16x6_kernel, grid, 128, smem, stream, (const uint8_t *)Kpacked,
+                                 (const uint8_t *)Vpacked, N, Bp, nsplit, out, (int *)workspace, stages));
     return PQ3D_OK;
 }
 

@@ -244,12 +244,18 @@ __device__ __forceinline__ void store_base_constants(float *p, int64_t stride, d
 // The state-dependent constants (fields 0-14) of the state (Tn0, T1, T2, psi)
 // (MPa, MPa, MPa, state), in float-float from the FP64 state: the FP64 work is
 // the four splits.  c0 = ln(eta V0) as float-float.
-__device__ __forceinline__ void store_base_state(float *p, int64_t stride, double Tn0, double T1, double T2,
-                                                 double psi, FF c0, MixedBase &m)
+struct BaseConst {
+    FF ia, ib, f0;
+};
+__device__ __forceinline__ BaseConst load_base_constants(const float *p, int64_t stride)
 {
-    const float *q = p;
-    const FF ia{q[16 * stride], q[20 * stride]}, ib{q[17 * stride], q[21 * stride]};
-    const FF f0{q[22 * stride], q[23 * stride]};
+    return BaseConst{FF{p[16 * stride], p[20 * stride]}, FF{p[17 * stride], p[21 * stride]},
+                     FF{p[22 * stride], p[23 * stride]}};
+}
+__device__ __forceinline__ void store_base_state(float *p, int64_t stride, const BaseConst &k, double Tn0, double T1,
+                                                 double T2, double psi, FF c0, MixedBase &m)
+{
+    const FF ia = k.ia, ib = k.ib, f0 = k.f0;
     const FF tn = ff_split(Tn0), t1 = ff_split(T1), t2 = ff_split(T2), ps = ff_split(psi);
     const FF r0 = ff_rcp(tn);
     const FF q1 = ff_mul(t1, r0), q2 = ff_mul(t2, r0);
@@ -272,7 +278,7 @@ __device__ __forceinline__ MixedBase load_base(const float *__restrict__ p, int6
 {
     float v[20];
 #pragma unroll
-    for (int k = 0; k < 20; ++k) v[k] = __ldg(p + k * stride);
+    for (int k = 0; k < 20; ++k) v[k] = __ldcg(p + k * stride);   // from L2: read before the previous kernel's end
     MixedBase m;
     m.Tn0 = v[0];
     m.q0[0] = v[1]; m.q0[1] = v[2];
@@ -295,11 +301,13 @@ __device__ __forceinline__ float base_slip_rate(const MixedBase &m, int k, float
 }
 
 // Right-hand side at y0 + (dTn, dT1, dT2, dpsi) (MPa, MPa, MPa, state):
-// dpsi/dt and dtau_k/dt (MPa/s).
+// dpsi/dt and dtau_k/dt (MPa/s).  Where a product could be fused into either of
+// two sums the rounding is spelt out: the attempt is compiled into more than one
+// kernel, and all give the same bits.
 __device__ __forceinline__ void mixed_rhs(const MixedBase &m, float dTn, float dT1, float dT2, float dpsi,
                                           float &dstate, float &dtau1, float &dtau2)
 {
-    const float rTn = __frcp_rn(m.Tn0 + dTn);
+    const float rTn = __frcp_rn(__fadd_rn(m.Tn0, dTn));
     const float iaTn = m.inv_a * rTn;                          // 1 / (a sigma), 1/MPa
     const float ed = ff_exp(ff_add(m.g0, -dpsi * m.inv_b));    // e^{(f0 - psi)/b}
     const float ds_dt = m.bdc * (m.V0 * ed - m.slipv);
@@ -307,17 +315,17 @@ __device__ __forceinline__ void mixed_rhs(const MixedBase &m, float dTn, float d
     float out[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        const float dx = ((k ? dT2 : dT1) - m.q0[k] * dTn) * iaTn;   // change of tau/(a sigma)
-        const float xs = m.x0[k] + dx;
+        const float dx = __fmul_rn(__fmaf_rn(-m.q0[k], dTn, k ? dT2 : dT1), iaTn);   // change of tau/(a sigma)
+        const float xs = __fadd_rn(m.x0[k], dx);
         const bool pos = xs >= 0.f;
         const float em = expm1f(-2.f * fabsf(xs));                  // r - 1
-        const FF lw = ff_add(pos ? m.Sp[k] : m.Sm[k], (pos ? dx : -dx) - dpa);   // ln W
+        const FF lw = ff_add(pos ? m.Sp[k] : m.Sm[k], __fsub_rn(pos ? dx : -dx, dpa));   // ln W
         const float w = ff_exp_neg_abs(lw);
         const float q = m.q0[k] + m.a * dx;                         // tau / sigma
         const float D = (2.f + em) * iaTn * 1e-6f;                  // (1 + r) / (a sigma), 1/Pa
-        const float M = D * q * m.dsf + m.inv_a * (pos ? -em : em) * ds_dt;
+        const float M = __fmaf_rn(__fmul_rn(D, q), m.dsf, __fmul_rn(__fmul_rn(m.inv_a, pos ? -em : em), ds_dt));
         const float L = m.L[k];
-        out[k] = (lw.hi >= 0.f) ? __fdiv_rn(fmaf(L, w, M), w + D) : __fdiv_rn(fmaf(w, M, L), fmaf(w, D, 1.f));
+        out[k] = (lw.hi >= 0.f) ? __fdiv_rn(fmaf(L, w, M), __fadd_rn(w, D)) : __fdiv_rn(fmaf(w, M, L), fmaf(w, D, 1.f));
     }
     dstate = ds_dt;
     dtau1 = out[0] * 1e-6f;
@@ -327,7 +335,7 @@ __device__ __forceinline__ void mixed_rhs(const MixedBase &m, float dTn, float d
 // |num| / |yo + num|: in FP32 where yo + num is in float range, else in FP64
 __device__ __forceinline__ float rel_err(float num, double yo)
 {
-    const float ay = fabsf((float)yo + num);
+    const float ay = fabsf(__fadd_rn((float)yo, num));
     if (ay >= 1e-30f && ay <= 1e30f) return __fdiv_rn(fabsf(num), ay);
     return (float)(fabs((double)num) / fabs(yo + (double)num));
 }
@@ -385,11 +393,11 @@ __device__ __forceinline__ void dp_attempt_mixed(const MixedBase &m, float dsig,
         e1t = fmaf(D[l], t[l], e1t);
         e2t = fmaf(D[l], u[l], e2t);
     }
-    es *= hf; e1t *= hf; e2t *= hf;
+    es = __fmul_rn(es, hf); e1t = __fmul_rn(e1t, hf); e2t = __fmul_rn(e2t, hf);
     // the normal stress: its rate is constant, the two orders differ by the
     // rounding of the weight sums
     const float wn = (float)((B81 + B83 + B84 + B85 + B86 + B87) - (B71 + B73 + B74 + B75 + B76));
-    const float en = hf * (wn * dn);
+    const float en = __fmul_rn(hf, __fmul_rn(wn, dn));
     e1 = rel_err(es, yo[3]);
     const float ea = rel_err(e1t, yo[1]), eb = rel_err(e2t, yo[2]), ec = rel_err(en, yo[0]);
     e2 = (isnan(ea) || isnan(eb) || isnan(ec)) ? NAN : fmaxf(fmaxf(ea, eb), ec);
