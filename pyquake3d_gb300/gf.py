@@ -96,25 +96,33 @@ def join_ops(ops):
     return K.reshape(3 * N, 2 * N)
 
 
-def _dp(a):
-    return a.ctypes.data_as(_lib.c_double_p)
+_VP, _D = ctypes.c_void_p, ctypes.c_double
+_POINTS = ctypes.CFUNCTYPE(None, _VP, _VP, _VP, ctypes.c_size_t, _VP, _VP, _VP, _D, _D, _D, _D, _D, ctypes.c_bool, _VP,
+                           _VP)
+_points = None
 
 
 def TDstressFS(X, Y, Z, P1, P2, P3, Ss, Ds, Ts, mu, lambda_, halfspace=False):
     """Reference-shaped call (src/SH_greenfunction.py:200, src/TDstressFS_C.cpp:2095)
-    on the GPU: returns (Stress (6, n), Strain (6, n)) like the NumPy twin."""
+    on the GPU: returns (Stress (6, n), Strain (6, n)) like the NumPy twin.
+
+    The library function is called with plain addresses: a typed pointer object
+    per array (eight of them) takes longer than the kernel on a small call."""
+    global _points
     L = _lib.load()
+    if _points is None:
+        _points = _POINTS(("TDstressFS_C", L))
     X, Y, Z = (np.ascontiguousarray(np.atleast_1d(v), dtype=np.float64) for v in (X, Y, Z))
     P1, P2, P3 = (np.ascontiguousarray(v, dtype=np.float64) for v in (P1, P2, P3))
     n = X.size
-    s = np.empty((n, 6))
-    e = np.empty((n, 6))
-    L.TDstressFS_C(_dp(X), _dp(Y), _dp(Z), n, _dp(P1), _dp(P2), _dp(P3), float(Ss), float(Ds), float(Ts),
-                   float(mu), float(lambda_), bool(halfspace), _dp(s), _dp(e))
-    err = L.pq3d_last_error().decode()
+    out = np.empty((2, n, 6))
+    at = out.ctypes.data
+    _points(X.ctypes.data, Y.ctypes.data, Z.ctypes.data, n, P1.ctypes.data, P2.ctypes.data, P3.ctypes.data, float(Ss),
+            float(Ds), float(Ts), float(mu), float(lambda_), bool(halfspace), at, at + 48 * n)
+    err = L.pq3d_last_error()
     if err:
-        raise _lib.PQ3DError(_lib.PQ3D_ERR_UNSUPPORTED, err)
-    return s.T.copy(), e.T.copy()
+        raise _lib.PQ3DError(_lib.PQ3D_ERR_UNSUPPORTED, err.decode())
+    return out[0].T.copy(), out[1].T.copy()
 
 
 def TDstressHS(X, Y, Z, P1, P2, P3, Ss, Ds, Ts, mu, lambda_):
