@@ -261,14 +261,14 @@ assemble_seg_kernel(const Tile *__restrict__ tiles, int ts, const double *__rest
     const bool on = t < ts && j < N;
     int e[3];
     unsigned sg[3];
-    double bs[3], bd[3];
+    double bs[2], bd[3];
     if (on) {
         const TileTri tri = T.tri[t];
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             e[q] = (tri.e[q] & 0x7fff) * kMatD;
             sg[q] = (unsigned)(tri.e[q] & 0x8000) << 16;
-            bs[q] = mat.scale * src[(F_SX + q) * N + j];
+            if (q < 2) bs[q] = mat.scale * src[(F_SX + q) * N + j];
             bd[q] = mat.scale * src[(F_DX + q) * N + j];
         }
     }
@@ -304,7 +304,7 @@ assemble_seg_kernel(const Tile *__restrict__ tiles, int ts, const double *__rest
             double vs[3], vd[3];
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                vs[a] = R[3 + 3 * a] * bs[0] + R[4 + 3 * a] * bs[1] + R[5 + 3 * a] * bs[2];
+                vs[a] = R[3 + 3 * a] * bs[0] + R[4 + 3 * a] * bs[1];   // the strike axis is horizontal
                 vd[a] = R[3 + 3 * a] * bd[0] + R[4 + 3 * a] * bd[1] + R[5 + 3 * a] * bd[2];
             }
             double ts3[3], td3[3];
@@ -443,8 +443,7 @@ assemble_hs_kernel(const Tile *__restrict__ tiles, const TileHs *__restrict__ hs
                     double vs[3], vd[3];
 #pragma unroll
                     for (int a = 0; a < 3; ++a) {
-                        vs[a] = mat.scale * (R[3 + 3 * a] * tab[F_SX * N + j] + R[4 + 3 * a] * tab[F_SY * N + j] +
-                                             R[5 + 3 * a] * tab[F_SZ * N + j]);
+                        vs[a] = mat.scale * (R[3 + 3 * a] * tab[F_SX * N + j] + R[4 + 3 * a] * tab[F_SY * N + j]);
                         vd[a] = mat.scale * (R[3 + 3 * a] * tab[F_DX * N + j] + R[4 + 3 * a] * tab[F_DY * N + j] +
                                              R[5 + 3 * a] * tab[F_DZ * N + j]);
                     }
