@@ -71,8 +71,8 @@ __global__ void setup_elements_kernel(const double *__restrict__ nodes, const in
 }
 
 // ---------------------------------------------------------------------------
-// tiles of sources: the triangles [tile * ts, tile * ts + ts) and the distinct
-// vertices and edges they use
+// tiles of sources: ts triangles next to one another (in the mesh's order or in
+// order_tiles_kernel's) and the distinct vertices and edges they use
 
 constexpr int kTileMax = 256;   // triangles of a tile at most
 constexpr int kTileItems = 3 * kTileMax;
@@ -90,6 +90,7 @@ struct Tile {
     double vert[kTileItems][3];
     TileEdge edge[kTileItems];
     TileTri tri[kTileMax];
+    int32_t id[kTileMax];   // the triangles' numbers in the mesh
 };
 constexpr int kSegDoubles = (int)(sizeof(Tile) / sizeof(double));
 static_assert(sizeof(Tile) % 16 == 0, "tiles start 16-byte aligned");
@@ -130,8 +131,9 @@ inline int tile_size(int64_t N, bool half = false)
 constexpr int kHash = 2048;
 __global__ void __launch_bounds__(kTileMax)
 setup_tiles_kernel(const double *__restrict__ nodes, const int64_t *__restrict__ tris, int64_t N, int ts,
-                   Tile *__restrict__ tiles, TileHs *__restrict__ hs)
+                   const int32_t *__restrict__ order, Tile *__restrict__ tiles, TileHs *__restrict__ hs)
 {
+    if (order && order[N] == 0) return;   // the tiles stand as they are
     __shared__ unsigned long long vkey[kHash], ekey[kHash];
     __shared__ uint16_t vidx[kHash], eidx[kHash];
     __shared__ int nv, ne;
@@ -140,8 +142,9 @@ setup_tiles_kernel(const double *__restrict__ nodes, const int64_t *__restrict__
     if (t == 0) nv = ne = 0;
     __syncthreads();
     Tile &T = tiles[blockIdx.x];
-    const int64_t j = (int64_t)blockIdx.x * ts + t;
-    const bool on = t < ts && j < N;
+    const int64_t pos = (int64_t)blockIdx.x * ts + t;
+    const bool on = t < ts && pos < N;
+    const int64_t j = on && order ? order[pos] : pos;
     int vs[3], es[3];
     bool vown[3], eown[3];
     int64_t id[3];
@@ -193,8 +196,126 @@ setup_tiles_kernel(const double *__restrict__ nodes, const int64_t *__restrict__
             tri.e[q] = (uint16_t)(e | (rev ? 0x8000 : 0));
         }
         T.tri[t] = tri;
+        T.id[t] = (int32_t)j;
     }
     if (t == 0) { T.nv = nv; T.ne = ne; }
+}
+
+// A spatial order of the triangles for meshes whose own order leaves tiles of
+// many edges: the stable sort of the centroids' Morton codes (10 bits an axis),
+// by one block, into order[0 .. N); order[N] = 1, or 0 where the tiles are kept.
+// `tiles` is scratch from there on (12 bytes a triangle; they are set up anew).
+//
+// A tile of consecutive triangles is a strip of a structured mesh (1.75 edges a
+// triangle at 163 columns of 62 squares) and anything up to 3 in an unordered
+// one.  N = 20,000, FP64 output: in column order 167.7 -> 161.5 ms, shuffled 286.6
+// -> 162.0 ms; half space, N = 2,500, shuffled 61.3 -> 36.5 ms.
+// The lines: below 2^24 pairs (7 ms; half space 2^20, 6 ms) the two launches and
+// the sort (40 us at N = 4,200, 130 us at 20,000) are a visible part of the call;
+// at 1.66 edges a triangle there is little left to gain.
+constexpr int64_t kOrderPairs = 1 << 24, kOrderPairsHs = 1 << 20;
+constexpr int kOrderEdges = 166;   // per 100 triangles
+constexpr int kOrderThreads = 1024;
+
+__global__ void __launch_bounds__(kOrderThreads)
+order_tiles_kernel(const double *__restrict__ recv, int64_t N, int64_t ntiles, Tile *tiles, int32_t *order)
+{
+    constexpr int kW = kOrderThreads / 32;
+    __shared__ int hist[256][kW + 1];
+    __shared__ float lo[3][kW], hi[3][kW];
+    __shared__ int total;
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+    if (t == 0) total = 0;
+    __syncthreads();
+    for (int64_t q = t; q < ntiles; q += kOrderThreads) atomicAdd(&total, tiles[q].ne);
+    __syncthreads();
+    const bool sort = 100 * (int64_t)total > kOrderEdges * N;
+    if (t == 0) order[N] = sort;
+    if (!sort) return;
+    // the centroids' box (fminf and fmaxf pass over NaN)
+    float a[3] = {INFINITY, INFINITY, INFINITY}, b[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int64_t j = t; j < N; j += kOrderThreads)
+        for (int c = 0; c < 3; ++c) {
+            const float x = (float)recv[j * kRecvStride + c];
+            a[c] = fminf(a[c], x);
+            b[c] = fmaxf(b[c], x);
+        }
+    float ext = 0.f;
+    for (int c = 0; c < 3; ++c) {
+        for (int o = 16; o > 0; o >>= 1) {
+            a[c] = fminf(a[c], __shfl_xor_sync(0xffffffffu, a[c], o));
+            b[c] = fmaxf(b[c], __shfl_xor_sync(0xffffffffu, b[c], o));
+        }
+        if (lane == 0) { lo[c][w] = a[c]; hi[c][w] = b[c]; }
+    }
+    __syncthreads();
+    for (int c = 0; c < 3; ++c) {
+        for (int q = 0; q < kW; ++q) { a[c] = fminf(a[c], lo[c][q]); b[c] = fmaxf(b[c], hi[c][q]); }
+        ext = fmaxf(ext, b[c] - a[c]);
+    }
+    const float scale = ext > 0.f ? 1023.f / ext : 0.f;
+    uint32_t *key[2] = {(uint32_t *)tiles, (uint32_t *)tiles + N};
+    int32_t *idx[2] = {order, (int32_t *)tiles + 2 * N};
+    for (int64_t j = t; j < N; j += kOrderThreads) {
+        uint32_t k = 0;
+        for (int c = 0; c < 3; ++c) {
+            const float x = ((float)recv[j * kRecvStride + c] - a[c]) * scale;
+            uint32_t v = (uint32_t)(int)fminf(fmaxf(x, 0.f), 1023.f);
+            v = (v | v << 16) & 0x030000ffu;
+            v = (v | v << 8) & 0x0300f00fu;
+            v = (v | v << 4) & 0x030c30c3u;
+            v = (v | v << 2) & 0x09249249u;
+            k |= v << c;
+        }
+        key[0][j] = k;
+        idx[0][j] = (int32_t)j;
+    }
+    // four passes of 8 bits, a warp a contiguous part of the list
+    const int64_t part = (N + kOrderThreads - 1) / kOrderThreads * 32;
+    const int64_t j0 = w * part, j1 = j0 + part < N ? j0 + part : N;
+    for (int pass = 0; pass < 4; ++pass) {
+        const uint32_t *ki = key[pass & 1];
+        const int32_t *ii = idx[pass & 1];
+        uint32_t *ko = key[1 - (pass & 1)];
+        int32_t *io = idx[1 - (pass & 1)];
+        __syncthreads();   // the last pass's lists are in
+        for (int q = t; q < 256 * (kW + 1); q += kOrderThreads) (&hist[0][0])[q] = 0;
+        __syncthreads();
+        for (int64_t j = j0 + lane; j < j1; j += 32) atomicAdd(&hist[(ki[j] >> (8 * pass)) & 255][w], 1);
+        __syncthreads();
+        // exclusive sums over (digit, warp): a warp takes 8 digits
+        int sum = 0;
+        for (int d = 8 * w; d < 8 * w + 8; ++d) {
+            int v = hist[d][lane], x = v;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            hist[d][lane] = sum + x - v;
+            sum += __shfl_sync(0xffffffffu, x, 31);
+        }
+        if (lane == 0) hist[w][kW] = sum;
+        __syncthreads();
+        int before = 0;
+        for (int q = 0; q < w; ++q) before += hist[q][kW];
+        for (int d = 8 * w; d < 8 * w + 8; ++d) hist[d][lane] += before;
+        __syncthreads();
+        for (int64_t jb = j0; jb < j1; jb += 32) {
+            const int64_t j = jb + lane;
+            const bool on = j < j1;
+            const uint32_t k = on ? ki[j] : 0u;
+            const int32_t i = on ? ii[j] : 0;
+            const int d = on ? (int)((k >> (8 * pass)) & 255) : 256;
+            const unsigned same = __match_any_sync(0xffffffffu, d);
+            const int rank = __popc(same & ((1u << lane) - 1u));
+            int at = 0;
+            if (on) at = hist[d][w] + rank;
+            __syncwarp();
+            if (on && rank == 0) hist[d][w] += __popc(same);
+            __syncwarp();
+            if (on) { ko[at] = k; io[at] = i; }
+        }
+    }
 }
 
 // Half-space records of source j: the mirrored triangle's source record
@@ -221,7 +342,7 @@ __global__ void setup_hs_kernel(const double *__restrict__ nodes, const int64_t 
 //
 // Bound: the FP64 pipe (2 lanes per clock and SM).  About 21 FP64 operations
 // per vertex, 95 per edge and 54 per pair; on a structured mesh a tile of 256
-// triangles has 0.7 vertices and 1.7 edges per triangle, so a pair takes ~230
+// triangles has 0.6 vertices and 1.63 edges per triangle, so a pair takes ~220
 // (520 as three angular dislocations per pair).  256 triangles per tile: 128
 // have 1.9 edges per triangle; more would leave one block per SM.
 constexpr int kSegThreads = 256;
@@ -257,8 +378,8 @@ assemble_seg_kernel(const Tile *__restrict__ tiles, int ts, const double *__rest
     const int batch = min(nrec, kSegSmem / (int)sizeof(double) / (nv * kVertD + ne * kMatD));
     double *sv = s_buf, *sm = s_buf + (size_t)batch * nv * kVertD;
     // this thread's triangle: edges, and its slip directions times mu/(4 pi)
-    const int64_t j = (int64_t)blockIdx.x * ts + t;
-    const bool on = t < ts && j < N;
+    const bool on = t < ts && (int64_t)blockIdx.x * ts + t < N;
+    const int64_t j = on ? T.id[t] : 0;
     int e[3];
     unsigned sg[3];
     double bs[2], bd[3];
@@ -431,7 +552,7 @@ assemble_hs_kernel(const Tile *__restrict__ tiles, const TileHs *__restrict__ hs
         }
         __syncthreads();
         for (int q = t; q < nt; q += kHsThreads) {
-            const int64_t j = j0 + q;
+            const int64_t j = T.id[q];
             const TileTri tri = T.tri[q];
             const bool surface = fsc[kFscSurface * N + j] != 0.0;
             for (int r = 0; r < nb; ++r) {
@@ -773,16 +894,19 @@ static int point_many_sources(double x, double y, double z, const double *P1, co
 // Workspace: source table [kSrcStride][N], receiver table [N][kRecvStride],
 // for the half space the image table [kImgStride][N] and the side table
 // [kFscStride][N], then (from an even offset) the tiles, and for the half space
-// their edges' surface records.
+// their edges' surface records, last the triangles' order (N + 1 integers).
 static size_t tables_doubles(int64_t N, bool half)
 {
     return (size_t)N * (kSrcStride + kRecvStride + (half ? kImgStride + kFscStride : 0));
 }
 static size_t tiles_offset(int64_t N, bool half) { return (tables_doubles(N, half) + 1) & ~(size_t)1; }
+static size_t order_offset(int64_t N, bool half)
+{
+    return tiles_offset(N, half) + (size_t)tile_count(N, half) * (kSegDoubles + (half ? kHsDoubles : 0));
+}
 static size_t ws_bytes(int64_t N, bool half)
 {
-    return (tiles_offset(N, half) + (size_t)tile_count(N, half) * (kSegDoubles + (half ? kHsDoubles : 0))) *
-           sizeof(double);
+    return order_offset(N, half) * sizeof(double) + ((size_t)N / 2 + 1) * sizeof(double);
 }
 
 static void setup_elements(const double *nodes, const int64_t *tris, int64_t N, double *src, double *recv,
@@ -844,7 +968,13 @@ static int assemble_rows(const double *nodes, const int64_t *tris, int64_t N, in
         const int th = 128;
         setup_elements(nodes, tris, N, src, recv, st);
         if (half) setup_hs_kernel<<<(unsigned)((N + th - 1) / th), th, 0, st>>>(nodes, tris, N, img, fsc);
-        setup_tiles_kernel<<<(unsigned)nt, kTileMax, 0, st>>>(nodes, tris, N, ts, tiles, hs);
+        setup_tiles_kernel<<<(unsigned)nt, kTileMax, 0, st>>>(nodes, tris, N, ts, nullptr, tiles, hs);
+        const int64_t rows = row1 > row0 ? row1 - row0 : N;   // no rows: they follow, all of them
+        if (rows * N >= (half ? kOrderPairsHs : kOrderPairs)) {
+            int32_t *order = (int32_t *)(ws + order_offset(N, half));
+            order_tiles_kernel<<<1, kOrderThreads, 0, st>>>(recv, N, nt, tiles, order);
+            setup_tiles_kernel<<<(unsigned)nt, kTileMax, 0, st>>>(nodes, tris, N, ts, order, tiles, hs);
+        }
         PQ3D_CUDA_TRY(cudaGetLastError());
     }
     if (row0 == row1) return PQ3D_OK;
@@ -881,7 +1011,8 @@ static int assemble_rows(const double *nodes, const int64_t *tris, int64_t N, in
 // held by every GPU that loads this library.
 constexpr int64_t kNoAllocMaxN = 32768;
 static __device__ __align__(256) double g_noalloc_scratch[(size_t)(kSrcStride + kRecvStride) * kNoAllocMaxN +
-                                                          (size_t)(kNoAllocMaxN / kTileMax) * kSegDoubles];
+                                                          (size_t)(kNoAllocMaxN / kTileMax) * kSegDoubles +
+                                                          (size_t)kNoAllocMaxN / 2 + 1];
 
 // Device address of the fixed scratch on the current device, looked up with
 // that device current on every call (cheap): a cached address would go stale
