@@ -222,8 +222,10 @@ gemm_fix_kernel(const uint8_t *__restrict__ Kp, const uint8_t *__restrict__ Vp, 
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = *(volatile uint32_t *)tmem_slot;
+    // no chain_release: this kernel's registers leave no room beside it, and an
+    // attempt let in early would crowd onto the SMs without a product block
+    // (N = 700, B = 10, FP64 attempt: 140 us an iteration in step, 229 let in)
     chain_wait();
-    chain_release();   // from here on the previous iteration is complete: the attempt may read its state
 
     if (warp == 0) {
         if (lane == 0) {

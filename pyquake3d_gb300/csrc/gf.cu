@@ -917,13 +917,13 @@ static void setup_elements(const double *nodes, const int64_t *tris, int64_t N, 
 }
 
 // Receivers per block: the grid's tail costs up to one block's time, so the
-// count (a quarter of the most .. the most) with the fewest receivers on a
-// slot's path wins; one extra receiver stands for a block's start.
+// count with the fewest receivers on a slot's path wins (one receiver a block on
+// the smallest meshes); one extra receiver stands for a block's start.
 static int seg_receivers(int most, int64_t tiles, int64_t rows, int64_t slots)
 {
     int best = most;
     int64_t cost = INT64_MAX;
-    for (int nr = most; nr >= most / 4; --nr) {
+    for (int nr = most; nr >= 1; --nr) {
         const int64_t waves = (tiles * ((rows + nr - 1) / nr) + slots - 1) / slots;
         const int64_t c = waves * (nr + 1);
         if (c < cost) { cost = c; best = nr; }
