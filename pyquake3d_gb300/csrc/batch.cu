@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(256, kMixed ? 4 : (kFF ? 3 : 2)) attempt_kerne
     // What the previous iteration left (the product that runs before this
     // kernel has waited for it) is read while the product ends; its rates after.
     // All reads before chain_wait go to L2 (__ldcg).
-    chain_release();
+    if (kMixed) chain_release();
     __shared__ unsigned long long red[32];
     __shared__ int act;
     __shared__ double hs;
@@ -522,7 +522,7 @@ template <bool kMixed>
 __global__ void __launch_bounds__(256) update_kernel(pq3d_batch_sim S)
 {
     // constants before the wait
-    chain_release();
+    if (kMixed) chain_release();
     __shared__ int acc;
     __shared__ double hs, lnv0;
     __shared__ float inv_eta, c0hi, c0lo;
@@ -858,10 +858,13 @@ extern "C" int pq3d_batch_iterate_begin(const pq3d_batch_sim *sim, void *workspa
     if (rc) return rc;
     // 2. attempt (FP64 arm: the reference arithmetic; mixed arms: dp_attempt_mixed)
     dim3 grid((unsigned)((S.N + 255) / 256), (unsigned)S.B);
-    PQ3D_CUDA_TRY(launch_chained(mixed_attempt(S) ? attempt_kernel<true>
-                                 : S.attempt64 == 2 && S.precision != PQ3D_BATCH_FP64 ? attempt_kernel<false, true>
-                                                                                      : attempt_kernel<false>,
-                                 grid, 256, 0, st, S));
+    // only the mixed kernels are let in early: blocks of the FP64-bound ones would
+    // settle two and more to an SM beside what still runs there (FP32 product, FP64
+    // attempt, N = 2,000, B = 20: 383 us an iteration, 405 let in)
+    if (mixed_attempt(S)) PQ3D_CUDA_TRY(launch_chained(attempt_kernel<true>, grid, 256, 0, st, S));
+    else if (S.attempt64 == 2 && S.precision != PQ3D_BATCH_FP64) attempt_kernel<false, true><<<grid, 256, 0, st>>>(S);
+    else attempt_kernel<false><<<grid, 256, 0, st>>>(S);
+    PQ3D_CUDA_TRY(cudaGetLastError());
     return PQ3D_OK;
 }
 
@@ -875,7 +878,9 @@ extern "C" int pq3d_batch_iterate_end(const pq3d_batch_sim *sim, void *stream)
     // 3-4. decide, update
     PQ3D_CUDA_TRY(launch_chained(decide_kernel, (2 * S.B + 127) / 128, 128, 0, st, S.ctrl, S.B));
     dim3 grid((unsigned)((S.N + 255) / 256), (unsigned)S.B);
-    PQ3D_CUDA_TRY(launch_chained(mixed_attempt(S) ? update_kernel<true> : update_kernel<false>, grid, 256, 0, st, S));
+    if (mixed_attempt(S)) PQ3D_CUDA_TRY(launch_chained(update_kernel<true>, grid, 256, 0, st, S));
+    else update_kernel<false><<<grid, 256, 0, st>>>(S);
+    PQ3D_CUDA_TRY(cudaGetLastError());
     if (S.precision == PQ3D_BATCH_BF16X18 && !fused_rhs_pack(S))   // v' of every run from its slip rates
         return fx::pack_rhs_from_state(S.slipv1, S.slipv2, S.cos_rake0, S.sin_rake0, S.Vpl, S.fix_order, S.N, S.B,
                                        S.vop, st);

@@ -1007,7 +1007,7 @@ static int assemble_rows(const double *nodes, const int64_t *tris, int64_t N, in
 
 // ---------------------------------------------------------------------------
 // Fixed scratch for pq3d_assemble_dense_noalloc: the source and receiver
-// tables and the tiles of one call for up to kNoAllocMaxN elements, 19.1 MB
+// tables, the tiles and their order of one call for up to kNoAllocMaxN elements, 19.4 MB
 // held by every GPU that loads this library.
 constexpr int64_t kNoAllocMaxN = 32768;
 static __device__ __align__(256) double g_noalloc_scratch[(size_t)(kSrcStride + kRecvStride) * kNoAllocMaxN +
