@@ -131,22 +131,21 @@ def fp64_peak_tflops(torch, dev):
     return 2.0 * n ** 3 / best / 1e12
 
 
-# FP64 operations of one (receiver, source) pair of the assembly kernel
-# (both unit slips, 6 entries): 318 add + 403 mul + 5 div + 3 sqrt, counted by
-# oracle/count_gf_flops.cpp on the kernel's own device math.
-GF_FLOP_PER_PAIR = 729
+# FP64 operations of one (receiver, source) pair of the tiled assembly (both
+# unit slips, 6 entries; add, sub, mul, div and sqrt one each), counted on the
+# kernel's own device math: 27 per vertex, 127 per edge and 72 per pair, with the
+# 0.648 vertices and 1.645 edges per triangle of the tiles of the N = 20,000 mesh.
+GF_FLOP_PER_PAIR = 298
 # The same pair with the published angular-dislocation expressions
 # (src/TDstressFS_C.cpp:51-121) evaluated term by term and rotated tensor by
 # tensor (src/TDstressFS_C.cpp:185-256), both slips sharing the geometry and
 # 11 divisions: 1,016, counted by the same tool (the kernel's first form).
 GF_FLOP_PER_PAIR_TERM_BY_TERM = 1016
-# The same for the half-space kernel (main + image dislocation, the
-# free-surface correction of the three sides in dual numbers): 5,412.7 add +
-# 8,793.4 mul + 66.9 div + 18.0 sqrt per pair (and 18.0 transcendental calls),
-# counted by oracle/count_hs_flops.cpp over every pair of the 40 x 20 km,
-# N = 2,500 mesh of bench_halfspace (the count depends weakly on the mesh
-# through the branches of the angular dislocations).
-HS_FLOP_PER_PAIR = 14291
+# The same for the half-space kernel: 2,682 per edge (of which the free-surface
+# correction's two end points 2,131: 826 add + 1,295 mul + 8 div + 2 sqrt) and 168
+# per pair, with the 1.634 edges per triangle of the N = 2,500 mesh of
+# bench_halfspace (a pair by itself, as the single-source calls take it: 8,263).
+HS_FLOP_PER_PAIR = 4550
 # Stores per pair: 6 FP64 + 6 FP32 entries.
 GF_BYTES_PER_PAIR = 72
 
@@ -339,17 +338,16 @@ def bench_ours(args):
         else:
             roof.update({"achieved": None, "frac": None})
         # DRAM bytes of one launch: ncu on the N=6,000 case (2.6 GB of stores,
-        # 20x the L2) measured 70.7 B/pair (2.532 GB written + 13 MB read for
-        # 3.6e7 pairs; ~60 MB of the 2.592 GB of stores still dirty in L2 at
-        # kernel end); scaled to this launch by pairs.
+        # 20x the L2) measured 71.5 B/pair (2.565 GB written + 9 MB read for
+        # 3.6e7 pairs); scaled to this launch by pairs.
         # the FP64 pipe is the bound: DGEMM issues only 2-flop DFMAs, this
-        # kernel averages ~1.33 flops per FP64-pipe instruction (550 per
-        # pair); ncu on the N = 6,000 case: FP64 pipe 90 % busy (active cycles)
-        roof["fp64_pipe_active_pct"] = 89.8
-        roof["pipe_note"] = ("ncu sm__inst_executed_pipe_fp64 pct_of_peak_sustained_active, capture of the N=6000 "
+        # kernel averages ~1.33 flops per FP64-pipe instruction (224 per
+        # pair); ncu on the N = 6,000 case: FP64 pipe 87 % busy (active cycles)
+        roof["fp64_pipe_active_pct"] = 87.4
+        roof["pipe_note"] = ("ncu sm__pipe_fp64_cycles_active pct_of_peak_sustained_active, capture of the N=6000 "
                              "case (bench.py --case gf_assembly)")
-        roof["traffic"] = 70.7 * N * N
-        roof["traffic_note"] = ("ncu dram__bytes_read+write at N=6000 (70.7 B/pair, 2.6 GB of stores, 20x the L2) "
+        roof["traffic"] = 71.5 * N * N
+        roof["traffic_note"] = ("ncu dram__bytes_read+write at N=6000 (71.5 B/pair, 2.6 GB of stores, 20x the L2) "
                                 "scaled by pairs (bench.py --case gf_assembly); algorithmic stores are %d B/pair"
                                 % GF_BYTES_PER_PAIR)
         out["roofline"] = roof
@@ -388,7 +386,7 @@ def bench_ours(args):
                        "l2": "output operator (%.1f GB FP64 + FP32 per step) streams through L2; inputs are the "
                              "mesh only" % (K64.numel() * 12 / 1e9),
                        "parallelism": "replicas" if world > 1 else "single"},
-            "gpu_launches": 3 * args.steps}
+            "gpu_launches": 5 * args.steps}
     line.update(out)
     if "batched" in out:
         # the primary metric's numbers in one compact key, last in the line
@@ -1035,8 +1033,8 @@ def L_ws_bytes(N):
 def profile_case(case):
     """Small single-kernel cases for ncu captures (no timing, no JSON):
     gf_assembly  full-space assembly, rough 60x25 km, N=6,000, FP64 + FP32 copy
-                 (2.6 GB of stores, 20x the L2; 2 launches)
-    hs_assembly  half-space assembly, rough 20x10 km to the surface, N=1,600 (2 launches)
+                 (2.6 GB of stores, 20x the L2; 5 launches)
+    hs_assembly  half-space assembly, rough 20x10 km to the surface, N=1,600 (6 launches)
     hmat_product H-matrix product, rough 200x40 km, N=100,000, B=1 (13 products)
     hmat_product_40k  the same, rough 100x40 km, N=40,000 (build scratch released
                  before the products; ~2 GB resident)
