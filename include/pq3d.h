@@ -306,7 +306,9 @@ typedef struct pq3d_batch_sim {
 /* Packed operator of the tensor-core product: the FP64 operator split into
  * three BF16 pieces, stored as [3N/128 tiles][2N/32 blocks][3][128 x 32]
  * shared-memory images (8-row x 16-byte core matrices).  Bytes, and the packing
- * kernel (run once after assembly). */
+ * kernel (run once after assembly).  A product or iteration queued after it, or
+ * after a caller's own writer of the images, on the same stream reads what that
+ * one wrote; nothing has to stand between them. */
 size_t pq3d_batch_operator_bytes(int64_t N);
 int pq3d_batch_pack_operator(const double *K64, int64_t N, void *Kpacked, void *stream);
 /* Bytes of the packed right-hand side for B runs (BF16X6). */

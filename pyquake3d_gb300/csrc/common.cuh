@@ -29,12 +29,19 @@ void clear_error();
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// Launch that may start before the stream's previous kernel has ended, if that
-// kernel lets it (chain_release by all its blocks); the kernel must call
-// chain_wait, in every block, before it touches anything an earlier kernel
-// reads or writes: the previous kernel is then complete, and with it everything
-// before it.  A small batched iteration is four kernels of 5-10 us, so launch
-// latency and prologues are a visible part of it.
+// Launch that may start before the stream's previous kernel has ended: when all
+// that kernel's blocks have called chain_release or ended.  A kernel launched
+// so calls chain_wait in every block, also in one that has nothing to do: it
+// returns once the previous kernel is complete and its writes are visible.
+// Before it, a kernel may read only what no kernel since the last one known to be
+// complete writes, and writes nothing.  Known to be complete, with its writes
+// visible: everything before the previous kernel, where that one (the product,
+// ahead of an attempt or a cluster step: both launched by one call) releases
+// after its own chain_wait, or never.  So an attempt may read the state that the
+// last update left while the product still runs; a product, whose previous kernel
+// is the caller's (perhaps the writer of the operator), reads nothing early.  A
+// small batched iteration is four kernels of 5-10 us, so launch latency and
+// prologues are a visible part of it.
 template <typename... P, typename... A>
 inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
 {

@@ -89,15 +89,13 @@ gemm_bf16x6_kernel(const uint8_t *__restrict__ Kp, const uint8_t *__restrict__ V
     tc_fence_after();
     const uint32_t tmem = *(volatile uint32_t *)tmem_slot;
 
-    // the first stages' operator images, which no kernel of an iteration writes,
-    // come in while the previous kernel ends
-    const int early = nkb < stages ? nkb : stages;
+    // Every read waits, the operator's too: the kernel before this one may be its
+    // writer (a packing kernel or the caller's own), and only the wait makes its
+    // stores visible to the bulk copies.  Until then the first stages' operator
+    // images are brought into L2 only (a prefetch returns no data, and L2 is where
+    // a writer's stores go).
     if (warp == 0 && lane == 0)
-        for (int it = 0; it < early; ++it) {
-            mbar_expect_tx(full0 + 8 * it, stage_bytes);
-            bulk_g2s(smem_u32(smem + (size_t)it * stage_bytes), Kp + (size_t)(mt * KB + kb0 + it) * a_bytes, a_bytes,
-                     full0 + 8 * it);
-        }
+        bulk_prefetch_l2(Kp + (size_t)(mt * KB + kb0) * a_bytes, (uint32_t)(nkb < stages ? nkb : stages) * a_bytes);
     __syncwarp();
     chain_wait();
     chain_release();   // from here on the previous iteration is complete: the attempt may read its state
@@ -106,13 +104,11 @@ gemm_bf16x6_kernel(const uint8_t *__restrict__ Kp, const uint8_t *__restrict__ V
         // producer: two bulk copies per stage
         for (int it = 0; it < nkb; ++it) {
             const int st = it % stages, use = it / stages;
+            if (!mbar_wait(empty0 + 8 * st, (use & 1) ^ 1)) { atomicExch(err, 1); break; }
             const uint32_t sa = smem_u32(smem + (size_t)st * stage_bytes);
             const int64_t kb = kb0 + it;
-            if (it >= early) {
-                if (!mbar_wait(empty0 + 8 * st, (use & 1) ^ 1)) { atomicExch(err, 1); break; }
-                mbar_expect_tx(full0 + 8 * st, stage_bytes);
-                bulk_g2s(sa, Kp + (size_t)(mt * KB + kb) * a_bytes, a_bytes, full0 + 8 * st);
-            }
+            mbar_expect_tx(full0 + 8 * st, stage_bytes);
+            bulk_g2s(sa, Kp + (size_t)(mt * KB + kb) * a_bytes, a_bytes, full0 + 8 * st);
             bulk_g2s(sa + a_bytes, Vp + (size_t)kb * b_bytes, b_bytes, full0 + 8 * st);
         }
     } else if (warp == 1 && lane == 0) {
