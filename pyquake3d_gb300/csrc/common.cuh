@@ -29,6 +29,16 @@ void clear_error();
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Dynamic shared memory beyond 48 KB for the next launch of `kernel`.  Set on every
+// call (well below a microsecond) and not once per device: the attribute is one of
+// the loaded code, and nothing in CUDA's documents says that it outlives a reset of
+// the device between calls (with runtime 13.0 it does).
+template <typename... P>
+inline cudaError_t allow_smem(void (*kernel)(P...), size_t bytes)
+{
+    return cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 // Launch that may start before the stream's previous kernel has ended: when all
 // that kernel's blocks have called chain_release or ended.  A kernel launched
 // so calls chain_wait in every block, also in one that has nothing to do: it

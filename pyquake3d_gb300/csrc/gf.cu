@@ -931,29 +931,6 @@ static int seg_receivers(int most, int64_t tiles, int64_t rows, int64_t slots)
     return best;
 }
 
-struct SegCfg {
-    int device = -1;
-    int sms = 0;
-};
-static thread_local SegCfg g_seg;
-
-static int seg_config(int *sms)
-{
-    int dev;
-    PQ3D_CUDA_TRY(cudaGetDevice(&dev));
-    if (g_seg.device != dev) {
-        const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        PQ3D_CUDA_TRY(cudaDeviceGetAttribute(&g_seg.sms, cudaDevAttrMultiProcessorCount, dev));
-        PQ3D_CUDA_TRY(cudaFuncSetAttribute(assemble_seg_kernel<true>, a, kSegSmem));
-        PQ3D_CUDA_TRY(cudaFuncSetAttribute(assemble_seg_kernel<false>, a, kSegSmem));
-        PQ3D_CUDA_TRY(cudaFuncSetAttribute(assemble_hs_kernel<true>, a, kHsSmem));
-        PQ3D_CUDA_TRY(cudaFuncSetAttribute(assemble_hs_kernel<false>, a, kHsSmem));
-        g_seg.device = dev;
-    }
-    *sms = g_seg.sms;
-    return PQ3D_OK;
-}
-
 static int assemble_rows(const double *nodes, const int64_t *tris, int64_t N, int64_t row0, int64_t row1, double mu,
                          double lam, double *K64, float *K32, double *ws, bool do_setup, cudaStream_t st,
                          bool half = false)
@@ -978,28 +955,23 @@ static int assemble_rows(const double *nodes, const int64_t *tris, int64_t N, in
         PQ3D_CUDA_TRY(cudaGetLastError());
     }
     if (row0 == row1) return PQ3D_OK;
-    int sms = 0;
-    const int rc = seg_config(&sms);
-    if (rc) return rc;
+    int dev, sms;
+    PQ3D_CUDA_TRY(cudaGetDevice(&dev));
+    PQ3D_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const double nu = poisson(mu, lam);
     const SegMat mat = seg_material(nu, 2.0 * mu, lam);
     const int nr = seg_receivers(half ? kHsRecv : kSegRecv, nt, row1 - row0, 2 * (int64_t)sms);
     const dim3 grid((unsigned)nt, (unsigned)((row1 - row0 + nr - 1) / nr));
     if (half) {
-        if (K32)
-            assemble_hs_kernel<true><<<grid, kHsThreads, kHsSmem, st>>>(tiles, hs, ts, src, recv, img, fsc, N, row0,
-                                                                        row1, nr, mat, nu, kfac(nu), 2.0 * mu, lam, K64,
-                                                                        K32);
-        else
-            assemble_hs_kernel<false><<<grid, kHsThreads, kHsSmem, st>>>(tiles, hs, ts, src, recv, img, fsc, N, row0,
-                                                                         row1, nr, mat, nu, kfac(nu), 2.0 * mu, lam,
-                                                                         K64, nullptr);
-    } else if (K32) {
-        assemble_seg_kernel<true><<<grid, kSegThreads, kSegSmem, st>>>(tiles, ts, src, recv, N, row0, row1, nr, mat, nu,
-                                                                       kfac(nu), 2.0 * mu, lam, K64, K32);
+        const auto kernel = K32 ? assemble_hs_kernel<true> : assemble_hs_kernel<false>;
+        PQ3D_CUDA_TRY(allow_smem(kernel, kHsSmem));
+        kernel<<<grid, kHsThreads, kHsSmem, st>>>(tiles, hs, ts, src, recv, img, fsc, N, row0, row1, nr, mat, nu,
+                                                  kfac(nu), 2.0 * mu, lam, K64, K32);
     } else {
-        assemble_seg_kernel<false><<<grid, kSegThreads, kSegSmem, st>>>(tiles, ts, src, recv, N, row0, row1, nr, mat,
-                                                                        nu, kfac(nu), 2.0 * mu, lam, K64, nullptr);
+        const auto kernel = K32 ? assemble_seg_kernel<true> : assemble_seg_kernel<false>;
+        PQ3D_CUDA_TRY(allow_smem(kernel, kSegSmem));
+        kernel<<<grid, kSegThreads, kSegSmem, st>>>(tiles, ts, src, recv, N, row0, row1, nr, mat, nu, kfac(nu), 2.0 * mu,
+                                                    lam, K64, K32);
     }
     PQ3D_CUDA_TRY(cudaGetLastError());
     return PQ3D_OK;

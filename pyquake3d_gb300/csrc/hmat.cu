@@ -1444,14 +1444,7 @@ extern "C" int pq3d_hmat_apply_masked(const pq3d_hmat *H, const double *X, int B
         const int ngroups = (B + 7) / 8;
         Pair2 *Xs = (Pair2 *)workspace, *T = Xs + (size_t)(slots / 2) * 2 * N;
         int32_t *list = (int32_t *)(T + (size_t)(slots / 2) * H->t_rows);
-        static thread_local int smem_dev = -1;
-        int dev;
-        PQ3D_CUDA_TRY(cudaGetDevice(&dev));
-        if (smem_dev != dev) {
-            PQ3D_CUDA_TRY(cudaFuncSetAttribute(leaf_rows_runs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               kRunSmem));
-            smem_dev = dev;
-        }
+        PQ3D_CUDA_TRY(allow_smem(leaf_rows_runs_kernel, kRunSmem));
         PQ3D_REQUIRE((short_ctas + H->t_nlong) * 2 * ngroups < (int64_t)INT32_MAX &&
                          (int64_t)H->nleaves * ngroups * kRunPasses < (int64_t)INT32_MAX && ngroups < 65536,
                      "pq3d_hmat_apply: too many rank rows or leaves x runs");
