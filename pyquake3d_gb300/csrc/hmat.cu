@@ -1314,34 +1314,27 @@ static PairGen<kHalf> make_gen(const double *tables, int64_t N, double mu, doubl
                           2.0 * mu, lambda_};
 }
 
-// The second stream of an ACA call and the events that fork it off the
-// caller's stream and join it again; one set per host thread and device.
+// The second stream of one ACA call and the events that fork it off the
+// caller's stream and join it again.  They live as long as the call (what is
+// queued on them goes on; CUDA gives them back when it is done): nothing is left
+// in a host thread that ends, or behind a device reset.
 struct AcaFork {
-    int device = -1;
     cudaStream_t stream = nullptr;
     cudaEvent_t begin = nullptr, end = nullptr;
-};
-
-static int aca_fork(AcaFork **out)
-{
-    static thread_local AcaFork f;
-    int dev;
-    PQ3D_CUDA_TRY(cudaGetDevice(&dev));
-    if (f.device != dev) {
-        if (f.device >= 0) {   // another device before: its set goes
-            cudaStreamDestroy(f.stream);
-            cudaEventDestroy(f.begin);
-            cudaEventDestroy(f.end);
-            f = AcaFork();
-        }
-        PQ3D_CUDA_TRY(cudaStreamCreateWithFlags(&f.stream, cudaStreamNonBlocking));
-        PQ3D_CUDA_TRY(cudaEventCreateWithFlags(&f.begin, cudaEventDisableTiming));
-        PQ3D_CUDA_TRY(cudaEventCreateWithFlags(&f.end, cudaEventDisableTiming));
-        f.device = dev;
+    cudaError_t open()
+    {
+        cudaError_t e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&begin, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&end, cudaEventDisableTiming);
+        return e;
     }
-    *out = &f;
-    return PQ3D_OK;
-}
+    ~AcaFork()
+    {
+        if (end) cudaEventDestroy(end);
+        if (begin) cudaEventDestroy(begin);
+        if (stream) cudaStreamDestroy(stream);
+    }
+};
 
 extern "C" int pq3d_hmat_aca(const double *tables, int64_t N, const int64_t *perm, int nblocks, const int64_t *blk,
                              const int32_t *kcap, double tol, double mu, double lambda_, int halfspace, double *UV,
@@ -1357,9 +1350,12 @@ extern "C" int pq3d_hmat_aca(const double *tables, int64_t N, const int64_t *per
     // the work order lives for this call only (stream-ordered scratch); grids
     // of nblocks clusters and CTAs serve any split, those past the last leave
     PQ3D_REQUIRE(nblocks <= INT32_MAX / kAcaCluster, "pq3d_hmat_aca: too many blocks");
-    AcaFork *fork;
-    int rc = aca_fork(&fork);
-    if (rc) return rc;
+    // A captured call takes both launches on the caller's stream, one after the
+    // other: a graph is to hold no stream of ours.
+    cudaStreamCaptureStatus capturing;
+    PQ3D_CUDA_TRY(cudaStreamIsCapturing(st, &capturing));
+    AcaFork fork;
+    if (capturing == cudaStreamCaptureStatusNone) PQ3D_CUDA_TRY(fork.open());
     int32_t *split = nullptr;
     PQ3D_CUDA_TRY(cudaMallocAsync(&split, ((size_t)nblocks + 2) * sizeof(int32_t), st));
     aca_order_kernel<<<1, 1024, 0, st>>>(blk, nblocks, split + 2, split);
@@ -1374,19 +1370,21 @@ extern "C" int pq3d_hmat_aca(const double *tables, int64_t N, const int64_t *per
         cfg.stream = st;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
-        cudaError_t e = cudaEventRecord(fork->begin, st);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(fork->stream, fork->begin, 0);
+        cudaError_t e = cudaGetLastError();   // of aca_order_kernel
+        if (e == cudaSuccess && fork.stream) e = cudaEventRecord(fork.begin, st);
+        if (e == cudaSuccess && fork.stream) e = cudaStreamWaitEvent(fork.stream, fork.begin, 0);
         if (e == cudaSuccess)
             e = cudaLaunchKernelEx(&cfg, kernel, true, gen, recv, perm, blk, (const int32_t *)(split + 2),
                                    (const int32_t *)split, nblocks, kcap, tol, UV, uv_off, used, used_off, rank, status);
-        if (e != cudaSuccess) return e;
-        kernel<<<nblocks, kAcaThreads, 0, fork->stream>>>(false, gen, recv, perm, blk, split + 2, split, nblocks, kcap,
-                                                          tol, UV, uv_off, used, used_off, rank, status);
+        if (e != cudaSuccess) return e;   // nothing is on the second stream yet
+        kernel<<<nblocks, kAcaThreads, 0, fork.stream ? fork.stream : st>>>(
+            false, gen, recv, perm, blk, split + 2, split, nblocks, kcap, tol, UV, uv_off, used, used_off, rank, status);
         e = cudaGetLastError();
-        // joined whatever happened: a capturing stream must not be left forked
-        const cudaError_t e1 = cudaEventRecord(fork->end, fork->stream);
-        const cudaError_t e2 = cudaStreamWaitEvent(st, fork->end, 0);
-        return e != cudaSuccess ? e : (e1 != cudaSuccess ? e1 : e2);
+        if (e == cudaSuccess && fork.stream) e = cudaEventRecord(fork.end, fork.stream);
+        if (e == cudaSuccess && fork.stream) e = cudaStreamWaitEvent(st, fork.end, 0);
+        // not joined: the caller's stream must not go on beside what may run there
+        if (e != cudaSuccess && fork.stream) cudaStreamSynchronize(fork.stream);
+        return e;
     };
     const cudaError_t launched = halfspace ? launch(aca_kernel<true>, make_gen<true>(tables, N, mu, lambda_))
                                            : launch(aca_kernel<false>, make_gen<false>(tables, N, mu, lambda_));
