@@ -212,7 +212,12 @@ setup_tiles_kernel(const double *__restrict__ nodes, const int64_t *__restrict__
 // -> 162.0 ms; half space, N = 2,500, shuffled 61.3 -> 36.5 ms.
 // The lines: below 2^24 pairs (7 ms; half space 2^20, 6 ms) the two launches and
 // the sort (40 us at N = 4,200, 130 us at 20,000) are a visible part of the call;
-// at 1.66 edges a triangle there is little left to gain.
+// at 1.66 edges a triangle there is little left to gain.  Full space into host
+// memory keeps the mesh's order: neighbouring lanes' triangles are not neighbours in
+// a row, and the link takes isolated 16- and 8-byte stores at a third of the rate
+// (N = 20,040, shuffled, FP64 / with the FP32 copy: 436 / 903 ms sorted, 288 / 290 ms
+// as it is; in column order 181 / 319 and 168 / 170 ms).  The half space is slow
+// enough for the link either way (N = 3,600, shuffled: 77 ms sorted).
 constexpr int64_t kOrderPairs = 1 << 24, kOrderPairsHs = 1 << 20;
 constexpr int kOrderEdges = 166;   // per 100 triangles
 constexpr int kOrderThreads = 1024;
@@ -933,7 +938,7 @@ static int seg_receivers(int most, int64_t tiles, int64_t rows, int64_t slots)
 
 static int assemble_rows(const double *nodes, const int64_t *tris, int64_t N, int64_t row0, int64_t row1, double mu,
                          double lam, double *K64, float *K32, double *ws, bool do_setup, cudaStream_t st,
-                         bool half = false)
+                         bool half = false, bool to_host = false)
 {
     double *src = ws, *recv = src + (size_t)kSrcStride * N;
     double *img = recv + (size_t)kRecvStride * N, *fsc = img + (size_t)kImgStride * N;
@@ -947,7 +952,7 @@ static int assemble_rows(const double *nodes, const int64_t *tris, int64_t N, in
         if (half) setup_hs_kernel<<<(unsigned)((N + th - 1) / th), th, 0, st>>>(nodes, tris, N, img, fsc);
         setup_tiles_kernel<<<(unsigned)nt, kTileMax, 0, st>>>(nodes, tris, N, ts, nullptr, tiles, hs);
         const int64_t rows = row1 > row0 ? row1 - row0 : N;   // no rows: they follow, all of them
-        if (rows * N >= (half ? kOrderPairsHs : kOrderPairs)) {
+        if (rows * N >= (half ? kOrderPairsHs : kOrderPairs) && (half || !to_host)) {
             int32_t *order = (int32_t *)(ws + order_offset(N, half));
             order_tiles_kernel<<<1, kOrderThreads, 0, st>>>(recv, N, nt, tiles, order);
             setup_tiles_kernel<<<(unsigned)nt, kTileMax, 0, st>>>(nodes, tris, N, ts, order, tiles, hs);
@@ -1087,10 +1092,11 @@ static void *mapped_device_ptr(void *host)
     return (a.type == cudaMemoryTypeHost) ? a.devicePointer : nullptr;
 }
 
-// Output already in mapped page-locked host memory: the assembly kernel
-// stores straight into it (its output rate, ~40 GB/s at N = 20,000, is far
-// below the host link's), one launch over all rows, no staging buffers and
-// no separate copies.
+// Output already in mapped page-locked host memory: the assembly kernel stores
+// straight into it, one launch over all rows, no staging buffers and no separate
+// copies.  In the mesh's own order a warp's stores are 512 contiguous bytes, which
+// the host link takes as fast as they come (N = 20,040: 168 ms, 115 GB/s; 170 ms,
+// 170 GB/s, with the FP32 copy).
 static int assemble_host_direct(const double *nodes_host, int64_t n_nodes, const int64_t *tris_host, int64_t N,
                                 double mu, double lambda_, bool half, double *dK64, float *dK32)
 {
@@ -1112,7 +1118,7 @@ static int assemble_host_direct(const double *nodes_host, int64_t n_nodes, const
     PQ3D_D_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     PQ3D_D_TRY(cudaMemcpyAsync(d_nodes, nodes_host, 3 * n_nodes * sizeof(double), cudaMemcpyHostToDevice, st));
     PQ3D_D_TRY(cudaMemcpyAsync(d_tris, tris_host, 3 * N * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-    rc = assemble_rows(d_nodes, d_tris, N, 0, N, mu, lambda_, dK64, dK32, d_ws, true, st, half);
+    rc = assemble_rows(d_nodes, d_tris, N, 0, N, mu, lambda_, dK64, dK32, d_ws, true, st, half, true);
     if (rc) goto done;
     PQ3D_D_TRY(cudaStreamSynchronize(st));
 done:
