@@ -604,19 +604,14 @@ __device__ __forceinline__ void t_row_group(const float *__restrict__ v, int nc,
     for (int j = 0; j < 4; ++j) out[j] = warp_sum_ff(sum[j]);
 }
 
-__global__ void __launch_bounds__(kTWarps * 32, 6)
-lowrank_T_kernel(const float *__restrict__ data, const longlong2 *__restrict__ t_info,
-                 const int32_t *__restrict__ t_sched, const longlong2 *__restrict__ t_grp, int64_t ngrp,
-                 int64_t nshort, int64_t nlong, int64_t short_ctas,
-                 const float2 *__restrict__ Xs, int64_t N, int B, float2 *__restrict__ T, const int32_t *act,
-                 int act_stride)
+// CTA cta of the rank rows of run r (of B): all threads of a block of kTWarps warps.
+__device__ __forceinline__ void lowrank_T_cta(int64_t cta, const float *__restrict__ data,
+                                              const longlong2 *__restrict__ t_info, const int32_t *__restrict__ t_sched,
+                                              const longlong2 *__restrict__ t_grp, int64_t ngrp, int64_t nshort,
+                                              int64_t nlong, int64_t short_ctas, const float2 *__restrict__ xr, int B,
+                                              int r, float2 *__restrict__ T, FF *part)
 {
-    __shared__ FF part[kTWarps];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int r = (int)(blockIdx.x % (unsigned)B);
-    const int64_t cta = blockIdx.x / (unsigned)B;
-    if (!run_on(act, act_stride, r)) return;   // uniform per CTA
-    const float2 *xr = Xs + (int64_t)r * 2 * N;
     if (cta < short_ctas) {
         const int64_t g0 = (cta * kTWarps + wid) * kTGroupsPerWarp;
         if (g0 >= ngrp) return;
@@ -652,6 +647,33 @@ lowrank_T_kernel(const float *__restrict__ data, const longlong2 *__restrict__ t
         for (int k = 1; k < kTWarps; ++k) t = ff_add(t, part[k]);
         T[w * (int64_t)B + r] = make_float2(t.hi, t.lo);
     }
+}
+
+__global__ void __launch_bounds__(kTWarps * 32, 6)
+lowrank_T_kernel(const float *__restrict__ data, const longlong2 *__restrict__ t_info,
+                 const int32_t *__restrict__ t_sched, const longlong2 *__restrict__ t_grp, int64_t ngrp,
+                 int64_t nshort, int64_t nlong, int64_t short_ctas,
+                 const float2 *__restrict__ Xs, int64_t N, int B, float2 *__restrict__ T, const int32_t *act,
+                 int act_stride)
+{
+    __shared__ FF part[kTWarps];
+    const int r = (int)(blockIdx.x % (unsigned)B);
+    const int64_t cta = blockIdx.x / (unsigned)B;
+    if (!run_on(act, act_stride, r)) return;   // uniform per CTA
+    lowrank_T_cta(cta, data, t_info, t_sched, t_grp, ngrp, nshort, nlong, short_ctas, Xs + (int64_t)r * 2 * N, B, r, T,
+                  part);
+}
+
+// The same for a batch's only run that takes part (list: run_list_kernel).
+__global__ void __launch_bounds__(kTWarps * 32, 6)
+lowrank_T_only_kernel(const float *__restrict__ data, const longlong2 *__restrict__ t_info,
+                      const int32_t *__restrict__ t_sched, const longlong2 *__restrict__ t_grp, int64_t ngrp,
+                      int64_t nshort, int64_t nlong, int64_t short_ctas, const float2 *__restrict__ xr,
+                      float2 *__restrict__ T, const int32_t *__restrict__ list)
+{
+    __shared__ FF part[kTWarps];
+    if (list[0] != 1) return;
+    lowrank_T_cta(blockIdx.x, data, t_info, t_sched, t_grp, ngrp, nshort, nlong, short_ctas, xr, 1, 0, T, part);
 }
 
 // ---------------------------------------------------------------------------
@@ -758,13 +780,17 @@ __device__ __forceinline__ FFPair ff_add2p(FFPair a, uint64_t b)
 }
 
 __global__ void permute_split_runs_kernel(const double *__restrict__ X, const int64_t *__restrict__ perm, int64_t N,
-                                          const int32_t *__restrict__ list, Pair2 *__restrict__ Xs)
+                                          const int32_t *__restrict__ list, bool only, Pair2 *__restrict__ Xs)
 {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int left = list[0] - 8 * (int)blockIdx.y;
     if (i >= 2 * N || left <= 0) return;
     const int64_t col = 2 * perm[i >> 1] + (i & 1);
     const int32_t *run = list + 1 + 8 * blockIdx.y;
+    if (only && list[0] == 1) {
+        reinterpret_cast<float2 *>(Xs)[i] = split2(X[(int64_t)run[0] * 2 * N + col]);
+        return;
+    }
     for (int h = 0; h < group_width(left) / 2; ++h) {
         float2 v[2];
         for (int j = 0; j < 2; ++j)
@@ -876,7 +902,7 @@ __global__ void __launch_bounds__(kTWarps * 32, 4)
 lowrank_T_runs_kernel(const float *__restrict__ data, const longlong2 *__restrict__ t_info,
                       const int32_t *__restrict__ t_sched, const longlong2 *__restrict__ t_grp, int64_t ngrp,
                       int64_t nshort, int64_t nlong, int64_t short_ctas, const Pair2 *__restrict__ Xs, int64_t N,
-                      int64_t t_rows, int nquads, Pair2 *__restrict__ T, const int32_t *__restrict__ list)
+                      int64_t t_rows, int nquads, Pair2 *__restrict__ T, const int32_t *__restrict__ list, bool only)
 {
     __shared__ FF part[kTWarps];
     __shared__ FFPair kept[kTWarps][8 * 32];
@@ -884,7 +910,7 @@ lowrank_T_runs_kernel(const float *__restrict__ data, const longlong2 *__restric
     const int quad = (int)(blockIdx.x % (unsigned)nquads), grp = quad >> 1, half = quad & 1;
     const int64_t cta = blockIdx.x / (unsigned)nquads;
     const int left = list[0] - 8 * grp;
-    if (left <= 4 * half) return;   // uniform per CTA
+    if (left <= 4 * half || (only && list[0] == 1)) return;   // uniform per CTA
     const int nr = min(4, group_width(left));
     const Pair2 *xg = Xs + (4 * grp + 2 * half) * 2 * N;
     Pair2 *Tg = T + (4 * grp + 2 * half) * t_rows;
@@ -1045,24 +1071,19 @@ __device__ __forceinline__ void load_leaf_blocks(BlkDesc *desc, int *wpre, int n
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kThreads, 3)
-leaf_rows_kernel(const float *__restrict__ data, const int64_t *__restrict__ off, const int64_t *__restrict__ blk,
-                 const int32_t *__restrict__ rank, const int64_t *__restrict__ leaf, const int64_t *__restrict__ leaf_ptr,
-                 const int32_t *__restrict__ leaf_blocks, const int64_t *__restrict__ perm, const float2 *__restrict__ Xs,
-                 const float2 *__restrict__ T, const int64_t *__restrict__ t_off, int64_t N, int B,
-                 double *__restrict__ Y, const int32_t *act, int act_stride)
+// Leaf L of run r (of B), whose x values are xr and whose output is Yr: all threads.
+__device__ __forceinline__ void leaf_rows_cta(int L, const float *__restrict__ data, const int64_t *__restrict__ off,
+                                              const int64_t *__restrict__ blk, const int32_t *__restrict__ rank,
+                                              const int64_t *__restrict__ leaf, const int64_t *__restrict__ leaf_ptr,
+                                              const int32_t *__restrict__ leaf_blocks, const int64_t *__restrict__ perm,
+                                              const float2 *__restrict__ xr, const float2 *__restrict__ T,
+                                              const int64_t *__restrict__ t_off, int B, int r, double *__restrict__ Yr,
+                                              BlkDesc *desc, int *wpre, double (*red)[kPassRows])
 {
-    __shared__ BlkDesc desc[kMaxLeafBlocks];
-    __shared__ int wpre[kMaxLeafBlocks + 1];
-    __shared__ double red[kWarps][kPassRows];
-    const int L = (int)(blockIdx.x / (unsigned)B), r = (int)(blockIdx.x % (unsigned)B);
-    if (!run_on(act, act_stride, r)) return;   // uniform per CTA: before any barrier
     const int64_t p0 = leaf[2 * L], p1 = leaf[2 * L + 1];
     const int rows = 3 * (int)(p1 - p0);
     const int64_t q0 = leaf_ptr[L], q1 = leaf_ptr[L + 1];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const float2 *xr = Xs + (int64_t)r * 2 * N;
-    double *Yr = Y + (int64_t)r * 3 * N;
     for (int pr0 = 0; pr0 < rows; pr0 += kPassRows) {
         const int prow = min(kPassRows, rows - pr0);
         const int R = (prow + 31) / 32;
@@ -1097,6 +1118,39 @@ leaf_rows_kernel(const float *__restrict__ data, const int64_t *__restrict__ off
     }
 }
 
+__global__ void __launch_bounds__(kThreads, 3)
+leaf_rows_kernel(const float *__restrict__ data, const int64_t *__restrict__ off, const int64_t *__restrict__ blk,
+                 const int32_t *__restrict__ rank, const int64_t *__restrict__ leaf, const int64_t *__restrict__ leaf_ptr,
+                 const int32_t *__restrict__ leaf_blocks, const int64_t *__restrict__ perm, const float2 *__restrict__ Xs,
+                 const float2 *__restrict__ T, const int64_t *__restrict__ t_off, int64_t N, int B,
+                 double *__restrict__ Y, const int32_t *act, int act_stride)
+{
+    __shared__ BlkDesc desc[kMaxLeafBlocks];
+    __shared__ int wpre[kMaxLeafBlocks + 1];
+    __shared__ double red[kWarps][kPassRows];
+    const int L = (int)(blockIdx.x / (unsigned)B), r = (int)(blockIdx.x % (unsigned)B);
+    if (!run_on(act, act_stride, r)) return;   // uniform per CTA: before any barrier
+    leaf_rows_cta(L, data, off, blk, rank, leaf, leaf_ptr, leaf_blocks, perm, Xs + (int64_t)r * 2 * N, T, t_off, B, r,
+                  Y + (int64_t)r * 3 * N, desc, wpre, red);
+}
+
+// The same for a batch's only run that takes part.
+__global__ void __launch_bounds__(kThreads, 3)
+leaf_rows_only_kernel(const float *__restrict__ data, const int64_t *__restrict__ off, const int64_t *__restrict__ blk,
+                      const int32_t *__restrict__ rank, const int64_t *__restrict__ leaf,
+                      const int64_t *__restrict__ leaf_ptr, const int32_t *__restrict__ leaf_blocks,
+                      const int64_t *__restrict__ perm, const float2 *__restrict__ xr, const float2 *__restrict__ T,
+                      const int64_t *__restrict__ t_off, int64_t N, double *__restrict__ Y,
+                      const int32_t *__restrict__ list)
+{
+    __shared__ BlkDesc desc[kMaxLeafBlocks];
+    __shared__ int wpre[kMaxLeafBlocks + 1];
+    __shared__ double red[kWarps][kPassRows];
+    if (list[0] != 1) return;
+    leaf_rows_cta((int)blockIdx.x, data, off, blk, rank, leaf, leaf_ptr, leaf_blocks, perm, xr, T, t_off, 1, 0,
+                  Y + (int64_t)list[1] * 3 * N, desc, wpre, red);
+}
+
 // The leaf rows for NR runs: as leaf_rows_kernel, a CTA per (leaf, group of
 // runs), the work columns in the same 8 ranges.  Lanes own up to kRunRows / NR
 // rows (24 f32x2 accumulators a lane).  The x values of 32 columns come into
@@ -1105,14 +1159,17 @@ leaf_rows_kernel(const float *__restrict__ data, const int64_t *__restrict__ off
 // on (4 in wide passes) as soon as it is used; the float-float sums, touched
 // once per block segment, live in shared memory.  The row passes of a leaf are
 // independent: two CTAs take every other one (N = 30,000: 512 leaves are 1,024
-// CTAs for 304 places, whose last round was half empty).
+// CTAs for 304 places, whose last round was half empty).  What a CTA leaves of its
+// share of shared memory is L1: with the warps' sums in place of the staged x, no
+// longer needed then, 60 KB instead of 28 (N = 29,756: 16 runs 1,028 -> 985 us, 2 runs
+// 418 -> 365).
 constexpr int kRunRows = 24;
 constexpr int kRunMaxR = 6;
 constexpr int kRunPasses = 2;   // CTAs of a leaf and run group
 constexpr int kRunFF = kRunRows * kThreads * (int)sizeof(float2);                  // float-float sums
 constexpr int kRunX = kWarps * 2 * 32 * 4 * (int)sizeof(Pair2);                    // staged x, two chunks
 constexpr int kRunRed = kWarps * 32 * kRunMaxR * (int)sizeof(double);              // one run's warp sums
-constexpr int kRunSmem = kRunFF + kRunX + kRunRed;
+constexpr int kRunSmem = kRunFF + (kRunX > kRunRed ? kRunX : kRunRed);
 
 __device__ __forceinline__ void copy16_async(void *smem, const void *gmem)
 {
@@ -1218,7 +1275,7 @@ __device__ __forceinline__ void leaf_rows_runs(const float *__restrict__ data, c
                                                const int32_t *__restrict__ leaf_blocks, const int64_t *__restrict__ perm,
                                                const Pair2 *__restrict__ xg, const Pair2 *__restrict__ Tg,
                                                const int64_t *__restrict__ t_off, int64_t t_rows, int64_t N, int runs,
-                                               const int32_t *__restrict__ run, double *__restrict__ Y, int pass0, BlkDesc *desc,
+                                               const int32_t *__restrict__ run, double *__restrict__ Y, int pass0, int pass_rows, BlkDesc *desc,
                                                int *wpre, char *smem)
 {
     constexpr int kR = kRunRows / NR < kRunMaxR ? kRunRows / NR : kRunMaxR;
@@ -1226,10 +1283,11 @@ __device__ __forceinline__ void leaf_rows_runs(const float *__restrict__ data, c
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     FFPair *ff = reinterpret_cast<FFPair *>(smem) + threadIdx.x;
     Pair2 *sx = reinterpret_cast<Pair2 *>(smem + kRunFF) + wid * 2 * 32 * 4;
-    double *red = reinterpret_cast<double *>(smem + kRunFF + kRunX);
+    double *red = reinterpret_cast<double *>(smem + kRunFF);   // once the staged x is done with
     const int rows = 3 * (int)(p1 - p0);
-    for (int pr0 = pass0 * kPass; pr0 < rows; pr0 += kRunPasses * kPass) {
-        const int prow = min(kPass, rows - pr0);
+    const int pass = min(kPass, pass_rows);
+    for (int pr0 = pass0 * pass; pr0 < rows; pr0 += kRunPasses * pass) {
+        const int prow = min(pass, rows - pr0);
         const int R = (prow + 31) / 32;
         for (int i = 0; i < kR * NR / 2; ++i) ff[i * kThreads] = FFPair{0ull, 0ull};
         for (int64_t qs = q0; qs < q1; qs += kMaxLeafBlocks) {
@@ -1270,7 +1328,7 @@ leaf_rows_runs_kernel(const float *__restrict__ data, const int64_t *__restrict_
                       const int64_t *__restrict__ leaf_ptr, const int32_t *__restrict__ leaf_blocks,
                       const int64_t *__restrict__ perm, const Pair2 *__restrict__ Xs, const Pair2 *__restrict__ T,
                       const int64_t *__restrict__ t_off, int64_t t_rows, int64_t N, int ngroups,
-                      const int32_t *__restrict__ list, double *__restrict__ Y)
+                      const int32_t *__restrict__ list, bool only, int pass_rows, double *__restrict__ Y)
 {
     extern __shared__ __align__(16) char smem_runs[];
     __shared__ BlkDesc desc[kMaxLeafBlocks];
@@ -1279,20 +1337,20 @@ leaf_rows_runs_kernel(const float *__restrict__ data, const int64_t *__restrict_
     const unsigned lp = blockIdx.x / (unsigned)ngroups;
     const int L = (int)(lp / kRunPasses), pass0 = (int)(lp % kRunPasses);
     const int left = list[0] - 8 * grp;
-    if (left <= 0) return;   // uniform per CTA
+    if (left <= 0 || (only && list[0] == 1)) return;   // uniform per CTA
     const int w = group_width(left), runs = min(left, 8);
     const Pair2 *xg = Xs + 4 * grp * 2 * N, *Tg = T + 4 * grp * t_rows;
     const int32_t *run = list + 1 + 8 * grp;
     const int64_t p0 = leaf[2 * L], p1 = leaf[2 * L + 1], q0 = leaf_ptr[L], q1 = leaf_ptr[L + 1];
     if (w == 8)
         leaf_rows_runs<8>(data, off, blk, rank, p0, p1, q0, q1, leaf_blocks, perm, xg, Tg, t_off, t_rows, N, runs, run, Y, pass0,
-                          desc, wpre, smem_runs);
+                          pass_rows, desc, wpre, smem_runs);
     else if (w == 4)
         leaf_rows_runs<4>(data, off, blk, rank, p0, p1, q0, q1, leaf_blocks, perm, xg, Tg, t_off, t_rows, N, runs, run, Y, pass0,
-                          desc, wpre, smem_runs);
+                          pass_rows, desc, wpre, smem_runs);
     else
         leaf_rows_runs<2>(data, off, blk, rank, p0, p1, q0, q1, leaf_blocks, perm, xg, Tg, t_off, t_rows, N, runs, run, Y, pass0,
-                          desc, wpre, smem_runs);
+                          pass_rows, desc, wpre, smem_runs);
 }
 
 }  // namespace hm
@@ -1435,49 +1493,68 @@ extern "C" int pq3d_hmat_apply_masked(const pq3d_hmat *H, const double *X, int B
     PQ3D_REQUIRE(workspace_bytes >= need && aligned16(workspace), "pq3d_hmat_apply: workspace too small (%zu < %zu)",
                  workspace_bytes, need);
     cudaStream_t st = (cudaStream_t)stream;
+    const longlong2 *t_info = (const longlong2 *)H->t_info, *t_grp = (const longlong2 *)H->t_grp;
     const int64_t nshort = H->t_rows - H->t_nlong;
     const int64_t short_ctas = (H->t_ngrp + kTWarps * kTGroupsPerWarp - 1) / (kTWarps * kTGroupsPerWarp);
-    if (B > 1) {
-        const int64_t slots = run_slots(B);
-        const int ngroups = (B + 7) / 8;
-        Pair2 *Xs = (Pair2 *)workspace, *T = Xs + (size_t)(slots / 2) * 2 * N;
-        int32_t *list = (int32_t *)(T + (size_t)(slots / 2) * H->t_rows);
-        PQ3D_CUDA_TRY(allow_smem(leaf_rows_runs_kernel, kRunSmem));
-        PQ3D_REQUIRE((short_ctas + H->t_nlong) * 2 * ngroups < (int64_t)INT32_MAX &&
-                         (int64_t)H->nleaves * ngroups * kRunPasses < (int64_t)INT32_MAX && ngroups < 65536,
+    const int64_t t_ctas = short_ctas + H->t_nlong;
+    const unsigned cols = (unsigned)((2 * N + 255) / 256);
+    int dev, sms;
+    PQ3D_CUDA_TRY(cudaGetDevice(&dev));
+    PQ3D_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // One run, or so few leaves that a CTA for each and every run still finds room on
+    // the chip: run by run, the run fastest in the block index.  (8 runs: N = 900, 32
+    // leaves 35 us, 47 in a group; N = 2,500, 64 leaves 76, 71.)
+    if (B == 1 || (int64_t)H->nleaves * B <= 2 * sms) {
+        PQ3D_REQUIRE(t_ctas * B < (int64_t)INT32_MAX && (int64_t)H->nleaves * B < (int64_t)INT32_MAX,
                      "pq3d_hmat_apply: too many rank rows or leaves x runs");
-        run_list_kernel<<<1, 32, 0, st>>>(B, run_active, active_stride, list);
-        permute_split_runs_kernel<<<dim3((unsigned)((2 * N + 255) / 256), (unsigned)ngroups), 256, 0, st>>>(
-            X, H->perm, N, list, Xs);
+        float2 *Xs = (float2 *)workspace, *T = Xs + (size_t)B * 2 * N;
+        permute_split_kernel<<<dim3(cols, (unsigned)B), 256, 0, st>>>(X, H->perm, N, B, Xs, run_active, active_stride);
         if (H->t_rows > 0)
-            lowrank_T_runs_kernel<<<(unsigned)((short_ctas + H->t_nlong) * 2 * ngroups), kTWarps * 32, 0, st>>>(
-                H->data, (const longlong2 *)H->t_info, H->t_sched, (const longlong2 *)H->t_grp, H->t_ngrp, nshort,
-                H->t_nlong, short_ctas, Xs, N, H->t_rows, 2 * ngroups, T, list);
-        leaf_rows_runs_kernel<<<(unsigned)(H->nleaves * ngroups * kRunPasses), kThreads, kRunSmem, st>>>(
-            H->data, H->off, H->blk, H->rank, H->leaf, H->leaf_ptr, H->leaf_blocks, H->perm, Xs, T, H->t_off, H->t_rows,
-            N, ngroups, list, Y);
+            lowrank_T_kernel<<<(unsigned)(t_ctas * B), kTWarps * 32, 0, st>>>(
+                H->data, t_info, H->t_sched, t_grp, H->t_ngrp, nshort, H->t_nlong, short_ctas, Xs, N, B, T, run_active,
+                active_stride);
+        leaf_rows_kernel<<<(unsigned)(H->nleaves * B), kThreads, 0, st>>>(
+            H->data, H->off, H->blk, H->rank, H->leaf, H->leaf_ptr, H->leaf_blocks, H->perm, Xs, T, H->t_off, N, B, Y,
+            run_active, active_stride);
         PQ3D_CUDA_TRY(cudaGetLastError());
         return PQ3D_OK;
     }
-    float2 *Xs = (float2 *)workspace;
-    float2 *T = (float2 *)((char *)workspace + (size_t)B * 2 * N * sizeof(float2));
-    dim3 g1((unsigned)((2 * N + 255) / 256), (unsigned)B);
-    permute_split_kernel<<<g1, 256, 0, st>>>(X, H->perm, N, B, Xs, run_active, active_stride);
-    // all runs in one launch, run fastest in the block index; a run's result
-    // does not depend on B
-    if (H->t_rows > 0) {
-        const int64_t nT = (short_ctas + H->t_nlong) * B;
-        PQ3D_REQUIRE(nT < (int64_t)INT32_MAX, "pq3d_hmat_apply: too many rank rows x runs");
-        lowrank_T_kernel<<<(unsigned)nT, kTWarps * 32, 0, st>>>(H->data, (const longlong2 *)H->t_info, H->t_sched,
-                                                               (const longlong2 *)H->t_grp,
-                                                       H->t_ngrp, nshort,
-                                                       H->t_nlong, short_ctas, Xs, N, B, T, run_active,
-                                                       active_stride);
+    const int64_t slots = run_slots(B);
+    const int ngroups = (B + 7) / 8;
+    PQ3D_REQUIRE(t_ctas * 2 * ngroups < (int64_t)INT32_MAX &&
+                     (int64_t)H->nleaves * ngroups * kRunPasses < (int64_t)INT32_MAX && ngroups < 65536,
+                 "pq3d_hmat_apply: too many rank rows or leaves x runs");
+    Pair2 *Xs = (Pair2 *)workspace, *T = Xs + (size_t)(slots / 2) * 2 * N;
+    int32_t *list = (int32_t *)(T + (size_t)(slots / 2) * H->t_rows);
+    // Rows of a leaf's pass: half of them where the leaves leave SMs without a CTA, so
+    // that a leaf's second CTA takes the rest (2 runs: N = 8,100, 184 leaves 144 us,
+    // whole passes 158; N = 12,100, 256 leaves 188, 175).
+    const int pass_rows = 3 * (int64_t)H->nleaves * ngroups <= 4 * sms ? kPassRows / 2 : kPassRows;
+    // How many runs take part is known on the device only.  A batch's only run does
+    // better with the one-run kernels, from about four leaves an SM on (N = 99,856:
+    // 1,075 us, 1,189 as half a pair; N = 29,756, 512 leaves: 362, 361): they follow
+    // those below, which leave it to them, and else end at once (15 us there).
+    const bool only = run_active && H->nleaves > 4 * sms;
+    PQ3D_CUDA_TRY(allow_smem(leaf_rows_runs_kernel, kRunSmem));
+    run_list_kernel<<<1, 32, 0, st>>>(B, run_active, active_stride, list);
+    permute_split_runs_kernel<<<dim3(cols, (unsigned)ngroups), 256, 0, st>>>(X, H->perm, N, list, only, Xs);
+    if (H->t_rows > 0)
+        lowrank_T_runs_kernel<<<(unsigned)(t_ctas * 2 * ngroups), kTWarps * 32, 0, st>>>(
+            H->data, t_info, H->t_sched, t_grp, H->t_ngrp, nshort, H->t_nlong, short_ctas, Xs, N, H->t_rows, 2 * ngroups,
+            T, list, only);
+    leaf_rows_runs_kernel<<<(unsigned)(H->nleaves * ngroups * kRunPasses), kThreads, kRunSmem, st>>>(
+        H->data, H->off, H->blk, H->rank, H->leaf, H->leaf_ptr, H->leaf_blocks, H->perm, Xs, T, H->t_off, H->t_rows, N,
+        ngroups, list, only, pass_rows, Y);
+    if (only) {
+        const float2 *x1 = (const float2 *)Xs;
+        float2 *T1 = (float2 *)T;
+        if (H->t_rows > 0)
+            lowrank_T_only_kernel<<<(unsigned)t_ctas, kTWarps * 32, 0, st>>>(
+                H->data, t_info, H->t_sched, t_grp, H->t_ngrp, nshort, H->t_nlong, short_ctas, x1, T1, list);
+        leaf_rows_only_kernel<<<(unsigned)H->nleaves, kThreads, 0, st>>>(
+            H->data, H->off, H->blk, H->rank, H->leaf, H->leaf_ptr, H->leaf_blocks, H->perm, x1, T1, H->t_off, N, Y,
+            list);
     }
-    PQ3D_REQUIRE((int64_t)H->nleaves * B < (int64_t)INT32_MAX, "pq3d_hmat_apply: too many leaves x runs");
-    const unsigned gL = (unsigned)(H->nleaves * B);
-    leaf_rows_kernel<<<gL, kThreads, 0, st>>>(H->data, H->off, H->blk, H->rank, H->leaf, H->leaf_ptr, H->leaf_blocks,
-                                              H->perm, Xs, T, H->t_off, N, B, Y, run_active, active_stride);
     PQ3D_CUDA_TRY(cudaGetLastError());
     return PQ3D_OK;
 }
