@@ -102,13 +102,14 @@ __device__ __forceinline__ float4 split_v(double v1, double v2)
     return make_float4(h1, h2, (float)(v1 - (double)h1), (float)(v2 - (double)h2));
 }
 
+template <int U>   // 64 U sources in flight
 __device__ __forceinline__ void rows3_f32(const float2 *__restrict__ K, const float4 *__restrict__ v, int64_t N,
                                           int64_t i, int64_t j0, int64_t j1, int lane, double acc[3])
 {
     const float2 *r0 = K + (3 * i) * N, *r1 = r0 + N, *r2 = r1 + N;
     Acc2 a0{0.f, 0.f}, a1{0.f, 0.f}, a2{0.f, 0.f};
     int64_t j = j0 + lane;
-#pragma unroll 4   // 256 sources in flight (N = 15,000: 1.29 ms a step with 64, 0.97)
+#pragma unroll U
     for (; j + 32 < j1; j += 64) {
         const float4 x0 = __ldg(v + j), x1 = __ldg(v + j + 32);
         const float2 k00 = __ldcs(r0 + j), k10 = __ldcs(r1 + j), k20 = __ldcs(r2 + j);
@@ -137,14 +138,14 @@ __device__ __forceinline__ void rows3_f32(const float2 *__restrict__ K, const fl
 // of the first.  A warp has two rounds of loads in flight, so a small operator
 // (in L2) needs more than N warps to keep the FP64 pipe fed: N = 1,600 with S =
 // 1 (11 warps per SM) 46.9 us, S = 2 39.1 us, against 24.5 us of multiply-adds.
-template <bool kF32, int S>
+template <bool kF32, int S, int U>
 __device__ __forceinline__ void receiver_rows(const void *K, const void *v, int64_t N, int64_t i, double acc[3])
 {
     __shared__ double part[8][3];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, p = w % S;
     const int64_t len = (N + 32 * S - 1) / (32 * S) * 32, j0 = p * len, j1 = min(N, j0 + len);
     if (i < N) {
-        if (kF32) rows3_f32((const float2 *)K, (const float4 *)v, N, i, j0, j1, lane, acc);
+        if (kF32) rows3_f32<U>((const float2 *)K, (const float4 *)v, N, i, j0, j1, lane, acc);
         else rows3_f64((const double2 *)K, (const double2 *)v, N, i, j0, j1, lane, acc);
     }
     if (S == 1) return;
@@ -155,21 +156,48 @@ __device__ __forceinline__ void receiver_rows(const void *K, const void *v, int6
             for (int c = 0; c < 3; ++c) acc[c] += part[w + q][c];
 }
 
-// warps per receiver: at least 16 warps per SM where the mesh is too small for that
-static int receiver_warps(int64_t N, int sms)
+// How a product is launched: S warps per receiver (1, 2 or 4), and for the FP32
+// operator the blocks that an SM holds (2 with 256 sources in flight a warp, 3 with
+// the same in fewer registers, 4 with 64).
+struct RowShape {
+    int s, r;
+};
+
+// b: an SM's blocks of 8 receivers.  Up to two of them the warps per receiver are
+// those for which the busiest SM's blocks times a block's time (its sources and
+// about 200 more for its start and sums) is least; more, and none are split
+// (FP64), since blocks come and go.  The FP32 operator is bound by the loads in
+// flight, and its blocks are best all resident at once: three and four take the
+// builds that allow it, and from five on two warps per receiver even out the last
+// ones.  us (one warp per receiver and 2 blocks per SM / as chosen):
+// FP64 N = 400 8.1 / 6.2, 1,000 18.3 / 18.3 (with 4 warps 23.4), 1,600 43.6 / 37.4;
+// FP32 N = 304 4.8 / 4.0, 2,500 37.9 / 29.6, 3,000 52.0 / 38.0, 4,000 70.1 / 65.6,
+// 5,000 120 / 105, 8,000 259 / 249, 20,000 1,458 / 1,401.
+static RowShape row_shape(int64_t N, bool f32, int sms)
 {
-    int s = 1;
-    while (s < 8 && N * s < 16 * (int64_t)sms) s *= 2;
-    return s;
+    const int64_t b = (N + 8 * sms - 1) / (8 * (int64_t)sms);
+    if (b > 2) return f32 ? (b == 3 ? RowShape{1, 3} : (b == 4 ? RowShape{1, 4} : RowShape{2, 3})) : RowShape{1, 2};
+    int best = 1;
+    int64_t cost = INT64_MAX;
+    for (int s = 1; s <= 4 && 32 * (s - 1) < N; s *= 2) {   // none without sources
+        const int64_t blocks = (N * s + 7) / 8, c = (blocks + sms - 1) / sms * (N / s + 200);
+        if (c < cost) { cost = c; best = s; }
+    }
+    return RowShape{best, 2};
 }
 
-template <bool kF32, int S>
-__global__ void __launch_bounds__(256, kF32 ? 1 : 0) matvec_kernel(const void *__restrict__ K, const void *__restrict__ v,
+// the builds' registers (FP64: the compiler's own choice) and loads in flight
+#define PQ3D_ROWS_BOUNDS __launch_bounds__(256, kF32 ? R : 0)
+template <int R>
+constexpr int kRowsUnroll = R == 4 ? 1 : 4;
+
+template <bool kF32, int S, int R>
+__global__ void PQ3D_ROWS_BOUNDS matvec_kernel(const void *__restrict__ K, const void *__restrict__ v,
                                                      int64_t N, double *__restrict__ out)
 {
     const int64_t i = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) / S;
     double acc[3];
-    receiver_rows<kF32, S>(K, v, N, i, acc);
+    receiver_rows<kF32, S, kRowsUnroll<R>>(K, v, N, i, acc);
     if (i < N && (threadIdx.x & 31) == 0 && (threadIdx.x >> 5) % S == 0) {
         out[3 * i] = acc[0];
         out[3 * i + 1] = acc[1];
@@ -250,12 +278,12 @@ __global__ void __launch_bounds__(256) vprime_kernel(pq3d_dense_sim S)
 
 // (1) traction rates of one step (src/QDsim_gpu.py:948-957): the normal
 // component with the normal loading added (or the loading alone with fix_Tn)
-template <bool kF32, int S>
-__global__ void __launch_bounds__(256, kF32 ? 1 : 0) step_rates_kernel(pq3d_dense_sim D)
+template <bool kF32, int S, int R>
+__global__ void PQ3D_ROWS_BOUNDS step_rates_kernel(pq3d_dense_sim D)
 {
     const int64_t i = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) / S;
     double acc[3];
-    receiver_rows<kF32, S>(kF32 ? (const void *)D.K32 : (const void *)D.K64, D.vprime, D.N, i, acc);
+    receiver_rows<kF32, S, kRowsUnroll<R>>(kF32 ? (const void *)D.K32 : (const void *)D.K64, D.vprime, D.N, i, acc);
     if (i < D.N && (threadIdx.x & 31) == 0 && (threadIdx.x >> 5) % S == 0) {
         D.rates[3 * i] = acc[0];
         D.rates[3 * i + 1] = acc[1];
@@ -545,24 +573,31 @@ static int attempt_grid(const LaunchCfg &c, bool f32, int64_t N)
 // the FP64 pipe as four warps of quads, whose chains are three times shorter.
 constexpr int64_t kQuadCells = 32;
 
+// kernel<kF32, S, R> of a shape
+#define PQ3D_ROWS_LAUNCH(kernel, shape, N, st, ...)                                                        \
+    do {                                                                                                   \
+        const unsigned blocks_ = (unsigned)(((N) * (shape).s + 7) / 8);                                    \
+        if (!kF32 || (shape).r == 2) {                                                                     \
+            if ((shape).s == 1) kernel<kF32, 1, 2><<<blocks_, 256, 0, st>>>(__VA_ARGS__);                  \
+            else if ((shape).s == 2) kernel<kF32, 2, 2><<<blocks_, 256, 0, st>>>(__VA_ARGS__);             \
+            else kernel<kF32, 4, 2><<<blocks_, 256, 0, st>>>(__VA_ARGS__);                                 \
+        } else if constexpr (kF32) {                                                                       \
+            if ((shape).r == 4) kernel<true, 1, 4><<<blocks_, 256, 0, st>>>(__VA_ARGS__);                  \
+            else if ((shape).s == 1) kernel<true, 1, 3><<<blocks_, 256, 0, st>>>(__VA_ARGS__);             \
+            else kernel<true, 2, 3><<<blocks_, 256, 0, st>>>(__VA_ARGS__);                                 \
+        }                                                                                                  \
+    } while (0)
+
 template <bool kF32>
-static void launch_rates(const pq3d_dense_sim &S, int s, cudaStream_t st)
+static void launch_rates(const pq3d_dense_sim &S, RowShape shape, cudaStream_t st)
 {
-    const unsigned blocks = (unsigned)((S.N * s + 7) / 8);
-    if (s == 1) step_rates_kernel<kF32, 1><<<blocks, 256, 0, st>>>(S);
-    else if (s == 2) step_rates_kernel<kF32, 2><<<blocks, 256, 0, st>>>(S);
-    else if (s == 4) step_rates_kernel<kF32, 4><<<blocks, 256, 0, st>>>(S);
-    else step_rates_kernel<kF32, 8><<<blocks, 256, 0, st>>>(S);
+    PQ3D_ROWS_LAUNCH(step_rates_kernel, shape, S.N, st, S);
 }
 
 template <bool kF32>
-static void launch_matvec(const void *K, const void *v, int64_t N, int s, double *out, cudaStream_t st)
+static void launch_matvec(const void *K, const void *v, int64_t N, RowShape shape, double *out, cudaStream_t st)
 {
-    const unsigned blocks = (unsigned)((N * s + 7) / 8);
-    if (s == 1) matvec_kernel<kF32, 1><<<blocks, 256, 0, st>>>(K, v, N, out);
-    else if (s == 2) matvec_kernel<kF32, 2><<<blocks, 256, 0, st>>>(K, v, N, out);
-    else if (s == 4) matvec_kernel<kF32, 4><<<blocks, 256, 0, st>>>(K, v, N, out);
-    else matvec_kernel<kF32, 8><<<blocks, 256, 0, st>>>(K, v, N, out);
+    PQ3D_ROWS_LAUNCH(matvec_kernel, shape, N, st, K, v, N, out);
 }
 
 }  // namespace step
@@ -580,9 +615,9 @@ static int matvec(const void *K, int64_t N, const void *v, double *out, void *st
     LaunchCfg *cfg;
     const int rc = launch_cfg(&cfg);
     if (rc) return rc;
-    const int s = receiver_warps(N, cfg->sms);
-    if (f32) launch_matvec<true>(K, v, N, s, out, (cudaStream_t)stream);
-    else launch_matvec<false>(K, v, N, s, out, (cudaStream_t)stream);
+    const RowShape shape = row_shape(N, f32, cfg->sms);
+    if (f32) launch_matvec<true>(K, v, N, shape, out, (cudaStream_t)stream);
+    else launch_matvec<false>(K, v, N, shape, out, (cudaStream_t)stream);
     PQ3D_CUDA_TRY(cudaGetLastError());
     return PQ3D_OK;
 }
@@ -614,7 +649,8 @@ extern "C" int pq3d_dense_step(const pq3d_dense_sim *sim, int nsteps, double *h_
     LaunchCfg *cfg;
     const int rc = launch_cfg(&cfg);
     if (rc) return rc;
-    const int grid = attempt_grid(*cfg, f32, sim->N), s = receiver_warps(sim->N, cfg->sms);
+    const int grid = attempt_grid(*cfg, f32, sim->N);
+    const RowShape shape = row_shape(sim->N, f32, cfg->sms);
     // clear the reduction slots and the barrier counter of the control block
     cudaStream_t st = (cudaStream_t)stream;
     PQ3D_CUDA_TRY(cudaMemsetAsync(&sim->ctrl->err_slot[0], 0, sizeof(uint64_t) * 7 + sizeof(uint32_t), st));
@@ -631,8 +667,8 @@ extern "C" int pq3d_dense_step(const pq3d_dense_sim *sim, int nsteps, double *h_
     int step = 0;
     void *args[] = {(void *)&S, (void *)&step, (void *)&h_hist, (void *)&t_hist, (void *)&h_force};
     for (; step < nsteps; ++step) {
-        if (f32) launch_rates<true>(S, s, st);
-        else launch_rates<false>(S, s, st);
+        if (f32) launch_rates<true>(S, shape, st);
+        else launch_rates<false>(S, shape, st);
         PQ3D_CUDA_TRY(cudaGetLastError());
         PQ3D_CUDA_TRY(cudaLaunchCooperativeKernel(attempt, grid, 256, args, 0, st));
     }
