@@ -442,9 +442,7 @@ int pq3d_hmat_partition(const double *xg, int64_t N, int min_size, int mini_leaf
  * admissible blocks, each on a quarter CTA, a CTA or an 8-CTA cluster by its
  * size, rows and columns generated by the GF kernel from `tables`
  * (pq3d_gf_setup).  Takes 4 (nblocks + 2) bytes from the device's memory pool for
- * the call (stream-ordered), and works on a second stream of its own beside
- * `stream`, forked off it and joined to it by events; a captured call stays on
- * `stream` alone.  Per block b: kcap[b] = rank cap,
+ * the call (stream-ordered).  Per block b: kcap[b] = rank cap,
  * UV + uv_off[b] = FP64 scratch for U (kcap x 3m) then V (kcap x 2n),
  * used + used_off[b] = 3m zeroed bytes.  Outputs rank[b] and status[b]
  * (0 converged, 1 rank cap reached, 2 non-finite).  Replaces ACA_worker /

@@ -41,8 +41,9 @@ inline cudaError_t allow_smem(void (*kernel)(P...), size_t bytes)
 
 // Launch that may start before the stream's previous kernel has ended: when all
 // that kernel's blocks have called chain_release or ended.  A kernel launched
-// so calls chain_wait in every block, also in one that has nothing to do: it
-// returns once the previous kernel is complete and its writes are visible.
+// so calls chain_wait, which returns once the previous kernel is complete and its
+// writes are visible: in every block that touches what that kernel writes, and in
+// one at least, since the next kernel on the stream waits for this one only.
 // Before it, a kernel may read only what no kernel since the last one known to be
 // complete writes, and writes nothing.  Known to be complete, with its writes
 // visible: everything before the previous kernel, where that one (the product,

@@ -65,7 +65,11 @@ struct PairGen {
 // ACA.  A block is worked on by a group of kAcaSmall threads (a quarter of a
 // CTA), by a CTA, or by a cluster of kAcaCluster CTAs; each kind only meets at
 // its own barriers.  The clusters are one launch, the rest another beside it
-// (clusters alone leave the SMs of a GPC that make no eighth idle).
+// (clusters alone leave the SMs of a GPC that make no eighth idle), let in once
+// every cluster is on the chip: eight free SMs of a GPC hardly come about while
+// single CTAs take them (beside one another from the start, N = 900, 198 blocks of up
+// to 450 elements: 7.55 ms, 5.57 so; N = 12,100: 35.9 and 30.6 ms; 30,000, without
+// clusters: 106 ms).
 //
 // Bound: the FP64 pipe -- per iteration n + m pair evaluations of 520
 // operations, 2 k (M + Nc) multiply-adds for the residual row and column and
@@ -218,6 +222,9 @@ aca_kernel(bool clusters, PairGen<kHalf> gen, const double *__restrict__ recv, c
            int32_t *__restrict__ rank_out, int32_t *__restrict__ status_out)
 {
     __shared__ AcaSlot slots[2 * kAcaWarps];
+    if (clusters) chain_release();
+    // one CTA of the second launch, with a block to work on or without, ends after the clusters
+    const bool last = !clusters && blockIdx.x == gridDim.x - 1;
     const int nh = split[0], nl = split[1];
     AcaGroup g;
     g.turn = 0;
@@ -244,7 +251,10 @@ aca_kernel(bool clusters, PairGen<kHalf> gen, const double *__restrict__ recv, c
         pos = nh + nl + (pos - nl) * kAcaGroups + q;
         end = nblocks;
     }
-    if (pos >= end) return;   // whole groups (and whole clusters) leave
+    if (pos >= end) {   // whole groups (and whole clusters) leave
+        if (last) chain_wait();
+        return;
+    }
     if (g.id == 0) g.sync();  // every CTA of the cluster runs before its shared memory is written to
     const int b = order[pos];
     const int64_t r0 = blk[4 * b], r1 = blk[4 * b + 1], c0 = blk[4 * b + 2], c1 = blk[4 * b + 3];
@@ -372,6 +382,7 @@ aca_kernel(bool clusters, PairGen<kHalf> gen, const double *__restrict__ recv, c
         rank_out[b] = k;
         status_out[b] = status;
     }
+    if (last) chain_wait();
 }
 
 // Storage of block b at data + off[b] (FP32, column-major so that the lanes
@@ -1372,28 +1383,6 @@ static PairGen<kHalf> make_gen(const double *tables, int64_t N, double mu, doubl
                           2.0 * mu, lambda_};
 }
 
-// The second stream of one ACA call and the events that fork it off the
-// caller's stream and join it again.  They live as long as the call (what is
-// queued on them goes on; CUDA gives them back when it is done): nothing is left
-// in a host thread that ends, or behind a device reset.
-struct AcaFork {
-    cudaStream_t stream = nullptr;
-    cudaEvent_t begin = nullptr, end = nullptr;
-    cudaError_t open()
-    {
-        cudaError_t e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&begin, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&end, cudaEventDisableTiming);
-        return e;
-    }
-    ~AcaFork()
-    {
-        if (end) cudaEventDestroy(end);
-        if (begin) cudaEventDestroy(begin);
-        if (stream) cudaStreamDestroy(stream);
-    }
-};
-
 extern "C" int pq3d_hmat_aca(const double *tables, int64_t N, const int64_t *perm, int nblocks, const int64_t *blk,
                              const int32_t *kcap, double tol, double mu, double lambda_, int halfspace, double *UV,
                              const int64_t *uv_off, uint8_t *used, const int64_t *used_off, int32_t *rank,
@@ -1408,12 +1397,6 @@ extern "C" int pq3d_hmat_aca(const double *tables, int64_t N, const int64_t *per
     // the work order lives for this call only (stream-ordered scratch); grids
     // of nblocks clusters and CTAs serve any split, those past the last leave
     PQ3D_REQUIRE(nblocks <= INT32_MAX / kAcaCluster, "pq3d_hmat_aca: too many blocks");
-    // A captured call takes both launches on the caller's stream, one after the
-    // other: a graph is to hold no stream of ours.
-    cudaStreamCaptureStatus capturing;
-    PQ3D_CUDA_TRY(cudaStreamIsCapturing(st, &capturing));
-    AcaFork fork;
-    if (capturing == cudaStreamCaptureStatusNone) PQ3D_CUDA_TRY(fork.open());
     int32_t *split = nullptr;
     PQ3D_CUDA_TRY(cudaMallocAsync(&split, ((size_t)nblocks + 2) * sizeof(int32_t), st));
     aca_order_kernel<<<1, 1024, 0, st>>>(blk, nblocks, split + 2, split);
@@ -1428,20 +1411,15 @@ extern "C" int pq3d_hmat_aca(const double *tables, int64_t N, const int64_t *per
         cfg.stream = st;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
+        const int32_t *order = split + 2;
         cudaError_t e = cudaGetLastError();   // of aca_order_kernel
-        if (e == cudaSuccess && fork.stream) e = cudaEventRecord(fork.begin, st);
-        if (e == cudaSuccess && fork.stream) e = cudaStreamWaitEvent(fork.stream, fork.begin, 0);
         if (e == cudaSuccess)
-            e = cudaLaunchKernelEx(&cfg, kernel, true, gen, recv, perm, blk, (const int32_t *)(split + 2),
-                                   (const int32_t *)split, nblocks, kcap, tol, UV, uv_off, used, used_off, rank, status);
-        if (e != cudaSuccess) return e;   // nothing is on the second stream yet
-        kernel<<<nblocks, kAcaThreads, 0, fork.stream ? fork.stream : st>>>(
-            false, gen, recv, perm, blk, split + 2, split, nblocks, kcap, tol, UV, uv_off, used, used_off, rank, status);
-        e = cudaGetLastError();
-        if (e == cudaSuccess && fork.stream) e = cudaEventRecord(fork.end, fork.stream);
-        if (e == cudaSuccess && fork.stream) e = cudaStreamWaitEvent(st, fork.end, 0);
-        // not joined: the caller's stream must not go on beside what may run there
-        if (e != cudaSuccess && fork.stream) cudaStreamSynchronize(fork.stream);
+            e = cudaLaunchKernelEx(&cfg, kernel, true, gen, recv, perm, blk, order, (const int32_t *)split, nblocks, kcap,
+                                   tol, UV, uv_off, used, used_off, rank, status);
+        if (e == cudaSuccess)
+            e = launch_chained(kernel, dim3((unsigned)nblocks), dim3(kAcaThreads), 0, st, false, gen, recv, perm, blk,
+                               order, (const int32_t *)split, nblocks, kcap, tol, UV, uv_off, used, used_off, rank,
+                               status);
         return e;
     };
     const cudaError_t launched = halfspace ? launch(aca_kernel<true>, make_gen<true>(tables, N, mu, lambda_))
