@@ -85,14 +85,17 @@ constexpr int kAcaSmall = 64;     // (the barrier counts of AcaGroup::sync)
 constexpr int kAcaGroups = kAcaThreads / kAcaSmall;
 constexpr int kAcaCluster = 8;
 constexpr int kAcaWarps = kAcaCluster * kAcaThreads / 32;
-// A block with more elements (m + n) than the average share of kAcaSlots CTAs
-// (one per SM) would end last on one CTA: it gets a cluster, from 256 elements
-// on.  A small group is for blocks of at most kAcaSmallSide elements a side
-// (four rounds of the group) and of at most the share of a group's slot: with
-// few blocks (N = 3,600: 216) the SMs would idle while groups of 64 threads
-// walk 256-element sides.
+// A block with more elements (m + n) than the average share of a CTA per SM would
+// end last on one CTA: it gets a cluster, from 256 elements on -- unless the blocks
+// are few (three an SM) and the clusters more than the chip holds at once, so that
+// their second round ends last (156 blocks, 24 of them of more than 256 elements:
+// 5.0 ms with clusters, 3.4 ms on a CTA each; 426: 6.4 and 4.3).
+// A small group is for blocks of at most kAcaSmallSide elements a side (four rounds
+// of the group) and of at most the share of a group's slot: with few blocks (N =
+// 3,600: 216) the SMs would idle while groups of 64 threads walk 256-element sides.
+// (The group's width is the order of the norms' sums: the factors' values do not
+// depend on it, their number only where the stopping rule is a matter of rounding.)
 constexpr int kAcaSmallSide = 256;
-constexpr int kAcaSlots = 152;
 constexpr int kAcaHugeMin = 256;
 
 struct __align__(16) AcaSlot {
@@ -171,13 +174,14 @@ struct AcaGroup {
 // order within a class does not matter).  split = {huge blocks, large blocks}.
 constexpr int kAcaClasses = 64;
 __global__ void __launch_bounds__(1024)
-aca_order_kernel(const int64_t *__restrict__ blk, int nblocks, int32_t *__restrict__ order, int32_t *__restrict__ split)
+aca_order_kernel(const int64_t *__restrict__ blk, int nblocks, int sms, int32_t *__restrict__ order,
+                 int32_t *__restrict__ split)
 {
-    __shared__ int count[3 * kAcaClasses];
+    __shared__ int count[3 * kAcaClasses], nhuge;
     __shared__ unsigned long long total;
     const int t = threadIdx.x;
     if (t < 3 * kAcaClasses) count[t] = 0;
-    if (t == 0) total = 0;
+    if (t == 0) { total = 0; nhuge = 0; }
     __syncthreads();
     auto side_m = [&](int b) { return blk[4 * b + 1] - blk[4 * b]; };
     auto side_n = [&](int b) { return blk[4 * b + 3] - blk[4 * b + 2]; };
@@ -185,8 +189,14 @@ aca_order_kernel(const int64_t *__restrict__ blk, int nblocks, int32_t *__restri
     for (int b = t; b < nblocks; b += blockDim.x) mine += (unsigned long long)(side_m(b) + side_n(b));
     atomicAdd(&total, mine);
     __syncthreads();
-    const int64_t huge = max((int64_t)kAcaHugeMin, (int64_t)(total / kAcaSlots));
-    const int64_t small = (int64_t)(total / (kAcaSlots * kAcaGroups));
+    int64_t huge = max((int64_t)kAcaHugeMin, (int64_t)(total / (unsigned)sms));
+    const int64_t small = (int64_t)(total / (unsigned)(sms * kAcaGroups));
+    if (nblocks <= 3 * sms) {
+        for (int b = t; b < nblocks; b += blockDim.x)
+            if (side_m(b) + side_n(b) > huge) atomicAdd(&nhuge, 1);
+        __syncthreads();
+        if (nhuge > sms / kAcaCluster) huge = INT64_MAX;
+    }
     auto cls = [&](int b) {
         const int64_t m = side_m(b), n = side_n(b);
         const int kind = m + n > huge ? 0 : (max(m, n) > kAcaSmallSide || m + n > small ? 1 : 2);
@@ -1397,9 +1407,12 @@ extern "C" int pq3d_hmat_aca(const double *tables, int64_t N, const int64_t *per
     // the work order lives for this call only (stream-ordered scratch); grids
     // of nblocks clusters and CTAs serve any split, those past the last leave
     PQ3D_REQUIRE(nblocks <= INT32_MAX / kAcaCluster, "pq3d_hmat_aca: too many blocks");
+    int dev, sms;
+    PQ3D_CUDA_TRY(cudaGetDevice(&dev));
+    PQ3D_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     int32_t *split = nullptr;
     PQ3D_CUDA_TRY(cudaMallocAsync(&split, ((size_t)nblocks + 2) * sizeof(int32_t), st));
-    aca_order_kernel<<<1, 1024, 0, st>>>(blk, nblocks, split + 2, split);
+    aca_order_kernel<<<1, 1024, 0, st>>>(blk, nblocks, sms, split + 2, split);
     auto launch = [&](auto kernel, auto gen) -> cudaError_t {
         cudaLaunchAttribute attr;
         attr.id = cudaLaunchAttributeClusterDimension;
