@@ -1492,10 +1492,10 @@ extern "C" int pq3d_hmat_apply_masked(const pq3d_hmat *H, const double *X, int B
     int dev, sms;
     PQ3D_CUDA_TRY(cudaGetDevice(&dev));
     PQ3D_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    // One run, or so few leaves that a CTA for each and every run still finds room on
-    // the chip: run by run, the run fastest in the block index.  (8 runs: N = 900, 32
-    // leaves 35 us, 47 in a group; N = 2,500, 64 leaves 76, 71.)
-    if (B == 1 || (int64_t)H->nleaves * B <= 2 * sms) {
+    // One run, or so few leaves that a CTA for each and every run (three to an SM) still
+    // finds room on the chip: run by run, the run fastest in the block index.  (8 runs:
+    // N = 900, 32 leaves 35 us, 47 in a group; N = 2,500, 64 leaves 76, 71.)
+    if (B == 1 || (int64_t)H->nleaves * B <= 3 * sms) {
         PQ3D_REQUIRE(t_ctas * B < (int64_t)INT32_MAX && (int64_t)H->nleaves * B < (int64_t)INT32_MAX,
                      "pq3d_hmat_apply: too many rank rows or leaves x runs");
         float2 *Xs = (float2 *)workspace, *T = Xs + (size_t)B * 2 * N;
@@ -1517,10 +1517,11 @@ extern "C" int pq3d_hmat_apply_masked(const pq3d_hmat *H, const double *X, int B
                  "pq3d_hmat_apply: too many rank rows or leaves x runs");
     Pair2 *Xs = (Pair2 *)workspace, *T = Xs + (size_t)(slots / 2) * 2 * N;
     int32_t *list = (int32_t *)(T + (size_t)(slots / 2) * H->t_rows);
-    // Rows of a leaf's pass: half of them where the leaves leave SMs without a CTA, so
-    // that a leaf's second CTA takes the rest (2 runs: N = 8,100, 184 leaves 144 us,
-    // whole passes 158; N = 12,100, 256 leaves 188, 175).
-    const int pass_rows = 3 * (int64_t)H->nleaves * ngroups <= 4 * sms ? kPassRows / 2 : kPassRows;
+    // Rows of a leaf's pass: half of them where the leaves of one group of runs leave
+    // SMs without a CTA, so that a leaf's second CTA takes the rest (2 runs: N = 8,100,
+    // 184 leaves 144 us, whole passes 158; N = 12,100, 256 leaves 188, 175; 20 runs,
+    // N = 2,200: an iteration 190 us, 176).
+    const int pass_rows = ngroups == 1 && 3 * H->nleaves <= 4 * sms ? kPassRows / 2 : kPassRows;
     // How many runs take part is known on the device only.  A batch's only run does
     // better with the one-run kernels, from about four leaves an SM on (N = 99,856:
     // 1,075 us, 1,189 as half a pair; N = 29,756, 512 leaves: 362, 361): they follow
