@@ -385,8 +385,10 @@ int pq3d_batch_iterate_end(const pq3d_batch_sim *sim, void *stream);
 /* ---------------- device: H-matrix ---------------- */
 
 /* Source and receiver tables of a mesh (the set-up step of the assembly) into
- * `workspace` (pq3d_gf_workspace_bytes(N)), and with halfspace != 0 the image
- * and free-surface tables: used by the H-matrix kernels. */
+ * `workspace` (pq3d_gf_setup_bytes(N, halfspace); the assembly's workspace is
+ * larger and serves too), and with halfspace != 0 the image and free-surface
+ * tables: used by the H-matrix kernels. */
+size_t pq3d_gf_setup_bytes(int64_t N, int halfspace);
 int pq3d_gf_setup(const double *nodes, const int64_t *tris, int64_t N, int halfspace, void *workspace,
                   size_t workspace_bytes, void *stream);
 

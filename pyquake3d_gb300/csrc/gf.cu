@@ -1232,12 +1232,17 @@ extern "C" int pq3d_assemble_dense_noalloc(const double *nodes, const int64_t *t
     return assemble_rows(nodes, tris, N, row0, row1, mu, lambda_, K64, K32, scratch, true, (cudaStream_t)stream);
 }
 
+extern "C" size_t pq3d_gf_setup_bytes(int64_t N, int halfspace)
+{
+    return N > 0 ? tables_doubles(N, halfspace != 0) * sizeof(double) : 0;
+}
+
 extern "C" int pq3d_gf_setup(const double *nodes, const int64_t *tris, int64_t N, int halfspace, void *workspace,
                              size_t workspace_bytes, void *stream)
 {
     clear_error();
     PQ3D_REQUIRE(nodes && tris && workspace && N > 0, "pq3d_gf_setup: bad arguments");
-    PQ3D_REQUIRE(workspace_bytes >= tables_doubles(N, halfspace != 0) * sizeof(double) && aligned16(workspace),
+    PQ3D_REQUIRE(workspace_bytes >= pq3d_gf_setup_bytes(N, halfspace) && aligned16(workspace),
                  "pq3d_gf_setup: workspace too small");
     double *src = (double *)workspace;
     double *recv = src + (size_t)kSrcStride * N;

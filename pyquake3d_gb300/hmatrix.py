@@ -116,9 +116,9 @@ class HMatrix:
         st = torch.cuda.current_stream(dev).cuda_stream
         self.nodes_t = torch.as_tensor(nodes, device=dev)
         self.tris_t = torch.as_tensor(tris, device=dev)
-        self.tables = torch.empty(L.pq3d_gf_workspace_bytes(N), dtype=torch.uint8, device=dev)
         hs = int(bool(halfspace))
         self.halfspace = bool(halfspace)
+        self.tables = torch.empty(L.pq3d_gf_setup_bytes(N, hs), dtype=torch.uint8, device=dev)
         _lib.check(L.pq3d_gf_setup(self.nodes_t.data_ptr(), self.tris_t.data_ptr(), N, hs, self.tables.data_ptr(),
                                    self.tables.numel(), st))
         phase("gf_tables")
