@@ -483,40 +483,6 @@ __device__ __noinline__ void pair_angular_hs(const double *src, const double *im
     pair_tractions_hs(F, Fi, G, R, nu, k, two_mu, lam, ts, td);
 }
 
-// The correction of one edge as a matrix like seg_matrix's, added to M.
-__device__ __forceinline__ void fsc_matrix(const TileSide &F, const double *R, double nu, double two_mu, double lam,
-                                           double M[9])
-{
-    double U[3][6];
-    if (!fsc_side_strains(F, R[0], R[1], R[2], nu, U)) return;
-    const double c1 = F(S_C1), s1 = F(S_S1);
-    // in units of mu/(4 pi): the strains' factor 1/(4 pi (1 - nu)) times 2 mu, lambda
-    const double c2 = 2.0 / (1.0 - nu), cl = c2 * lam / two_mu;
-    double r[3][3];   // the receiver's axes in the side's frame
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const double *e = R + 3 + 3 * a;
-        r[a][0] = e[0] * c1 + e[1] * s1;
-        r[a][1] = e[0] * s1 - e[1] * c1;
-        r[a][2] = -e[2];
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const double *e = U[k];
-        const double h3 = 0.5 * e[3], h4 = 0.5 * e[4], h5 = 0.5 * e[5];
-        const double u0 = e[0] * r[2][0] + h3 * r[2][1] + h4 * r[2][2];
-        const double u1 = h3 * r[2][0] + e[1] * r[2][1] + h5 * r[2][2];
-        const double u2 = h4 * r[2][0] + h5 * r[2][1] + e[2] * r[2][2];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            double t = c2 * (r[c][0] * u0 + r[c][1] * u1 + r[c][2] * u2);
-            if (c == 2) t += cl * (e[0] + e[1] + e[2]);
-#pragma unroll
-            for (int a = 0; a < 3; ++a) M[3 * c + a] += t * r[a][k];
-        }
-    }
-}
-
 template <bool kWrite32>
 __global__ void __launch_bounds__(kHsThreads, 2)
 assemble_hs_kernel(const Tile *__restrict__ tiles, const TileHs *__restrict__ hs, int ts,
