@@ -133,19 +133,20 @@ def fp64_peak_tflops(torch, dev):
 
 # FP64 operations of one (receiver, source) pair of the tiled assembly (both
 # unit slips, 6 entries; add, sub, mul, div and sqrt one each), counted on the
-# kernel's own device math: 27 per vertex, 127 per edge and 72 per pair, with the
-# 0.648 vertices and 1.645 edges per triangle of the tiles of the N = 20,000 mesh.
-GF_FLOP_PER_PAIR = 298
+# kernel's own device math by oracle/count_tile_flops.cpp: 27 per vertex, 127 per edge
+# and 72 per pair, with the 0.6703 vertices and 1.6664 edges per triangle of the tiles
+# of the N = 20,000 mesh.
+GF_FLOP_PER_PAIR = 302
 # The same pair with the published angular-dislocation expressions
 # (src/TDstressFS_C.cpp:51-121) evaluated term by term and rotated tensor by
 # tensor (src/TDstressFS_C.cpp:185-256), both slips sharing the geometry and
-# 11 divisions: 1,016, counted by the same tool (the kernel's first form).
+# 11 divisions: 1,016, counted by oracle/count_gf_flops.cpp (the kernel's first form).
 GF_FLOP_PER_PAIR_TERM_BY_TERM = 1016
-# The same for the half-space kernel: 2,682 per edge (of which the free-surface
-# correction's two end points 2,131: 826 add + 1,295 mul + 8 div + 2 sqrt) and 168
-# per pair, with the 1.634 edges per triangle of the N = 2,500 mesh of
-# bench_halfspace (a pair by itself, as the single-source calls take it: 8,263).
-HS_FLOP_PER_PAIR = 4550
+# The same for the half-space kernel: 2,689 per edge (of which the free-surface
+# correction's two end points 2,131) and 168 per pair, with the 1.634 edges per
+# triangle of the N = 2,500 mesh of bench_halfspace (a pair by itself, as the
+# single-source calls take it: 8,404, oracle/count_hs_flops.cpp).
+HS_FLOP_PER_PAIR = 4562
 # Stores per pair: 6 FP64 + 6 FP32 entries.
 GF_BYTES_PER_PAIR = 72
 

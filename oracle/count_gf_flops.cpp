@@ -1,4 +1,4 @@
-// Operation count of the GPU assembly kernel's per-pair arithmetic -- test
+// Operation count of a (receiver, source) pair evaluated by itself -- test
 // infrastructure.  Instantiates the device math of
 // pyquake3d_gb300/csrc/gf_device.cuh with a counting scalar type and runs it
 // over every (receiver, source) pair of a mesh read from stdin

@@ -1,9 +1,9 @@
-// Operation count of the GPU half-space assembly kernel's per-pair arithmetic
+// Operation count of a half-space (receiver, source) pair evaluated by itself
 // -- test infrastructure.  Compiles the device math of
 // pyquake3d_gb300/csrc/gf_device.cuh and hs_device.cuh with every `double`
-// replaced by a counting scalar type and runs the kernel body
+// replaced by a counting scalar type and runs the pair evaluation
 // (pair_tractions_hs: main dislocation, image dislocation, the free-surface
-// correction of the three sides in forward-mode dual numbers, two traction
+// correction of the three sides in forward mode, two traction
 // contractions) over every (receiver, source) pair of a mesh read from stdin
 // ("N" then N lines of 9 vertex coordinates; z <= 0).  Prints the mean number
 // of FP64 operations per pair as JSON.  Convention as the full-space count:

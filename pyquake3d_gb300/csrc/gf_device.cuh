@@ -34,7 +34,7 @@
 #include <math.h>
 
 #ifndef __CUDACC__
-// Host compilation (operation counting in oracle/count_gf_flops.cpp).
+// Host compilation (operation counts in oracle/, host checks in tests/).
 #include <cmath>
 #define __host__
 #define __device__
