@@ -695,8 +695,13 @@ template <bool kMany>
 static void launch_points_full(const SrcVal &s, const PointArgs &P, size_t n, cudaStream_t st)
 {
     const unsigned blocks = (unsigned)((n + kPointPairs - 1) / kPointPairs);
-    if (!kMany || n <= kPointShare) points_full_kernel<kMany, 3><<<blocks, 96, 0, st>>>(s, P);
-    else points_full_kernel<kMany, 1><<<blocks, 32, 0, st>>>(s, P);
+    if constexpr (kMany) {
+        if (n > kPointShare) {
+            points_full_kernel<true, 1><<<blocks, 32, 0, st>>>(s, P);
+            return;
+        }
+    }
+    points_full_kernel<kMany, 3><<<blocks, 96, 0, st>>>(s, P);
 }
 
 static inline double poisson(double mu, double lam) { return 1.0 / (1.0 + lam / mu) / 2.0; }

@@ -677,8 +677,10 @@ __device__ __forceinline__ void tractions_tdcs_scaled(const T E[6], const T ue1[
 // The six tractions of one (receiver, source) pair: receiver record R
 // (centroid, e1, e2, n), source fields F; ts = unit strike slip, td = unit dip
 // slip, components (e1, e2, n).  kScaledAxes: R's e1 and e2 come multiplied
-// by traction_axis_scale(k, two_mu) (the assembly kernel scales them once per
-// receiver tile).
+// by traction_axis_scale(k, two_mu).  No kernel takes that form (it was for a
+// receiver that meets many sources, which the tiled assembly has taken over); the
+// host check of the pair evaluation (tests/hs_host_check.cpp) and the operation
+// count go through it.
 __host__ __device__ inline double traction_axis_scale(double k, double two_mu) { return (0.5 * k) * two_mu; }
 
 template <class Src, bool kScaledAxes = false>

@@ -571,6 +571,7 @@ __device__ __forceinline__ void image_signs(double surface, double e[6])
     if (surface != 0.0) { e[4] = -e[4]; e[5] = -e[5]; }
 }
 
+// All parts by one thread: for the host check (the kernels share them over warps).
 template <class Src, class Fs>
 __device__ __forceinline__ void point_strain_hs(const Src &F, const Src &Fi, const Fs &G, double X, double Y,
                                                 double Z, double bx, double by, double bz, double nu, double k,
