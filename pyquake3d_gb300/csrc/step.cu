@@ -3,7 +3,8 @@
 //
 // Reference behaviour (src/QDsim_gpu.py):
 //   traction product K.(V - Vpl), once per accepted step        948-957
-//   right-hand side (aging law, radiation damping)             830-891
+//   right-hand side (aging law, radiation damping)             830-891, in
+//     reciprocal form with the reference formula's error (rhs_recip<true>)
 //   Dormand-Prince 5(4) attempt, max-relative error norm      1128-1262
 //   accept / reject and dt control                              959-985
 //   closed-form slip rate, rake, slip integration              994-1027
@@ -358,7 +359,7 @@ __global__ void __launch_bounds__(256) dense_attempt_kernel(pq3d_dense_sim S, in
                          S.P ? S.P[i] : 0.0, S.dPdt ? S.dPdt[i] : 0.0};
             const double y[4] = {S.Tno[i], S.Tt1o[i], S.Tt2o[i], S.state[i]};
             double yo[4], e1, e2;
-            dp_attempt<true>(c, S.V0, S.eta, h, y, yo, e1, e2);
+            dp_attempt<true, true>(c, S.V0, S.eta, h, y, yo, e1, e2);
             reinterpret_cast<double4_16a *>(S.cand)[i] = make_double4_16a(yo[0], yo[1], yo[2], yo[3]);
             m1 = (isnan(m1) || isnan(e1)) ? NAN : fmax(m1, e1);
             m2 = (isnan(m2) || isnan(e2)) ? NAN : fmax(m2, e2);
