@@ -170,14 +170,20 @@ struct RowShape {
 // (FP64), since blocks come and go.  The FP32 operator is bound by the loads in
 // flight, and its blocks are best all resident at once: three and four take the
 // builds that allow it, and from five on two warps per receiver even out the last
-// ones.  us (one warp per receiver and 2 blocks per SM / as chosen):
+// round of blocks where it is less than two thirds full.  us (one warp per receiver
+// and 2 blocks per SM / as chosen; a step at N = 6,500 237 us, split 242):
 // FP64 N = 400 8.1 / 6.2, 1,000 18.3 / 18.3 (with 4 warps 23.4), 1,600 43.6 / 37.4;
 // FP32 N = 304 4.8 / 4.0, 2,500 37.9 / 29.6, 3,000 52.0 / 38.0, 4,000 70.1 / 65.6,
 // 5,000 120 / 105, 8,000 259 / 249, 20,000 1,458 / 1,401.
 static RowShape row_shape(int64_t N, bool f32, int sms)
 {
     const int64_t b = (N + 8 * sms - 1) / (8 * (int64_t)sms);
-    if (b > 2) return f32 ? (b == 3 ? RowShape{1, 3} : (b == 4 ? RowShape{1, 4} : RowShape{2, 3})) : RowShape{1, 2};
+    if (b > 2) {
+        if (!f32) return RowShape{1, 2};
+        if (b <= 4) return RowShape{1, (int)b};
+        const int64_t round = 2 * sms, last = ((N + 7) / 8 - 1) % round + 1;
+        return 3 * last < 2 * round ? RowShape{2, 3} : RowShape{1, 2};
+    }
     int best = 1;
     int64_t cost = INT64_MAX;
     for (int s = 1; s <= 4 && 32 * (s - 1) < N; s *= 2) {   // none without sources
