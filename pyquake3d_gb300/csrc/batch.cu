@@ -614,8 +614,8 @@ __global__ void __launch_bounds__(256) update_kernel(pq3d_batch_sim S)
 // while it works out the next step size (rank 0's writes the control record).
 //
 // Bound: latency (two kernel boundaries, three trips to the control record and
-// the candidate through L2 gone).  N = 2,000, B = 16, BF16X6: iteration 47.8 us
-// as three kernels, 38.9 us, of which the product takes 23.5.
+// the candidate through L2 gone).  N = 2,000, B = 16, BF16X6: iteration 48.0 us
+// as three kernels, 42.5 us, of which the product takes 23.5.
 constexpr int kStepCluster = 8;   // blocks of a run at most
 constexpr int kStepCells = 512;   // cells of a block at most
 
@@ -714,9 +714,9 @@ static bool mixed_attempt(const pq3d_batch_sim &S) { return S.precision != PQ3D_
 // better ones: a run's blocks want SMs of their own (the FP64 conversions of a
 // cell are a third of its time), and a full chip leaves no room to place
 // clusters.  us an iteration of the BF16X6 product, cluster / three kernels:
-// N = 2,000: B = 16 45.6 / 51.5, B = 64 68.3 / 66.4, B = 200 154 / 124;
-// N = 1,000: B = 30 27.9 / 30.6, B = 38 (152 blocks) 34.6 / 32.1; N = 4,000 (512
-// cells a block): B = 9 108.8 / 114.6, B = 19 126.5 / 121.9.
+// N = 2,000: B = 16 42.5 / 48.0, B = 64 68.3 / 66.4, B = 200 154 / 124; N = 1,000: B = 30
+// 24.0 / 26.4, B = 38 (152 blocks) 34.6 / 32.1; N = 4,000 (512 cells a block): B = 9 105.0 /
+// 111.5, B = 19 126.5 / 121.9.
 static int step_clusters(const pq3d_batch_sim &S, int sms)
 {
     if (!mixed_attempt(S) || S.precision == PQ3D_BATCH_BF16X18 || S.N > kStepCluster * kStepCells) return 0;

@@ -716,7 +716,8 @@ lowrank_T_only_kernel(const float *__restrict__ data, const longlong2 *__restric
 // 19 instructions per 192 products -- 1.46 ms with 8 runs per entry (rank rows
 // 0.58, leaf rows 0.85), 1.06 ms with the loads kept in flight, the float-float
 // sums of two runs in one instruction and the row passes on two CTAs (0.35 and
-// 0.69).  A second set of registers for the next entries spills: 1.50 ms.
+// 0.69), 1.02 ms with more L1 left to the leaf rows (0.64).  A second set of
+// registers for the next entries spills: 1.50 ms.
 
 __host__ __device__ inline int group_width(int left) { return left > 4 ? 8 : (left > 2 ? 4 : 2); }
 // slots of n runs (B > 1)
