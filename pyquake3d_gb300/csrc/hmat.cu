@@ -23,7 +23,8 @@
 //     or in a batch).  The ACA tolerance (1e-4) dominates this rounding by
 //     orders of magnitude.
 //   * several right-hand sides share every loaded entry in groups of up to 8
-//     runs (leaf_rows_runs_kernel, lowrank_T_runs_kernel).
+//     runs (leaf_rows_runs_kernel, lowrank_T_runs_kernel); with few leaves they
+//     go run by run.
 // Index space: elements are renumbered so that every cluster is a contiguous
 // range (perm[p] = element at position p); a block is a pair of ranges.
 #include <math.h>

@@ -11,8 +11,9 @@
 //
 // GPU design, per accepted step two launches queued back to back (no host
 // synchronisation between steps): (1) the traction product, a warp per
-// receiver streaming its three operator rows (16-byte loads) against the
-// interleaved slip-rate deficit v', at the full occupancy of a small kernel;
+// receiver (two or four on small meshes) streaming its three operator rows
+// (16-byte loads) against the interleaved slip-rate deficit v', at the full
+// occupancy of a small kernel;
 // (2) one cooperative kernel: every thread runs the 7 right-hand-side
 // evaluations of its cells in registers (the traction rates are frozen over
 // the step, so the stages are cell-local), block-max + one atomicMax per block
